@@ -12,7 +12,8 @@
 // that reproduce the reference's entries have to run the same algorithm.
 // This file restates it:
 //   * gk21 / gk15i: the 21-point Gauss-Kronrod rule on [a, b], and the
-//     15-point rule on a subinterval of (0, 1] after x = bound + (1 - t) / t;
+//     15-point rule on a subinterval of (0, 1] after x = bound + (1 - t) / t,
+//     the node values first and then their sums (combine21 / combine15);
 //     each returns the Kronrod estimate, the QUADPACK error estimate (scaled
 //     |Kronrod - Gauss|, bounded below by 50 eps resabs), and |f| / |f - mean|
 //     integrals;
@@ -51,21 +52,22 @@ SFP_HD double rule_error(double abserr, double resabs, double resasc) {
     return abserr;
 }
 
-// 21-point Gauss-Kronrod on [a, b]
-template <class F>
-SFP_HD void gk21(const F& f, double a, double b, double& result, double& abserr, double& resabs, double& resasc) {
-    const double centr = 0.5 * (a + b), hlgth = 0.5 * (b - a), dhlgth = fabs(hlgth);
-    double fv1[10], fv2[10];
+// a rule on one subinterval: the Kronrod estimate, its error estimate and
+// the integrals of |f| and |f - mean|
+struct RuleValue {
+    double result, abserr, resabs, resasc;
+};
+
+// the 21-point rule from its node values: fc at the centre, fv1[j] / fv2[j]
+// at centre -/+ hlgth xgk21(j)
+SFP_HD void combine21(double fc, const double* fv1, const double* fv2, double hlgth, RuleValue& v) {
+    const double dhlgth = fabs(hlgth);
     double resg = 0.0;
-    const double fc = f(centr);
     double resk = sfp_gk::wgk21(10) * fc;
-    resabs = fabs(resk);
+    double resabs = fabs(resk);
     for (int j = 0; j < 5; ++j) {  // the Gauss nodes xgk[1], xgk[3], ..
         const int jtw = 2 * j + 1;
-        const double absc = hlgth * sfp_gk::xgk21(jtw);
-        const double f1 = f(centr - absc), f2 = f(centr + absc);
-        fv1[jtw] = f1;
-        fv2[jtw] = f2;
+        const double f1 = fv1[jtw], f2 = fv2[jtw];
         const double fsum = f1 + f2;
         resg += sfp_gk::wg21(j) * fsum;
         resk += sfp_gk::wgk21(jtw) * fsum;
@@ -73,54 +75,74 @@ SFP_HD void gk21(const F& f, double a, double b, double& result, double& abserr,
     }
     for (int j = 0; j < 5; ++j) {  // the Kronrod nodes xgk[0], xgk[2], ..
         const int jtwm1 = 2 * j;
-        const double absc = hlgth * sfp_gk::xgk21(jtwm1);
-        const double f1 = f(centr - absc), f2 = f(centr + absc);
-        fv1[jtwm1] = f1;
-        fv2[jtwm1] = f2;
+        const double f1 = fv1[jtwm1], f2 = fv2[jtwm1];
         const double fsum = f1 + f2;
         resk += sfp_gk::wgk21(jtwm1) * fsum;
         resabs += sfp_gk::wgk21(jtwm1) * (fabs(f1) + fabs(f2));
     }
     const double reskh = resk * 0.5;
-    resasc = sfp_gk::wgk21(10) * fabs(fc - reskh);
+    double resasc = sfp_gk::wgk21(10) * fabs(fc - reskh);
     for (int j = 0; j < 10; ++j) resasc += sfp_gk::wgk21(j) * (fabs(fv1[j] - reskh) + fabs(fv2[j] - reskh));
-    result = resk * hlgth;
-    resabs *= dhlgth;
-    resasc *= dhlgth;
-    abserr = rule_error(fabs((resk - resg) * hlgth), resabs, resasc);
+    v.result = resk * hlgth;
+    v.resabs = resabs * dhlgth;
+    v.resasc = resasc * dhlgth;
+    v.abserr = rule_error(fabs((resk - resg) * hlgth), v.resabs, v.resasc);
 }
 
-// 15-point Gauss-Kronrod on [a, b] of (0, 1] for the integral of f over
-// [bound, inf): x = bound + (1 - t) / t, dx = dt / t^2
+// 21-point Gauss-Kronrod on [a, b]
 template <class F>
-SFP_HD void gk15i(const F& f, double bound, double a, double b, double& result, double& abserr, double& resabs,
-                  double& resasc) {
+SFP_HD void gk21(const F& f, double a, double b, RuleValue& v) {
     const double centr = 0.5 * (a + b), hlgth = 0.5 * (b - a);
-    double fv1[7], fv2[7];
-    const double tabsc1 = bound + (1.0 - centr) / centr;
-    const double fc = (f(tabsc1) / centr) / centr;
+    double fv1[10], fv2[10];
+    const double fc = f(centr);
+    for (int j = 0; j < 10; ++j) {
+        const double absc = hlgth * sfp_gk::xgk21(j);
+        fv1[j] = f(centr - absc);
+        fv2[j] = f(centr + absc);
+    }
+    combine21(fc, fv1, fv2, hlgth, v);
+}
+
+// the 15-point rule from the node values of the transformed integrand
+SFP_HD void combine15(double fc, const double* fv1, const double* fv2, double hlgth, RuleValue& v) {
     double resg = sfp_gk::wg15(3) * fc;
     double resk = sfp_gk::wgk15(7) * fc;
-    resabs = fabs(resk);
+    double resabs = fabs(resk);
     for (int j = 0; j < 7; ++j) {
-        const double absc = hlgth * sfp_gk::xgk15(j);
-        const double absc1 = centr - absc, absc2 = centr + absc;
-        const double t1 = bound + (1.0 - absc1) / absc1, t2 = bound + (1.0 - absc2) / absc2;
-        const double f1 = (f(t1) / absc1) / absc1, f2 = (f(t2) / absc2) / absc2;
-        fv1[j] = f1;
-        fv2[j] = f2;
+        const double f1 = fv1[j], f2 = fv2[j];
         const double fsum = f1 + f2;
         if (j & 1) resg += sfp_gk::wg15(j >> 1) * fsum;
         resk += sfp_gk::wgk15(j) * fsum;
         resabs += sfp_gk::wgk15(j) * (fabs(f1) + fabs(f2));
     }
     const double reskh = resk * 0.5;
-    resasc = sfp_gk::wgk15(7) * fabs(fc - reskh);
+    double resasc = sfp_gk::wgk15(7) * fabs(fc - reskh);
     for (int j = 0; j < 7; ++j) resasc += sfp_gk::wgk15(j) * (fabs(fv1[j] - reskh) + fabs(fv2[j] - reskh));
-    result = resk * hlgth;
-    resasc *= hlgth;
-    resabs *= hlgth;
-    abserr = rule_error(fabs((resk - resg) * hlgth), resabs, resasc);
+    v.result = resk * hlgth;
+    v.resasc = resasc * hlgth;
+    v.resabs = resabs * hlgth;
+    v.abserr = rule_error(fabs((resk - resg) * hlgth), v.resabs, v.resasc);
+}
+
+// f over [bound, inf) at t in (0, 1]: x = bound + (1 - t) / t, dx = dt / t^2
+template <class F>
+SFP_HD double transformed(const F& f, double bound, double t) {
+    return (f(bound + (1.0 - t) / t) / t) / t;
+}
+
+// 15-point Gauss-Kronrod on [a, b] of (0, 1] for the integral of f over
+// [bound, inf)
+template <class F>
+SFP_HD void gk15i(const F& f, double bound, double a, double b, RuleValue& v) {
+    const double centr = 0.5 * (a + b), hlgth = 0.5 * (b - a);
+    double fv1[7], fv2[7];
+    const double fc = transformed(f, bound, centr);
+    for (int j = 0; j < 7; ++j) {
+        const double absc = hlgth * sfp_gk::xgk15(j);
+        fv1[j] = transformed(f, bound, centr - absc);
+        fv2[j] = transformed(f, bound, centr + absc);
+    }
+    combine15(fc, fv1, fv2, hlgth, v);
 }
 
 // Wynn's epsilon algorithm (QUADPACK qelg).  epstab[0..n-1] holds the
@@ -267,6 +289,28 @@ SFP_HD void qpsrt(int limit, int last, int& maxerr, double& ermax, const double*
     ermax = elist[maxerr - 1];
 }
 
+// The rule on one subinterval, and on the two halves of a bisected one, as
+// qag_core calls them: `bound` is QAGI's lower limit.  A functor whose values
+// are computed by a group of threads together (sfp_tables.cu) has overloads
+// of these two that spread the nodes over the group.
+template <bool INF>
+struct Interval {};  // tag: QAGI's transformed interval, or QAGS's finite one
+
+template <class F>
+SFP_HD void rule_one(Interval<false>, const F& f, double, double a, double b, RuleValue& v) {
+    gk21(f, a, b, v);
+}
+template <class F>
+SFP_HD void rule_one(Interval<true>, const F& f, double bound, double a, double b, RuleValue& v) {
+    gk15i(f, bound, a, b, v);
+}
+template <bool INF, class F>
+SFP_HD void rule_two(Interval<INF> tag, const F& f, double bound, double a1, double b1, double a2, double b2,
+                     RuleValue& v1, RuleValue& v2) {
+    rule_one(tag, f, bound, a1, b1, v1);
+    rule_one(tag, f, bound, a2, b2, v2);
+}
+
 // QAGS (rule 21, finite [a, b]) and QAGI (rule 15 after the transform,
 // [a, inf)); returns the result (abserr and ier through references)
 template <bool INF, class F>
@@ -285,8 +329,14 @@ SFP_HD double qag_core(const F& f, double a, double b, double epsabs, double eps
     elist[0] = 0.0;
     iord[0] = 0;
     double defabs, resabs;
-    if (INF) gk15i(f, a, lo, hi, result, abserr, defabs, resabs);
-    else gk21(f, lo, hi, result, abserr, defabs, resabs);
+    {
+        RuleValue v;
+        rule_one(Interval<INF>{}, f, a, lo, hi, v);
+        result = v.result;
+        abserr = v.abserr;
+        defabs = v.resabs;
+        resabs = v.resasc;
+    }
     double dres = fabs(result);
     double errbnd = dmax(epsabs, epsrel * dres);
     int last = 1;
@@ -314,14 +364,10 @@ SFP_HD double qag_core(const F& f, double a, double b, double epsabs, double eps
         const double a1 = alist[maxerr - 1], b1 = 0.5 * (alist[maxerr - 1] + blist[maxerr - 1]);
         const double a2 = b1, b2 = blist[maxerr - 1];
         const double erlast = errmax;
-        double area1, error1, area2, error2, defab1, defab2;
-        if (INF) {
-            gk15i(f, a, a1, b1, area1, error1, resabs, defab1);
-            gk15i(f, a, a2, b2, area2, error2, resabs, defab2);
-        } else {
-            gk21(f, a1, b1, area1, error1, resabs, defab1);
-            gk21(f, a2, b2, area2, error2, resabs, defab2);
-        }
+        RuleValue v1, v2;
+        rule_two(Interval<INF>{}, f, a, a1, b1, a2, b2, v1, v2);
+        const double area1 = v1.result, error1 = v1.abserr, defab1 = v1.resasc;
+        const double area2 = v2.result, error2 = v2.abserr, defab2 = v2.resasc;
         const double area12 = area1 + area2, erro12 = error1 + error2;
         errsum = errsum + erro12 - errmax;
         area = area + area12 - rlist[maxerr - 1];

@@ -21,8 +21,9 @@ struct AiFn {
     SFP_HD double operator()(double x) const { return sfp_airy::Ai(x); }
 };
 
-// int_Ai and Ai' at z
-SFP_HD void airy_terms(double z, double& ia, double& aip) {
+// int_Ai and Ai' at z (Fn: Ai as the integrand, evaluated by one thread or by a group)
+template <class Fn>
+SFP_HD void airy_terms_by(const Fn& fn, double z, double& ia, double& aip) {
     if (z >= sfp_airy::kAiryZero) {
         ia = 0.0;
         aip = 0.0;
@@ -30,11 +31,13 @@ SFP_HD void airy_terms(double z, double& ia, double& aip) {
     }
     double ai;
     sfp_airy::airy(z, ai, aip);
-    ia = sfp_quad::quad_inf(AiFn{}, z);
+    ia = sfp_quad::quad_inf(fn, z);
 }
+SFP_HD void airy_terms(double z, double& ia, double& aip) { airy_terms_by(AiFn{}, z, ia, aip); }
 
 // the differential rate of one chi row (kind 0: photon emission, 1: pair creation)
-struct RateFn {
+template <class Fn>
+struct RateFnBy {
     double chi, factor;
     int kind;
     SFP_HD double operator()(double delta) const {
@@ -45,11 +48,12 @@ struct RateFn {
         if (kind == 0) z = pow(chi_part / chi / chi_rest, 2.0 / 3.0);
         else z = pow(chi / chi_part / chi_rest, 2.0 / 3.0);
         double ia, aip;
-        airy_terms(z, ia, aip);
+        airy_terms_by(Fn{}, z, ia, aip);
         const double chi_g = kind == 0 ? chi_part : chi;
         const double s = kind == 0 ? 2.0 / z + chi_g * sqrt(z) : 2.0 / z - chi_g * sqrt(z);
         return factor * (ia + s * aip);
     }
 };
+using RateFn = RateFnBy<AiFn>;
 
 }  // namespace sfp_tab
