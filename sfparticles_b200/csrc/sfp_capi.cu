@@ -365,20 +365,12 @@ __global__ void k_inv_gamma(const double* __restrict__ ux, const double* __restr
 // interval early for the rounding of z, and the result is multiplied by 4
 // for the rounding of the device's float32 and float64 rate arithmetic.
 // The last bin, and any run without rejection-sampling tables, never skips.
-__global__ void k_pair_bound(const double* __restrict__ iA, const double* __restrict__ dA, int zN, double zmax,
-                             float* __restrict__ out) {
-    const int k = threadIdx.x;
-    if (k >= SFP_PAIR_BOUND_BINS) return;
-    if (zN < 2 || !iA || !dA || k == SFP_PAIR_BOUND_BINS - 1) {
-        out[k] = __int_as_float(0x7f800000);
-        return;
-    }
+__device__ float pair_bound_of(const double* __restrict__ iA, const double* __restrict__ dA, int zN, double zmax,
+                               int k) {
+    if (zN < 2 || !iA || !dA || k == SFP_PAIR_BOUND_BINS - 1) return __int_as_float(0x7f800000);
     const double chi = (double)__uint_as_float((unsigned int)(k + SFP_PAIR_BOUND_BASE + 1) << 20);
     const double zmin = pow(4.0 / chi, 2.0 / 3.0);
-    if (zmin * (1.0 - 1e-4) > zmax) {  // every z is beyond the table: rate 0
-        out[k] = 0.0f;
-        return;
-    }
+    if (zmin * (1.0 - 1e-4) > zmax) return 0.0f;  // every z is beyond the table: rate 0
     const double dz = zmax / (double)(zN - 1);
     long long j0 = (long long)floor(zmin / dz) - 1;
     if (j0 < 0) j0 = 0;
@@ -391,7 +383,26 @@ __global__ void k_pair_bound(const double* __restrict__ iA, const double* __rest
         b = fmax(b, ia + (dpos > 0.0 ? 2.0 / zl * dpos : 0.0) + chi * sqrt(zr) * dabs);
     }
     const double factor = ((sfp::kAlpha * sfp::kMe) * (sfp::kC * sfp::kC)) / sfp::kHbar;
-    out[k] = __double2float_ru(4.0 * factor * b);
+    return __double2float_ru(4.0 * factor * b);
+}
+
+// the bounds, and (pmax, if given) their prefix maximum, which every photon
+// launch reads
+__global__ void k_pair_bound(const double* __restrict__ iA, const double* __restrict__ dA, int zN, double zmax,
+                             float* __restrict__ out, float* __restrict__ pmax) {
+    __shared__ float s_m[SFP_PAIR_BOUND_BINS];
+    const int k = threadIdx.x;
+    const float b = pair_bound_of(iA, dA, zN, zmax, k);
+    out[k] = b;
+    if (!pmax) return;
+    s_m[k] = fmaxf(0.0f, b);
+    for (int o = 1; o < SFP_PAIR_BOUND_BINS; o <<= 1) {
+        __syncthreads();
+        const float m = k >= o ? fmaxf(s_m[k], s_m[k - o]) : s_m[k];
+        __syncthreads();
+        s_m[k] = m;
+    }
+    pmax[k] = s_m[k];
 }
 
 }  // namespace
@@ -401,7 +412,7 @@ int sfp_set_error(int code, const std::string& msg) { return fail(code, msg); }
 extern "C" int sfp_pair_rate_bound(const double* int_ai, const double* aip, int z_n, double z_max, float* out,
                                    void* stream) {
     if (!out || (z_n >= 2 && (!int_ai || !aip))) return fail(SFP_EINVAL, "sfp_pair_rate_bound: NULL argument");
-    k_pair_bound<<<1, SFP_PAIR_BOUND_BINS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(int_ai, aip, z_n, z_max, out);
+    k_pair_bound<<<1, SFP_PAIR_BOUND_BINS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(int_ai, aip, z_n, z_max, out, nullptr);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(SFP_ECUDA, std::string("sfp_pair_rate_bound: ") + cudaGetErrorString(e));
     return SFP_OK;
@@ -777,10 +788,12 @@ int sfp_inv_gamma(const double* ux, const double* uy, const double* uz, double* 
 
 // ================================ runs =======================================
 //
-// One step = book(prepare) + massive + photon [+ scan + appends] launches on
-// the run's stream.  The massive and photon kernels are persistent grids that
-// take warp tiles by ticket; the scan is one block; the appends kernel is a
-// grid over both groups' tile counters.
+// One step = massive + photon [+ appends] launches on the run's stream (a
+// call's first step is prepared by a bookkeeping launch).  The massive and
+// photon kernels are persistent grids that take warp tiles by ticket; the
+// appends kernel is a grid over both groups' tile counters; the event scan
+// and the bookkeeping of the next step run in the last block of the photon
+// (or only) group launch.
 
 #define SFP_SUPER_TILE_HOST 64
 // the any-tile kernels (..._t) of each form: ring stages and blocks per SM
@@ -797,17 +810,134 @@ struct sfp_group_host {
     long long* d_start = nullptr;
 };
 
+// Device memory and streams that a destroyed run leaves for the next one.  A
+// run's bookkeeping is one block of a few hundred KB: as seventeen
+// cudaMalloc / cudaFree calls, a stream and two events it cost 1.2 ms per
+// run (create 0.7, destroy 0.45; several times that on a busy host), against
+// 4 ms for 32 steps of 1e6 particles.  Bounded: at most kPoolBlocks blocks
+// and kPoolBytes bytes, and as many streams, over all devices; the rest goes
+// back to the driver at once, and everything does when an allocation fails.
+// A run gives its block and stream back only once its stream is idle, so no
+// work in flight can reach them; the lists are under one lock.
+namespace {
+
+constexpr size_t kPoolBlocks = 8, kPoolBytes = 32u << 20;
+
+struct run_block {
+    int dev = 0;
+    void* p = nullptr;
+    size_t bytes = 0;
+};
+struct run_stream {
+    int dev = 0;
+    cudaStream_t s = nullptr;
+    cudaEvent_t in = nullptr, out = nullptr;
+};
+std::mutex g_pool_mu;
+std::vector<run_block> g_blocks;
+std::vector<run_stream> g_streams;
+
+int device_now() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
+}
+
+bool block_get(size_t bytes, run_block* out) {
+    const int dev = device_now();
+    {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        size_t best = g_blocks.size();
+        for (size_t k = 0; k < g_blocks.size(); ++k)
+            if (g_blocks[k].dev == dev && g_blocks[k].bytes >= bytes &&
+                (best == g_blocks.size() || g_blocks[k].bytes < g_blocks[best].bytes))
+                best = k;
+        if (best < g_blocks.size()) {
+            *out = g_blocks[best];
+            g_blocks.erase(g_blocks.begin() + (long)best);
+            return true;
+        }
+    }
+    size_t n = 1u << 18;
+    while (n < bytes) n *= 2;
+    out->dev = dev;
+    out->bytes = n;
+    if (cudaMalloc(&out->p, n) == cudaSuccess) return true;
+    cudaGetLastError();
+    std::vector<run_block> old;
+    {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        old.swap(g_blocks);
+    }
+    for (run_block& b : old) cudaFree(b.p);
+    out->bytes = bytes;
+    if (cudaMalloc(&out->p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    out->p = nullptr;
+    return false;
+}
+
+void block_put(const run_block& b) {
+    if (!b.p) return;
+    {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        size_t held = b.bytes;
+        for (const run_block& o : g_blocks) held += o.bytes;
+        if (g_blocks.size() < kPoolBlocks && held <= kPoolBytes) {
+            g_blocks.push_back(b);
+            return;
+        }
+    }
+    cudaFree(b.p);
+}
+
+bool stream_get(run_stream* out) {
+    const int dev = device_now();
+    {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        for (size_t k = 0; k < g_streams.size(); ++k)
+            if (g_streams[k].dev == dev) {
+                *out = g_streams[k];
+                g_streams.erase(g_streams.begin() + (long)k);
+                return true;
+            }
+    }
+    out->dev = dev;
+    return cudaStreamCreateWithFlags(&out->s, cudaStreamNonBlocking) == cudaSuccess &&
+           cudaEventCreateWithFlags(&out->in, cudaEventDisableTiming) == cudaSuccess &&
+           cudaEventCreateWithFlags(&out->out, cudaEventDisableTiming) == cudaSuccess;
+}
+
+void stream_put(const run_stream& st, bool whole) {
+    if (whole) {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        if (g_streams.size() < kPoolBlocks) {
+            g_streams.push_back(st);
+            return;
+        }
+    }
+    if (st.in) cudaEventDestroy(st.in);
+    if (st.out) cudaEventDestroy(st.out);
+    if (st.s) cudaStreamDestroy(st.s);
+}
+
+}  // namespace
+
 struct sfp_run {
     sfp_module* mod = nullptr;
+    std::vector<run_block> blocks;  // the run's bookkeeping; the first holds all that creation needs
+    size_t block_at = 0;            // bytes of the last block handed out
+    run_stream rs;
     void* cfield = nullptr;  // the module's sfp_cfield (runs of one instance), or NULL
     size_t cfield_bytes = 0;
     void* ckeys = nullptr;           // the module's sfp_ckeys: the instance seed's Philox round keys
-    unsigned int* d_keys = nullptr;  // those keys, formed at creation (20 words, device)
-    cudaKernel_t k_massive = nullptr, k_photon = nullptr, k_scan = nullptr, k_appends = nullptr, k_book = nullptr;
+    unsigned int* d_keys = nullptr;  // those keys (20 words, device)
+    unsigned int keys[20] = {};      // formed at creation
+    cudaKernel_t k_massive = nullptr, k_photon = nullptr, k_appends = nullptr, k_book = nullptr;
     cudaKernel_t k_massive_t = nullptr, k_photon_t = nullptr;  // any tile length
     cudaKernel_t k_sync = nullptr, k_epoch = nullptr;           // photon positions written out
     int grid_m = 0, grid_p = 0, grid_a = 0, grid_mt = 0, grid_pt = 0;
-    size_t smem_m = 0, smem_p = 0, smem_mt = 0, smem_pt = 0;
+    size_t smem_m = 0, smem_p = 0, smem_mt = 0, smem_pt = 0, smem_end = 0;
     std::vector<long long> nb_lo;  // lower bounds of the device's n_buffered (it only grows between reads)
     cudaStream_t s = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
@@ -820,6 +950,20 @@ struct sfp_run {
     sfp_group_host mg, pg;
     std::vector<int> dseg;
 };
+
+// `bytes` of the run's bookkeeping, 256-byte aligned, from its last block
+static int run_carve(sfp_run* r, size_t bytes, void** out) {
+    bytes = (bytes + 255) / 256 * 256;
+    if (r->blocks.empty() || r->block_at + bytes > r->blocks.back().bytes) {
+        run_block b;
+        if (!block_get(bytes, &b)) return fail(SFP_ENOMEM, "device memory of a run's bookkeeping");
+        r->blocks.push_back(b);
+        r->block_at = 0;
+    }
+    *out = static_cast<char*>(r->blocks.back().p) + r->block_at;
+    r->block_at += bytes;
+    return SFP_OK;
+}
 
 // tile counters a group needs at full capacity: each segment's longest
 // tiles plus the padding up to the next multiple of a super-tile, and at
@@ -841,23 +985,18 @@ static int group_alloc(sfp_run* r, sfp_group_dev& G, long long need) {
     const long long n_old = G.max_tiles, ns_old = n_old ? n_old / SFP_SUPER_TILE_HOST + 2 : 0;
     unsigned int *cnt = nullptr, *scnt = nullptr;
     long long* spre = nullptr;
-    if (cudaMalloc(&cnt, n * sizeof(unsigned int)) != cudaSuccess ||
-        cudaMalloc(&scnt, ns * sizeof(unsigned int)) != cudaSuccess ||
-        cudaMalloc(&spre, ns * sizeof(long long)) != cudaSuccess) {
-        cudaFree(cnt);
-        cudaFree(scnt);
-        cudaFree(spre);
-        return fail(SFP_ENOMEM, "cudaMalloc of the tile counters");
-    }
+    int rc;
+    if ((rc = run_carve(r, n * sizeof(unsigned int), (void**)&cnt)) ||
+        (rc = run_carve(r, ns * sizeof(unsigned int), (void**)&scnt)) ||
+        (rc = run_carve(r, ns * sizeof(long long), (void**)&spre)))
+        return rc;
     if (n_old) {
         SFP_CUDA(cudaMemcpyAsync(cnt, G.tile_cnt, n_old * sizeof(unsigned int), cudaMemcpyDeviceToDevice, r->s));
         SFP_CUDA(cudaMemcpyAsync(scnt, G.super_cnt, ns_old * sizeof(unsigned int), cudaMemcpyDeviceToDevice, r->s));
         SFP_CUDA(cudaMemcpyAsync(spre, G.super_pre, ns_old * sizeof(long long), cudaMemcpyDeviceToDevice, r->s));
         SFP_CUDA(cudaStreamSynchronize(r->s));
     }
-    cudaFree(G.tile_cnt);
-    cudaFree(G.super_cnt);
-    cudaFree(G.super_pre);
+    // (outgrown counters stay in the run's blocks until it ends)
     G.tile_cnt = cnt;
     G.super_cnt = scnt;
     G.super_pre = spre;
@@ -945,6 +1084,7 @@ static int run_upload(sfp_run* r, const sfp_instance* inst, const int64_t* n_buf
 }
 
 // the kernel's dynamic shared memory limit, raised to at least `need` bytes
+// (read afresh: another thread's run may have raised it since)
 static cudaError_t raise_dynamic_smem(const void* k, size_t need) {
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, k);
@@ -1013,7 +1153,6 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     if ((rc = module_kernel(m, km.c_str(), &r->k_massive)) || (rc = module_kernel(m, kp.c_str(), &r->k_photon)) ||
         (rc = module_kernel(m, kmt.c_str(), &r->k_massive_t)) || (rc = module_kernel(m, kpt.c_str(), &r->k_photon_t)) ||
         (rc = module_kernel(m, ka.c_str(), &r->k_appends)) ||
-        (rc = module_kernel(m, "sfp_scan_kernel", &r->k_scan)) ||
         (rc = module_kernel(m, ksy.c_str(), &r->k_sync)) || (rc = module_kernel(m, "sfp_epoch_kernel", &r->k_epoch)) ||
         (rc = module_kernel(m, "sfp_book_kernel", &r->k_book))) {
         delete r;
@@ -1049,12 +1188,7 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
                 k0 += 0x9E3779B9u;
                 k1 += 0xBB67AE85u;
             }
-            if (cudaMalloc(&r->d_keys, sizeof(keys)) != cudaSuccess ||
-                cudaMemcpy(r->d_keys, keys, sizeof(keys), cudaMemcpyHostToDevice) != cudaSuccess) {
-                cudaFree(r->d_keys);
-                delete r;
-                return fail(SFP_ENOMEM, "sfp_run_create: Philox key array");
-            }
+            std::copy(keys, keys + 20, r->keys);
             r->ckeys = ck;
         } else {
             cudaGetLastError();  // no such symbol: parameters are read from global memory
@@ -1064,10 +1198,10 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
         sfp_run_destroy(r);
         return code;
     };
-    if (cudaStreamCreateWithFlags(&r->s, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&r->ev_in, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&r->ev_out, cudaEventDisableTiming) != cudaSuccess)
-        return cleanup(fail(SFP_ECUDA, "stream/event creation failed"));
+    if (!stream_get(&r->rs)) return cleanup(fail(SFP_ECUDA, "stream/event creation failed"));
+    r->s = r->rs.s;
+    r->ev_in = r->rs.in;
+    r->ev_out = r->rs.out;
     sfp_run_dev& h = r->h;
     h.n_seg = n_seg;
     h.n_inst = n_inst;
@@ -1085,8 +1219,16 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     h.rs = cfg->rs;
     h.od_photon = cfg->od_photon;
     h.od_pair = cfg->od_pair;
+    {   // one block for all of it: the arrays below and both groups' tile counters
+        const long long tiles = tiles_for(r, r->mg.seg) + tiles_for(r, r->pg.seg);
+        const size_t want = (size_t)n_seg * (sizeof(sfp_segment) + sizeof(sfp_end_seg) + 128) +
+                            (size_t)n_inst * sizeof(sfp_instance) + (size_t)(tiles + tiles / 4) * 5 + (1u << 16);
+        run_block blk;
+        if (!block_get(want, &blk)) return cleanup(fail(SFP_ENOMEM, "device memory of a run's bookkeeping"));
+        r->blocks.push_back(blk);
+    }
 #define ALLOC(ptr, bytes) \
-    if (cudaMalloc((void**)&(ptr), (bytes)) != cudaSuccess) return cleanup(fail(SFP_ENOMEM, "cudaMalloc " #ptr))
+    if ((rc = run_carve(r, (bytes), (void**)&(ptr)))) return cleanup(rc)
     sfp_segment* dseg;
     sfp_instance* dinst;
     int* dd;
@@ -1097,8 +1239,8 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     ALLOC(r->mg.d_seg, (r->mg.seg.size() + 1) * sizeof(int));
     ALLOC(r->pg.d_seg, (r->pg.seg.size() + 1) * sizeof(int));
     ALLOC(dd, (r->dseg.size() + 1) * sizeof(int));
-    ALLOC(r->mg.d_start, (r->mg.seg.size() + 1) * sizeof(long long));
-    ALLOC(r->pg.d_start, (r->pg.seg.size() + 1) * sizeof(long long));
+    ALLOC(r->mg.d_start, 2 * (r->mg.seg.size() + 1) * sizeof(long long));
+    ALLOC(r->pg.d_start, 2 * (r->pg.seg.size() + 1) * sizeof(long long));
     h.mg.seg = r->mg.d_seg;
     h.pg.seg = r->pg.d_seg;
     h.mg.tile_start = r->mg.d_start;
@@ -1106,15 +1248,20 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     h.dseg = dd;
     ALLOC(h.n_buffered, n_seg * sizeof(long long));
     ALLOC(h.appended, n_seg * sizeof(unsigned long long));
-    ALLOC(h.n_buf_step, n_seg * sizeof(long long));
+    ALLOC(h.n_buf_step, 2 * n_seg * sizeof(long long));
+    ALLOC(h.end_seg, n_seg * sizeof(sfp_end_seg));
+    ALLOC(h.end_app, n_seg * sizeof(unsigned long long));
+    ALLOC(h.end_nb, n_seg * sizeof(long long));
     ALLOC(h.st, sizeof(sfp_step_state));
     ALLOC(r->d, sizeof(sfp_run_dev));
+    ALLOC(r->d_keys, sizeof(r->keys));
     float* pb;
-    ALLOC(pb, SFP_PAIR_BOUND_BINS * sizeof(float));
+    ALLOC(pb, 2 * SFP_PAIR_BOUND_BINS * sizeof(float));
     h.pair_bound = pb;
 #undef ALLOC
     k_pair_bound<<<1, SFP_PAIR_BOUND_BINS, 0, r->s>>>(cfg->qed == SFP_QED_REJECTION ? cfg->rs.int_Ai : nullptr,
-                                                      cfg->rs.Aip, cfg->rs.z_N, cfg->rs.z_max, pb);
+                                                      cfg->rs.Aip, cfg->rs.z_N, cfg->rs.z_max, pb,
+                                                      pb + SFP_PAIR_BOUND_BINS);
     if (cudaGetLastError() != cudaSuccess) return cleanup(fail(SFP_ECUDA, "pair-rate bound table"));
     if ((!r->mg.seg.empty() && cudaMemcpyAsync(r->mg.d_seg, r->mg.seg.data(), r->mg.seg.size() * sizeof(int),
                                                cudaMemcpyHostToDevice, r->s) != cudaSuccess) ||
@@ -1122,8 +1269,9 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
                                                cudaMemcpyHostToDevice, r->s) != cudaSuccess) ||
         (!r->dseg.empty() &&
          cudaMemcpyAsync(dd, r->dseg.data(), r->dseg.size() * sizeof(int), cudaMemcpyHostToDevice, r->s) != cudaSuccess) ||
-        cudaMemsetAsync(r->mg.d_start, 0, (r->mg.seg.size() + 1) * sizeof(long long), r->s) != cudaSuccess ||
-        cudaMemsetAsync(r->pg.d_start, 0, (r->pg.seg.size() + 1) * sizeof(long long), r->s) != cudaSuccess ||
+        cudaMemcpyAsync(r->d_keys, r->keys, sizeof(r->keys), cudaMemcpyHostToDevice, r->s) != cudaSuccess ||
+        cudaMemsetAsync(r->mg.d_start, 0, 2 * (r->mg.seg.size() + 1) * sizeof(long long), r->s) != cudaSuccess ||
+        cudaMemsetAsync(r->pg.d_start, 0, 2 * (r->pg.seg.size() + 1) * sizeof(long long), r->s) != cudaSuccess ||
         cudaMemsetAsync(h.appended, 0, n_seg * sizeof(unsigned long long), r->s) != cudaSuccess)
         return cleanup(fail(SFP_ECUDA, "segment lists upload"));
     sfp_step_state st0{};
@@ -1153,6 +1301,9 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     r->smem_p = (size_t)h.ring_off + warps * stages * ((6 + od) * 256 + 32);
     r->smem_mt = (size_t)h.m_ring_off + warps * SFP_T_M_STAGES * (size_t)h.m_stage_bytes;
     r->smem_pt = (size_t)h.ring_off + warps * SFP_T_P_STAGES * ((6 + od) * 256 + 32);
+    // the end of a step uses the event launches' shared memory
+    r->smem_end = sizeof(sfp_end_smem);
+    for (size_t* q : {&r->smem_m, &r->smem_p, &r->smem_mt, &r->smem_pt}) *q = std::max(*q, r->smem_end);
     if ((rc = run_alloc_tiles(r))) return cleanup(rc);
     if ((rc = run_upload(r, inst, n_buffered))) return cleanup(rc);
     const size_t cap = 200 * 1024;
@@ -1164,7 +1315,8 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     if (raise_dynamic_smem((const void*)r->k_massive, r->smem_m) != cudaSuccess ||
         raise_dynamic_smem((const void*)r->k_photon, r->smem_p) != cudaSuccess ||
         raise_dynamic_smem((const void*)r->k_massive_t, r->smem_mt) != cudaSuccess ||
-        raise_dynamic_smem((const void*)r->k_photon_t, r->smem_pt) != cudaSuccess)
+        raise_dynamic_smem((const void*)r->k_photon_t, r->smem_pt) != cudaSuccess ||
+        raise_dynamic_smem((const void*)r->k_book, r->smem_end) != cudaSuccess)
         return cleanup(fail(SFP_ECUDA, "cannot raise dynamic shared memory"));
     r->grid_m = persistent_grid(r->k_massive, r->smem_m, minb);
     r->grid_p = persistent_grid(r->k_photon, r->smem_p, pminb);
@@ -1218,17 +1370,32 @@ struct cfield_guard {
     }
 };
 
-// one step: book(prepare), massive, photon, scan + appends; ev (6 events)
-// brackets the massive, the photon and the scan + appends kernels when given.
+// flags of the end of a step (sfp_step.cuh: SFP_PREP ... SFP_SCAN)
+enum { PREP = 1, PREP_M = 2, PREP_P = 4, FOLD = 8, SCAN = 16 };
+
+// the bookkeeping of a call's first step (PREP), or the fold of a resumed one
+static int launch_book(sfp_run* r, int flags) {
+    void* a[] = {&r->d, &flags};
+    SFP_CUDA(cudaLaunchKernel((const void*)r->k_book, dim3(1), dim3(256), a, r->smem_end, r->s));
+    return SFP_OK;
+}
+
+static int prep_flags(bool mlong, bool plong) { return PREP | (mlong ? PREP_M : 0) | (plong ? PREP_P : 0); }
+
+// one step: massive, photon, appends; the last block of the last event launch
+// (photon, or massive in a run without photons) scans the events, folds the
+// step and prepares the next one.  ev (6 events) brackets the massive, the
+// photon and the appends kernels when given.
 // mlong / plong: the group's steps all have SFP_TILE_MAX-long tiles, run by
 // the autotuned long-tile kernel; else by the any-tile kernel
 static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, bool plong) {
-    int prep = 1 | (mlong ? 2 : 0) | (plong ? 4 : 0);  // the book kernel checks the tiles the launches assume
-    void* a_book[] = {&r->d, &prep};
-    void* a[] = {&r->d};
-    SFP_CUDA(cudaLaunchKernel((const void*)r->k_book, dim3(1), dim3(256), a_book, 0, s));
+    const bool has_m = !r->mg.seg.empty(), has_p = !r->pg.seg.empty(), has_a = !r->dseg.empty();
+    // the bookkeeping checks the tiles that the next launches assume
+    int end = FOLD | prep_flags(mlong, plong) | (has_a ? SCAN : 0);
+    int none = 0;
     if (ev) SFP_CUDA(cudaEventRecord(ev[0], s));
-    if (!r->mg.seg.empty()) {
+    if (has_m) {
+        void* a[] = {&r->d, has_p ? &none : &end};
         if (mlong)
             SFP_CUDA(cudaLaunchKernel((const void*)r->k_massive, dim3(r->grid_m), dim3(SFP_TILE_HOST), a, r->smem_m, s));
         else
@@ -1237,7 +1404,8 @@ static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, 
     }
     if (ev) SFP_CUDA(cudaEventRecord(ev[1], s));
     if (ev) SFP_CUDA(cudaEventRecord(ev[2], s));
-    if (!r->pg.seg.empty()) {
+    if (has_p) {
+        void* a[] = {&r->d, &end};
         if (plong)
             SFP_CUDA(cudaLaunchKernel((const void*)r->k_photon, dim3(r->grid_p), dim3(SFP_TILE_HOST), a, r->smem_p, s));
         else
@@ -1246,18 +1414,11 @@ static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, 
     }
     if (ev) SFP_CUDA(cudaEventRecord(ev[3], s));
     if (ev) SFP_CUDA(cudaEventRecord(ev[4], s));
-    if (!r->dseg.empty()) {
-        SFP_CUDA(cudaLaunchKernel((const void*)r->k_scan, dim3(1), dim3(1024), a, 0, s));
+    if (has_a) {
+        void* a[] = {&r->d};
         SFP_CUDA(cudaLaunchKernel((const void*)r->k_appends, dim3(r->grid_a), dim3(SFP_TILE_HOST), a, 0, s));
     }
     if (ev) SFP_CUDA(cudaEventRecord(ev[5], s));
-    return SFP_OK;
-}
-
-static int launch_fold(sfp_run* r) {
-    int prep = 0;
-    void* a_book[] = {&r->d, &prep};
-    SFP_CUDA(cudaLaunchKernel((const void*)r->k_book, dim3(1), dim3(256), a_book, 0, r->s));
     return SFP_OK;
 }
 
@@ -1271,6 +1432,7 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
     if (const int rc0 = cg.put()) return rc0;
     int64_t done = 0;
     const bool ml = long_tiles(r, r->mg.seg), pl = long_tiles(r, r->pg.seg);
+    if (const int rc0 = launch_book(r, prep_flags(ml, pl))) return rc0;
     if (graph_chunk > 0 && nsteps >= graph_chunk) {
         const int key = graph_chunk * 4 + (ml ? 2 : 0) + (pl ? 1 : 0);
         auto it = r->graphs.find(key);
@@ -1294,9 +1456,7 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
         int rc = launch_unit(r, r->s, nullptr, ml, pl);
         if (rc) return rc;
     }
-    int rc = launch_fold(r);
-    if (rc) return rc;
-    if ((rc = cg.done())) return rc;
+    if (const int rc = cg.done()) return rc;
     SFP_CUDA(cudaEventRecord(r->ev_out, r->s));
     SFP_CUDA(cudaStreamWaitEvent(cs, r->ev_out, 0));
     return SFP_OK;
@@ -1315,8 +1475,8 @@ int sfp_run_steps_timed(sfp_run* r, int64_t nsteps, float* kernel_ms, void* stre
     for (auto& e : ev)
         if (cudaEventCreate(&e) != cudaSuccess) rc = fail(SFP_ECUDA, "cudaEventCreate");
     const bool ml = long_tiles(r, r->mg.seg), pl = long_tiles(r, r->pg.seg);
+    if (rc == SFP_OK) rc = launch_book(r, prep_flags(ml, pl));
     for (int64_t k = 0; k < nsteps && rc == SFP_OK; ++k) rc = launch_unit(r, r->s, &ev[6 * k], ml, pl);
-    if (rc == SFP_OK) rc = launch_fold(r);
     if (rc == SFP_OK) rc = cg.done();
     if (rc == SFP_OK && cudaStreamSynchronize(r->s) != cudaSuccess) rc = fail(SFP_ECUDA, "synchronize");
     const bool has[3] = {!r->mg.seg.empty(), !r->pg.seg.empty(), !r->dseg.empty()};
@@ -1388,32 +1548,34 @@ int sfp_run_clear_halt(sfp_run* r, void* stream) {
 int sfp_run_pending_need(sfp_run* r, int64_t* need) {
     if (!r || !need) return fail(SFP_EINVAL, "sfp_run_pending_need: NULL argument");
     sfp_step_state st;
-    std::vector<long long> nb(r->n_seg), ns(r->n_seg);
+    std::vector<long long> nb(r->n_seg), ns(2 * r->n_seg);
     std::vector<unsigned long long> ap(r->n_seg);
     SFP_CUDA(cudaMemcpyAsync(&st, r->h.st, sizeof(st), cudaMemcpyDeviceToHost, r->s));
     SFP_CUDA(cudaMemcpyAsync(nb.data(), r->h.n_buffered, r->n_seg * sizeof(long long), cudaMemcpyDeviceToHost, r->s));
-    SFP_CUDA(cudaMemcpyAsync(ns.data(), r->h.n_buf_step, r->n_seg * sizeof(long long), cudaMemcpyDeviceToHost, r->s));
+    SFP_CUDA(cudaMemcpyAsync(ns.data(), r->h.n_buf_step, 2 * r->n_seg * sizeof(long long), cudaMemcpyDeviceToHost,
+                             r->s));
     SFP_CUDA(cudaMemcpyAsync(ap.data(), r->h.appended, r->n_seg * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                              r->s));
     SFP_CUDA(cudaStreamSynchronize(r->s));
-    for (int s = 0; s < r->n_seg; ++s) need[s] = st.append_wait ? ns[s] + (long long)ap[s] : nb[s];
+    for (int s = 0; s < r->n_seg; ++s) need[s] = st.append_wait ? ns[st.cur * r->n_seg + s] + (long long)ap[s] : nb[s];
     return SFP_OK;
 }
 
 int sfp_run_resume(sfp_run* r, void* stream) {
     if (!r) return fail(SFP_EINVAL, "sfp_run_resume: NULL run");
     sfp_step_state st;
-    std::vector<long long> ns(r->n_seg);
+    std::vector<long long> ns(2 * r->n_seg);
     std::vector<unsigned long long> ap(r->n_seg);
     SFP_CUDA(cudaMemcpyAsync(&st, r->h.st, sizeof(st), cudaMemcpyDeviceToHost, r->s));
-    SFP_CUDA(cudaMemcpyAsync(ns.data(), r->h.n_buf_step, r->n_seg * sizeof(long long), cudaMemcpyDeviceToHost, r->s));
+    SFP_CUDA(cudaMemcpyAsync(ns.data(), r->h.n_buf_step, 2 * r->n_seg * sizeof(long long), cudaMemcpyDeviceToHost,
+                             r->s));
     SFP_CUDA(cudaMemcpyAsync(ap.data(), r->h.appended, r->n_seg * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                              r->s));
     SFP_CUDA(cudaStreamSynchronize(r->s));
     if (!st.append_wait) return SFP_OK;
     // the appends kernel runs only when every destination holds its children
     for (int c : r->dseg)
-        if (ns[c] + (long long)ap[c] > r->segs[c].capacity)
+        if (ns[st.cur * r->n_seg + c] + (long long)ap[c] > r->segs[c].capacity)
             return fail(SFP_EINVAL, "sfp_run_resume: segment " + std::to_string(c) +
                                         " still lacks room for the children of the stopped step");
     st.append_wait = 0;
@@ -1426,11 +1588,11 @@ int sfp_run_resume(sfp_run* r, void* stream) {
     SFP_CUDA(cudaStreamSynchronize(r->s));
     cfield_guard cg(r);
     if (const int rc0 = cg.put()) return rc0;
+    // fold the step, as its scan would have, then write its children
+    if (const int rc = launch_book(r, FOLD)) return rc;
     void* a[] = {&r->d};
     SFP_CUDA(cudaLaunchKernel((const void*)r->k_appends, dim3(r->grid_a), dim3(SFP_TILE_HOST), a, 0, r->s));
-    int rc = launch_fold(r);
-    if (rc) return rc;
-    if ((rc = cg.done())) return rc;
+    if (const int rc = cg.done()) return rc;
     SFP_CUDA(cudaEventRecord(r->ev_out, r->s));
     SFP_CUDA(cudaStreamWaitEvent(cs, r->ev_out, 0));
     return SFP_OK;
@@ -1438,30 +1600,13 @@ int sfp_run_resume(sfp_run* r, void* stream) {
 
 int sfp_run_destroy(sfp_run* r) {
     if (!r) return SFP_OK;
-    if (r->s) cudaStreamSynchronize(r->s);
+    const bool idle = r->s && cudaStreamSynchronize(r->s) == cudaSuccess;
     for (auto& kv : r->graphs) cudaGraphExecDestroy(kv.second);
-    cudaFree(r->d_keys);
-    cudaFree((void*)r->h.seg);
-    cudaFree((void*)r->h.inst);
-    cudaFree(r->mg.d_seg);
-    cudaFree(r->pg.d_seg);
-    cudaFree(r->mg.d_start);
-    cudaFree(r->pg.d_start);
-    cudaFree((void*)r->h.dseg);
-    cudaFree(r->h.n_buffered);
-    cudaFree(r->h.appended);
-    cudaFree(r->h.n_buf_step);
-    for (sfp_group_dev* G : {&r->h.mg, &r->h.pg}) {
-        cudaFree(G->tile_cnt);
-        cudaFree(G->super_cnt);
-        cudaFree(G->super_pre);
+    for (const run_block& b : r->blocks) {
+        if (idle) block_put(b);
+        else cudaFree(b.p);
     }
-    cudaFree(r->h.st);
-    cudaFree((void*)r->h.pair_bound);
-    cudaFree(r->d);
-    if (r->ev_in) cudaEventDestroy(r->ev_in);
-    if (r->ev_out) cudaEventDestroy(r->ev_out);
-    if (r->s) cudaStreamDestroy(r->s);
+    stream_put(r->rs, idle);
     delete r;
     return SFP_OK;
 }

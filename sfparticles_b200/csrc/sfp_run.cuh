@@ -1,7 +1,7 @@
 // sfp_run.cuh -- device-side layout of a fused-step run, shared by the host
 // C-ABI (nvcc) and the NVRTC-compiled step modules.
 //
-// A step runs four kernels after the bookkeeping kernel:
+// A step runs up to three kernels:
 //   massive -- warp tiles over the e+- (massive) segments, streamed through
 //              a ring of asynchronous copies: QED photon emission at t; an
 //              emitter is marked (pruned = 2) with its delta stored and is
@@ -9,14 +9,16 @@
 //              per-tile emission counts, summed per super-tile of 64;
 //   photon  -- warp tiles over the photon segments: pair creation (the
 //              converted photon is marked and its delta stored), photon
-//              push; per-tile event counts, summed per super-tile;
-//   scan    -- one block: exclusive scans of both groups' super-tile counts
-//              (segmented by instance, per append channel), the step's
-//              append counts, and the exact room check of every destination;
+//              push; per-tile event counts, summed per super-tile.  Its last
+//              block scans both groups' super-tile counts (segmented by
+//              instance, per append channel) into the step's append counts
+//              and checks the room of every destination exactly;
 //   appends -- photon children of the marked emitters (then their recoil
 //              and push) and e-/e+ children of the marked photons (pushed),
 //              each written at the slot the reference's find_event_index +
 //              create_* gives it.
+// The last block of the step's last launch folds the step's appends and
+// prepares the next step; a bookkeeping kernel prepares the first of a call.
 // Both groups' segments start at multiples of 64 tiles, so a super-tile
 // never spans two segments.  No kernel waits on another block: there is no
 // spin-wait anywhere in a step.
@@ -36,21 +38,28 @@
 #define SFP_TILE_MAX 1024
 #define SFP_TILE_TARGET 4096
 
-struct sfp_step_state {
-    double t;                   // time of the prepared / running step
-    long long step;             // steps completed
-    long long n_mtiles;         // massive-group tiles of the prepared step
+// what a step is planned with: its time and number, and each group's tiles
+struct sfp_step_plan {
+    double t;
+    long long step;
+    long long n_mtiles;         // massive-group tiles
     long long n_ptiles;         // photon-group tiles
+    int mtile;                  // particles per massive-group tile
+    int ptile;                  // particles per photon-group tile
+};
+
+struct sfp_step_state {
+    double t;                   // time of the next step
+    long long step;             // steps completed
+    sfp_step_plan plan[2];      // the next step's plan in slot `cur`, the last one's in the other
+    int cur;
     int mticket;                // next massive tile to hand out
     int pticket;                // next photon tile to hand out
     int skip;                   // 1: the prepared step must not run
     int halted;                 // sticky: a destination lacked room (host regrows, resumes)
     int error;                  // sticky device error (SFP_DEV_*)
-    int mtile;                  // particles per massive-group tile of the prepared step
-    int pending;                // a prepared step awaits folding
-    int append_wait;            // the prepared step stopped before writing its children (no room)
-    int ptile;                  // particles per photon-group tile of the prepared step
-    int pad0;
+    int blocks_done;            // blocks of the running launch that are done (sfp_last_block)
+    int append_wait;            // the step in slot `cur` stopped before writing its children (no room)
     long long particle_steps;   // sum over executed steps of all N_buffered
     // Photons fly straight: a photon segment stores each position as of the
     // start of step pos_epoch, and the photon at the start of step `step`
@@ -60,11 +69,36 @@ struct sfp_step_state {
     long long pos_epoch;
 };
 
+// a segment as the end of a step walks it (sfp_step_end)
+struct sfp_end_seg {
+    int super0;                 // first super-tile in the sequence of both groups'
+    int chain;                  // instance and group
+    int channel;
+    int dest0, dest1;           // segments that its events append to, or -1
+};
+
+// segments whose data sfp_step_end holds in shared memory; runs of more keep
+// them in the run's own scratch (end_seg, end_app, end_nb)
+#define SFP_END_SEGS 768
+// shared memory of sfp_step_end: the launch's dynamic shared memory, whose
+// tables and rings the block no longer needs (every launch that ends a step,
+// and sfp_book_kernel, has this much)
+struct sfp_end_smem {
+    uint4 wv[8];
+    unsigned int wh[8];
+    long long tiles[2], ps[8];
+    int tile[2];
+    int lacks, pad;
+    sfp_end_seg seg[SFP_END_SEGS];
+    unsigned long long app[SFP_END_SEGS];
+    long long nb[SFP_END_SEGS];
+};
+
 // one group of tiles (massive or photon): the tile map of its segments and
 // its per-tile / per-super-tile event counts
 struct sfp_group_dev {
     const int* seg;             // [n_seg] segment indices, in segment order
-    long long* tile_start;      // [n_seg + 1] first tile of each segment (multiples of 64)
+    long long* tile_start;      // [2][n_seg + 1] per plan slot: first tile of each segment (multiples of 64)
     unsigned int* tile_cnt;     // [max_tiles] events per tile
     unsigned int* super_cnt;    // [max_tiles / 64 + 2] events per super-tile
     long long* super_pre;       // [max_tiles / 64 + 2] exclusive prefix in its instance, per channel
@@ -98,12 +132,16 @@ struct sfp_run_dev {
     sfp_od_table od_pair;
     long long* n_buffered;        // [n_seg] authoritative buffered counts
     unsigned long long* appended; // [n_seg] children appended by the running step
-    long long* n_buf_step;        // [n_seg] counts at the start of the running step
+    long long* n_buf_step;        // [2][n_seg] per plan slot: counts at the start of the step
+    sfp_end_seg* end_seg;         // [n_seg] scratch of sfp_step_end for runs of many segments
+    unsigned long long* end_app;  // [n_seg]
+    long long* end_nb;            // [n_seg]
     const float* mlp_params;      // learned photon-energy sampler (optical depth), or NULL: the table
     sfp_step_state* st;
     // rejection sampling: per chi bin an upper bound of the pair rate over
     // every delta (SFP_PAIR_BOUND_BINS floats, the bins of sfp_pair_bin), so
-    // photons whose pair test no draw can pass skip the draw
+    // photons whose pair test no draw can pass skip the draw; then its prefix
+    // maximum (as many floats)
     const float* pair_bound;
 };
 

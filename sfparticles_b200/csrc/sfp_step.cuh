@@ -583,96 +583,357 @@ __device__ __forceinline__ int sfp_find_group_pos(const long long* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// Bookkeeping: fold the appends of the step that ran, advance t; then
-// (prepare, bit 0) each group's tile length and tile map, tickets,
-// super-tile counts.  Bits 1 and 2 of `prepare`: the step's massive /
-// photon launch is the long-tile kernel, so that group's tiles must be
-// SFP_TILE_MAX long.  One block of 256 threads.
+// The end of a step's event kernels (sfp_step_end), one block of 256 threads:
+//   scan    -- an exclusive scan of both groups' super-tile event counts in
+//              tile order, restarted at each instance and kept per append
+//              channel, so super_pre[s] is the number of children that the
+//              same instance's earlier segments and tiles with the same
+//              destinations append before super-tile s; every segment's
+//              events become its destinations' append counts, and if a
+//              destination lacks room for the step's children the step
+//              waits for the host (append_wait) with nothing changed;
+//   fold    -- the appends enter n_buffered, t and step advance;
+//   prepare -- each group's tile length and tile map for the next step,
+//              tickets, super-tile counts at zero.
+// The next step's plan goes to the other of two slots (st->plan, tile_start,
+// n_buf_step; st->cur then names it), as the appends kernel that follows
+// still works by the plan of the step that ran.
+//
+// It runs in the block that finishes last of the step's last event launch
+// (sfp_last_block).  As two launches of one block each, the scan and the
+// bookkeeping took 7 and 5 us of a small step (1e4 e-), most of it chains of
+// dependent loads, and two launch gaps of 2 us; here the segments' and the
+// steps' data are loaded at once and held in shared memory.
+// sfp_book_kernel prepares the first step of a call and folds a resumed one.
 // ---------------------------------------------------------------------------
-SFP_DEVICE_INLINE long long sfp_group_map(const sfp_run_dev* __restrict__ R, const sfp_group_dev& G, int tile) {
-    long long acc = 0;
-    for (int j = 0; j < G.n_seg; ++j) {
-        acc = (acc + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE * SFP_SUPER_TILE;
-        G.tile_start[j] = acc;
-        acc += (R->n_buffered[G.seg[j]] + tile - 1) / tile;
-    }
-    G.tile_start[G.n_seg] = acc;
-    return acc;
+#define SFP_PREP 1
+// the next step's massive / photon launch is the long-tile kernel, so that
+// group's tiles must be SFP_TILE_MAX long
+#define SFP_PREP_M 2
+#define SFP_PREP_P 4
+#define SFP_FOLD 8
+#define SFP_SCAN 16
+
+// a step as its kernels see it
+struct sfp_step_view {
+    double t, lag;  // lag: steps since the stored photon positions
+    long long step, n_mtiles, n_ptiles;
+    const long long *m_start, *p_start, *n_buf;
+    int mtile, ptile;
+};
+SFP_DEVICE_INLINE sfp_step_view sfp_view(const sfp_run_dev* __restrict__ R, int slot) {
+    const sfp_step_state* st = R->st;
+    const sfp_step_plan& p = st->plan[slot];
+    sfp_step_view v;
+    v.t = p.t;
+    v.step = p.step;
+    v.lag = (double)(p.step - st->pos_epoch);
+    v.n_mtiles = p.n_mtiles;
+    v.n_ptiles = p.n_ptiles;
+    v.mtile = p.mtile;
+    v.ptile = p.ptile;
+    v.m_start = R->mg.tile_start + slot * (R->mg.n_seg + 1);
+    v.p_start = R->pg.tile_start + slot * (R->pg.n_seg + 1);
+    v.n_buf = R->n_buf_step + slot * R->n_seg;
+    return v;
 }
 
-// the group's tile of this step (SFP_TILE_MIN..SFP_TILE_MAX, a power of two)
-// and its tile map; a map too long for the counters takes a longer tile
-SFP_DEVICE_INLINE long long sfp_group_plan(const sfp_run_dev* __restrict__ R, const sfp_group_dev& G, int& tile) {
-    long long n = 0;
-    for (int j = 0; j < G.n_seg; ++j) n += R->n_buffered[G.seg[j]];
-    tile = SFP_TILE_MIN;
-    while (tile < SFP_TILE_MAX && (long long)tile * SFP_TILE_TARGET < n) tile <<= 1;
-    long long tiles = sfp_group_map(R, G, tile);
-    while (tiles > G.max_tiles && tile < SFP_TILE_MAX) {
-        tile <<= 1;
-        tiles = sfp_group_map(R, G, tile);
+// true in every thread of the block of this launch that is last to arrive, of
+// `blocks` that take part; earlier blocks' writes are then visible to it
+__device__ __forceinline__ bool sfp_last_block(sfp_step_state* st, unsigned int blocks) {
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int n = atomicAdd(&st->blocks_done, 1);
+        s_last = n == (int)blocks - 1;
+        if (s_last) st->blocks_done = 0;
     }
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last != 0;
+}
+
+SFP_DEVICE_INLINE long long sfp_warp_sum64(long long v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+SFP_DEVICE_INLINE uint4 shfl_up_u4(uint4 v, int o) {
+    return uint4{__shfl_up_sync(0xffffffffu, v.x, o), __shfl_up_sync(0xffffffffu, v.y, o),
+                 __shfl_up_sync(0xffffffffu, v.z, o), __shfl_up_sync(0xffffffffu, v.w, o)};
+}
+
+// inclusive warp scan of (head, value) pairs: a head restarts the sum
+SFP_DEVICE_INLINE void seg_scan_warp(unsigned int& h, uint4& v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int oh = __shfl_up_sync(0xffffffffu, h, o);
+        const uint4 ov = shfl_up_u4(v, o);
+        if (lane >= o) {
+            if (!h) v = sfp::u4_add(ov, v);
+            h |= oh;
+        }
+    }
+}
+
+// the group's tile map for tiles of 2^sh particles, by a warp, from the next
+// step's counts nb: each segment's tiles start at a multiple of
+// SFP_SUPER_TILE; returns the number of tiles
+SFP_DEVICE_INLINE long long sfp_group_map(const sfp_group_dev& G, const long long* nb, int sh, long long* start) {
+    const int lane = threadIdx.x & 31;
+    long long carry = 0, end = 0;
+    for (int j0 = 0; j0 < G.n_seg; j0 += 32) {
+        const int j = j0 + lane;
+        const long long n = j < G.n_seg ? nb[G.seg[j]] : 0;
+        const long long t = (n + (1 << sh) - 1) >> sh;
+        const long long own = (t + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE * SFP_SUPER_TILE;
+        long long inc = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        const long long at = carry + inc - own;
+        if (j < G.n_seg) start[j] = at;
+        end = __shfl_sync(0xffffffffu, at + t, min(31, G.n_seg - 1 - j0));
+        carry += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) start[G.n_seg] = end;
+    return end;
+}
+
+// the group's tile of the next step (SFP_TILE_MIN..SFP_TILE_MAX, a power of
+// two) and its tile map; a map too long for the counters takes a longer tile
+SFP_DEVICE_INLINE long long sfp_group_plan(const sfp_group_dev& G, const long long* nb, long long* start, int& tile) {
+    long long n = 0;
+    for (int j = threadIdx.x & 31; j < G.n_seg; j += 32) n += nb[G.seg[j]];
+    n = sfp_warp_sum64(n);
+    int sh = 5;  // SFP_TILE_MIN
+    while ((1 << sh) < SFP_TILE_MAX && ((long long)SFP_TILE_TARGET << sh) < n) ++sh;
+    long long tiles = sfp_group_map(G, nb, sh, start);
+    while (tiles > G.max_tiles && (1 << sh) < SFP_TILE_MAX) tiles = sfp_group_map(G, nb, ++sh, start);
+    tile = 1 << sh;
     return tiles;
 }
 
-extern "C" __global__ void __launch_bounds__(256) sfp_book_kernel(const sfp_run_dev* __restrict__ R, int prepare) {
-    __shared__ long long s_nsuper_m, s_nsuper_p;
+__device__ __forceinline__ void sfp_step_end(const sfp_run_dev* __restrict__ R, int flags, sfp_end_smem& Q) {
     sfp_step_state* st = R->st;
-    const int n = R->n_seg;
-    // a step that stopped before writing its children is folded only once resumed
-    if (st->pending && !st->append_wait) {
-        for (int s = threadIdx.x; s < n; s += blockDim.x) {
-            R->n_buffered[s] += (long long)R->appended[s];
-            R->appended[s] = 0ull;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            st->t = st->t + R->dt;
-            st->step += 1;
-            st->pending = 0;
+    const int n = R->n_seg, nm = R->mg.n_seg, np = R->pg.n_seg;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool held = n <= SFP_END_SEGS;
+    sfp_end_seg* const seg = held ? Q.seg : R->end_seg;
+    unsigned long long* const app = held ? Q.app : R->end_app;
+    long long* const nb = held ? Q.nb : R->end_nb;
+    const int cur = st->cur, slot = (flags & SFP_FOLD) ? cur ^ 1 : cur;
+    const sfp_step_plan now = st->plan[cur];
+    const bool go = !(st->halted || st->error || st->append_wait);
+    const long long *m_start = R->mg.tile_start + cur * (nm + 1), *p_start = R->pg.tile_start + cur * (np + 1);
+    const long long* n_buf = R->n_buf_step + cur * n;
+    __syncthreads();  // the dynamic shared memory's earlier users are done
+    if (threadIdx.x == 0) Q.lacks = 0;
+    const int nsm = (int)((now.n_mtiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE);
+    const int nsp = (int)((now.n_ptiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE);
+    long long ps = 0;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const long long at = (flags & SFP_FOLD) ? n_buf[k] : __ldcg(&R->n_buffered[k]);
+        ps += at;
+        nb[k] = at;
+        app[k] = (flags & (SFP_FOLD | SFP_SCAN)) == SFP_FOLD ? __ldcg(&R->appended[k]) : 0ull;
+        if (flags & SFP_SCAN) {  // entry k of the massive group's segments, then the photon group's
+            const bool massive = k < nm;
+            const int j = massive ? k : k - nm;
+            const sfp_segment& S = R->seg[massive ? R->mg.seg[j] : R->pg.seg[j]];
+            sfp_end_seg e;
+            e.super0 = massive ? (int)(m_start[j] / SFP_SUPER_TILE) : nsm + (int)(p_start[j] / SFP_SUPER_TILE);
+            e.chain = 2 * S.instance + (massive ? 0 : 1);
+            e.channel = S.channel;
+            e.dest0 = massive ? S.photon_dest : S.ele_dest;
+            e.dest1 = massive ? -1 : S.pos_dest;
+            seg[k] = e;
         }
     }
     __syncthreads();
-    if (!prepare) return;
-    if (st->halted || st->error || st->append_wait) {
-        if (threadIdx.x == 0) st->skip = 1;
-        return;
-    }
-    if (threadIdx.x == 0) {
-        s_nsuper_m = s_nsuper_p = 0;
-        long long ps = 0;
-        for (int s = 0; s < n; ++s) {
-            R->n_buf_step[s] = R->n_buffered[s];
-            ps += R->n_buffered[s];
+    if (flags & SFP_SCAN) {
+        // the super-tiles of both groups as one sequence, a run of them per
+        // thread; a head is the first super-tile of its instance and group
+        const int ns = nsm + nsp;
+        const int per = (ns + (int)blockDim.x - 1) / (int)blockDim.x;
+        const int s0 = min(ns, (int)threadIdx.x * per), s1 = min(ns, s0 + per);
+        auto count = [&](int s) { return __ldcg(s < nsm ? &R->mg.super_cnt[s] : &R->pg.super_cnt[s - nsm]); };
+        // the last entry that starts at or before s
+        auto find = [&](int s) {
+            int lo = 0, hi = n - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (seg[mid].super0 <= s) lo = mid;
+                else hi = mid - 1;
+            }
+            return lo;
+        };
+        unsigned int h = 0, c0 = 0;
+        uint4 v{0u, 0u, 0u, 0u};
+        int j0 = 0, before = -1;  // the run's first entry; the chain of the super-tile before it
+        if (s0 < s1) {
+            c0 = count(s0);
+            j0 = find(s0);
+            if (s0 > 0) before = s0 - 1 >= seg[j0].super0 ? seg[j0].chain : seg[find(s0 - 1)].chain;
+            int j = j0, prev = before;
+            for (int s = s0; s < s1; ++s) {
+                while (j + 1 < n && seg[j + 1].super0 <= s) ++j;
+                if (seg[j].chain != prev) {
+                    h = 1;
+                    v = uint4{0u, 0u, 0u, 0u};
+                    prev = seg[j].chain;
+                }
+                v = sfp::u4_add(v, sfp::u4_one(seg[j].channel, s == s0 ? c0 : count(s)));
+            }
         }
-        // each segment's tiles start at a multiple of SFP_SUPER_TILE tiles
-        int mt = SFP_TILE_MAX, pt = SFP_TILE_MAX;
-        const long long m_tiles = sfp_group_plan(R, R->mg, mt);
-        const long long p_tiles = sfp_group_plan(R, R->pg, pt);
-        if (m_tiles > R->mg.max_tiles || p_tiles > R->pg.max_tiles) {
-            st->error = SFP_DEV_CAPACITY;
-            st->skip = 1;
-        } else if (((prepare & 2) && mt != SFP_TILE_MAX) || ((prepare & 4) && pt != SFP_TILE_MAX)) {
-            st->error = SFP_DEV_TILE;  // the long-tile kernels launched for a step with shorter tiles
+        seg_scan_warp(h, v);
+        if (lane == 31) {
+            Q.wh[warp] = h;
+            Q.wv[warp] = v;
+        }
+        __syncthreads();
+        // exclusive value of this thread: earlier warps, then earlier lanes of this warp
+        unsigned int lh = __shfl_up_sync(0xffffffffu, h, 1);
+        uint4 run = shfl_up_u4(v, 1);
+        if (lane == 0) {
+            lh = 0u;
+            run = uint4{0u, 0u, 0u, 0u};
+        }
+        for (int w = warp - 1; w >= 0 && !lh; --w) {
+            run = sfp::u4_add(Q.wv[w], run);
+            lh = Q.wh[w];
+        }
+        if (s0 < s1) {
+            int j = j0, prev = before;
+            unsigned long long acc = 0ull;
+            auto add = [&]() {
+                if (!acc) return;
+                if (seg[j].dest0 >= 0) atomicAdd(&app[seg[j].dest0], acc);
+                if (seg[j].dest1 >= 0) atomicAdd(&app[seg[j].dest1], acc);
+                acc = 0ull;
+            };
+            for (int s = s0; s < s1; ++s) {
+                while (j + 1 < n && seg[j + 1].super0 <= s) {
+                    add();
+                    ++j;
+                }
+                if (seg[j].chain != prev) {
+                    run = uint4{0u, 0u, 0u, 0u};
+                    prev = seg[j].chain;
+                }
+                const unsigned int c = s == s0 ? c0 : count(s);
+                (s < nsm ? R->mg.super_pre[s] : R->pg.super_pre[s - nsm]) = (long long)sfp::u4_get(run, seg[j].channel);
+                run = sfp::u4_add(run, sfp::u4_one(seg[j].channel, c));
+                acc += c;
+            }
+            add();
+        }
+        __syncthreads();  // every append count is in
+        // exact room check: the appends kernel writes nothing unless every
+        // destination holds its children; otherwise the step waits for the host
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            R->appended[k] = app[k];
+            if (app[k] && nb[k] + (long long)app[k] > R->seg[k].capacity) Q.lacks = 1;
+        }
+        __syncthreads();
+        if (Q.lacks) {
+            if (threadIdx.x == 0) {
+                st->append_wait = 1;
+                st->halted = 1;
+            }
+            return;
+        }
+    }
+    if (flags & SFP_FOLD) {
+        ps = sfp_warp_sum64(ps);
+        if (lane == 0) Q.ps[warp] = ps;
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            nb[k] += (long long)app[k];
+            R->n_buffered[k] = nb[k];
+            R->appended[k] = 0ull;
+        }
+        __syncthreads();
+    }
+    const double t = (flags & SFP_FOLD) ? now.t + R->dt : st->t;
+    const long long step = (flags & SFP_FOLD) ? now.step + 1 : st->step;
+    if (threadIdx.x == 0) {
+        if (flags & SFP_FOLD) {
+            long long all = 0;
+            for (int w = 0; w < 8; ++w) all += Q.ps[w];
+            st->particle_steps += all;
+            st->t = t;
+            st->step = step;
+            st->cur = slot;
+        }
+        if ((flags & SFP_PREP) && !go) st->skip = 1;
+    }
+    if (!(flags & SFP_PREP) || !go) return;
+    if (warp < 2) {
+        int tile = SFP_TILE_MAX;
+        const long long tiles =
+            warp == 0 ? sfp_group_plan(R->mg, nb, R->mg.tile_start + slot * (nm + 1), tile)
+                      : sfp_group_plan(R->pg, nb, R->pg.tile_start + slot * (np + 1), tile);
+        if (lane == 0) {
+            Q.tiles[warp] = tiles;
+            Q.tile[warp] = tile;
+        }
+    }
+    for (int k = threadIdx.x; k < n; k += blockDim.x) R->n_buf_step[slot * n + k] = nb[k];
+    __syncthreads();
+    const long long m_tiles = Q.tiles[0], p_tiles = Q.tiles[1];
+    const int mt = Q.tile[0], pt = Q.tile[1];
+    int error = SFP_DEV_OK;
+    if (m_tiles > R->mg.max_tiles || p_tiles > R->pg.max_tiles) error = SFP_DEV_CAPACITY;
+    else if (((flags & SFP_PREP_M) && mt != SFP_TILE_MAX) || ((flags & SFP_PREP_P) && pt != SFP_TILE_MAX))
+        error = SFP_DEV_TILE;  // the long-tile kernels launched for a step with shorter tiles
+    if (threadIdx.x == 0) {
+        if (error != SFP_DEV_OK) {
+            st->error = error;
             st->skip = 1;
         } else {
-            st->n_mtiles = m_tiles;
-            st->n_ptiles = p_tiles;
-            st->mtile = mt;
-            st->ptile = pt;
+            sfp_step_plan& P = st->plan[slot];
+            P.t = t;
+            P.step = step;
+            P.n_mtiles = m_tiles;
+            P.n_ptiles = p_tiles;
+            P.mtile = mt;
+            P.ptile = pt;
             st->mticket = 0;
             st->pticket = 0;
             st->skip = 0;
-            st->pending = 1;
-            st->particle_steps += ps;
-            s_nsuper_m = (m_tiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE;
-            s_nsuper_p = (p_tiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE;
         }
     }
-    __syncthreads();
+    if (error != SFP_DEV_OK) return;
     // the group kernels add into the super-tile counts: start them at zero
-    for (long long k = threadIdx.x; k < s_nsuper_m; k += blockDim.x) R->mg.super_cnt[k] = 0u;
-    for (long long k = threadIdx.x; k < s_nsuper_p; k += blockDim.x) R->pg.super_cnt[k] = 0u;
+    const long long zm = (m_tiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE;
+    const long long zp = (p_tiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE;
+    for (long long k = threadIdx.x; k < zm; k += blockDim.x) R->mg.super_cnt[k] = 0u;
+    for (long long k = threadIdx.x; k < zp; k += blockDim.x) R->pg.super_cnt[k] = 0u;
+}
+
+extern "C" __global__ void __launch_bounds__(256) sfp_book_kernel(const sfp_run_dev* __restrict__ R, int flags) {
+    extern __shared__ __align__(16) double s_tab[];
+    sfp_step_end(R, flags, *reinterpret_cast<sfp_end_smem*>(s_tab));
+}
+
+// what a launch does once its blocks are done (`tail`: sfp_step_end's flags,
+// or 0), in the last of them; `scratch`: its dynamic shared memory
+__device__ __noinline__ void sfp_tail(const sfp_run_dev* __restrict__ R, int tail, unsigned int blocks,
+                                      void* scratch) {
+    if (!tail || !sfp_last_block(R->st, blocks)) return;
+    sfp_step_end(R, tail, *static_cast<sfp_end_smem*>(scratch));
+}
+
+// blocks of a group launch that have tiles to take, of `grid`: one for four
+// tiles (the others leave at once), and one at least for the launch's tail
+SFP_DEVICE_INLINE unsigned int sfp_busy_blocks(long long n_tiles, unsigned int grid) {
+    const long long b = (n_tiles + 3) / 4;
+    return b < 1 ? 1u : b < (long long)grid ? (unsigned int)b : grid;
 }
 
 // ---------------------------------------------------------------------------
@@ -888,18 +1149,25 @@ __device__ __forceinline__ unsigned int sfp_massive_tile(const sfp_run_dev* __re
 // launches it while the group's population guarantees that, and the
 // bookkeeping kernel refuses a step planned otherwise with SFP_DEV_TILE).
 template <int FORM, int QED, int STAGES, bool LONG>
-__device__ __forceinline__ void sfp_massive_body(const sfp_run_dev* __restrict__ R) {
+__device__ __forceinline__ void sfp_massive_body(const sfp_run_dev* __restrict__ R, int tail) {
     using namespace sfp;
     constexpr int OD = QED == SFP_QED_OPTICAL_DEPTH ? 1 : 0;
     extern __shared__ __align__(16) double s_tab[];
     __shared__ char* s_desc[SFP_TILE / 32][6 + OD + 3 + 2];
     sfp_step_state* st = R->st;
-    if (st->skip || st->n_mtiles == 0) return;
-    const long long n_tiles = st->n_mtiles;
-    const int PT = LONG ? SFP_TILE_MAX : st->mtile;
-    const double t = st->t;
+    if (st->skip || st->halted) return;
+    const sfp_step_view V = sfp_view(R, st->cur);
+    const long long n_tiles = V.n_mtiles;
+    const unsigned int busy = sfp_busy_blocks(n_tiles, gridDim.x);
+    if (blockIdx.x >= busy) return;
+    if (n_tiles == 0) {
+        sfp_tail(R, tail, busy, s_tab);
+        return;
+    }
+    const int PT = LONG ? SFP_TILE_MAX : V.mtile;
+    const double t = V.t;
     const double dt = R->dt;
-    const unsigned int step = (unsigned int)st->step;
+    const unsigned int step = (unsigned int)V.step;
     const sfp_qed_smem T = sfp_stage_tables<FORM, QED>(R, s_tab);
     // learned photon-energy sampler: weights after the tables
     sfp_mlp::Smem& M = *reinterpret_cast<sfp_mlp::Smem*>(reinterpret_cast<unsigned char*>(s_tab) + R->mlp_off);
@@ -914,10 +1182,10 @@ __device__ __forceinline__ void sfp_massive_body(const sfp_run_dev* __restrict__
     long long tile = __shfl_sync(0xffffffffu, tk, 0);
     while (tile < n_tiles) {
         if (lane == 0) tk = atomicAdd(&st->mticket, 1);  // next ticket, in flight during this tile
-        const int pos = sfp_find_group_pos(R->mg.tile_start, R->mg.n_seg, tile);
+        const int pos = sfp_find_group_pos(V.m_start, R->mg.n_seg, tile);
         const sfp_segment& S = R->seg[R->mg.seg[pos]];
-        const long long N = R->n_buf_step[R->mg.seg[pos]];
-        const long long base = (tile - R->mg.tile_start[pos]) * (long long)PT;
+        const long long N = V.n_buf[R->mg.seg[pos]];
+        const long long base = (tile - V.m_start[pos]) * (long long)PT;
         unsigned int cnt = 0;
         if (base < N) {  // else: alignment padding between segments
             if (S.spin)
@@ -933,6 +1201,7 @@ __device__ __forceinline__ void sfp_massive_body(const sfp_run_dev* __restrict__
         }
         tile = __shfl_sync(0xffffffffu, tk, 0);
     }
+    sfp_tail(R, tail, busy, s_tab);
 }
 
 // ---------------------------------------------------------------------------
@@ -1088,7 +1357,7 @@ __device__ __forceinline__ void sfp_pair_enqueue(sfp_pair_queue<STATE>& q, unsig
 }
 
 template <int FORM, int QED, int STAGES, bool LONG>
-__device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ R) {
+__device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ R, int tail) {
     using namespace sfp;
     constexpr int OD = QED == SFP_QED_OPTICAL_DEPTH ? 1 : 0;
     constexpr bool QUEUE = QED == SFP_QED_REJECTION;
@@ -1101,24 +1370,26 @@ __device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ 
     __shared__ float s_pb[QUEUE ? SFP_PAIR_BOUND_BINS : 1];
     __shared__ float s_pbmax[QUEUE ? SFP_PAIR_BOUND_BINS : 1];  // its prefix maximum
     sfp_step_state* st = R->st;
-    if (st->skip || st->n_ptiles == 0) return;
-    const long long n_tiles = st->n_ptiles;
-    const int PT = LONG ? SFP_TILE_MAX : st->ptile;
-    const double t = st->t;
+    if (st->skip || st->halted) return;
+    const sfp_step_view V = sfp_view(R, st->cur);
+    const long long n_tiles = V.n_ptiles;
+    const unsigned int busy = sfp_busy_blocks(n_tiles, gridDim.x);
+    if (blockIdx.x >= busy) return;
+    if (n_tiles == 0) {
+        sfp_tail(R, tail, busy, s_tab);
+        return;
+    }
+    const int PT = LONG ? SFP_TILE_MAX : V.ptile;
+    const double t = V.t;
     const double dt = R->dt;
-    const unsigned int step = (unsigned int)st->step;
-    const double lag = (double)(st->step - st->pos_epoch);  // steps since the stored positions
+    const unsigned int step = (unsigned int)V.step;
+    const double lag = V.lag;  // steps since the stored positions
     const sfp_qed_smem T = sfp_stage_tables<FORM, QED>(R, s_tab);
     if (QUEUE)
-        for (int k = threadIdx.x; k < SFP_PAIR_BOUND_BINS; k += blockDim.x) s_pb[k] = R->pair_bound[k];
-    __syncthreads();
-    if (QUEUE && threadIdx.x == 0) {
-        float m = 0.0f;
-        for (int k = 0; k < SFP_PAIR_BOUND_BINS; ++k) {
-            m = fmaxf(m, s_pb[k]);
-            s_pbmax[k] = m;
+        for (int k = threadIdx.x; k < SFP_PAIR_BOUND_BINS; k += blockDim.x) {
+            s_pb[k] = R->pair_bound[k];
+            s_pbmax[k] = R->pair_bound[SFP_PAIR_BOUND_BINS + k];
         }
-    }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char* ring = reinterpret_cast<unsigned char*>(s_tab) + R->ring_off + (size_t)warp * STAGES * SB;
@@ -1130,14 +1401,14 @@ __device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ 
     long long tile = __shfl_sync(0xffffffffu, tk, 0);
     while (tile < n_tiles) {
         if (lane == 0) tk = atomicAdd(&st->pticket, 1);  // next ticket, in flight during this tile
-        const int pos = sfp_find_group_pos(R->pg.tile_start, R->pg.n_seg, tile);
+        const int pos = sfp_find_group_pos(V.p_start, R->pg.n_seg, tile);
         const int si = R->pg.seg[pos];
         const sfp_segment& S = R->seg[si];
         const sfp_instance& I = R->inst[S.instance];
         const double* __restrict__ P = sfp_field_params(I);
         const float cpg = QUEUE ? sfp_chi_per_gamma(P) : 0.0f;  // chi per gamma no photon exceeds here
-        const long long N = R->n_buf_step[si];
-        const long long base = (tile - R->pg.tile_start[pos]) * (long long)PT;
+        const long long N = V.n_buf[si];
+        const long long base = (tile - V.p_start[pos]) * (long long)PT;
         if (base >= N) {  // alignment padding between segments: no photons
             if (lane == 0) R->pg.tile_cnt[tile] = 0u;
             tile = __shfl_sync(0xffffffffu, tk, 0);
@@ -1251,160 +1522,7 @@ __device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ 
         }
         tile = __shfl_sync(0xffffffffu, tk, 0);
     }
-}
-
-// ---------------------------------------------------------------------------
-// Scan: one block.  For each group, an exclusive scan of the super-tile
-// event counts in tile order, restarted at each instance and kept per
-// append channel, so super_pre[s] is the number of children that the same
-// instance's earlier segments and tiles with the same destinations append
-// before super-tile s.  Adds every segment's events to its destinations'
-// append counts, then checks that every destination holds this step's
-// children; if one does not, the step waits for the host (append_wait).
-// ---------------------------------------------------------------------------
-// segment of super-tile s of group G and whether s starts a chain (the first
-// super-tile of its instance's tiles in that group)
-SFP_DEVICE_INLINE void sfp_super_info(const sfp_run_dev* __restrict__ R, const sfp_group_dev& G, long long s, int& si,
-                                      bool& head) {
-    const long long tile = s * SFP_SUPER_TILE;
-    si = G.seg[sfp_find_group_pos(G.tile_start, G.n_seg, tile)];
-    if (s == 0) {
-        head = true;
-        return;
-    }
-    const int prev = G.seg[sfp_find_group_pos(G.tile_start, G.n_seg, tile - SFP_SUPER_TILE)];
-    head = R->seg[prev].instance != R->seg[si].instance;
-}
-
-SFP_DEVICE_INLINE uint4 shfl_up_u4(uint4 v, int o) {
-    return uint4{__shfl_up_sync(0xffffffffu, v.x, o), __shfl_up_sync(0xffffffffu, v.y, o),
-                 __shfl_up_sync(0xffffffffu, v.z, o), __shfl_up_sync(0xffffffffu, v.w, o)};
-}
-
-// inclusive warp scan of (head, value) pairs: a head restarts the sum
-SFP_DEVICE_INLINE void seg_scan_warp(unsigned int& h, uint4& v) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned int oh = __shfl_up_sync(0xffffffffu, h, o);
-        const uint4 ov = shfl_up_u4(v, o);
-        if (lane >= o) {
-            if (!h) v = sfp::u4_add(ov, v);
-            h |= oh;
-        }
-    }
-}
-
-// a segment's events become appends of its destinations: photons (massive
-// group) or one electron and one positron each (photon group)
-template <bool MASSIVE>
-SFP_DEVICE_INLINE void sfp_add_appends(const sfp_run_dev* __restrict__ R, int si, unsigned long long n) {
-    if (!n) return;
-    const sfp_segment& S = R->seg[si];
-    if (MASSIVE) {
-        atomicAdd(&R->appended[S.photon_dest], n);
-    } else {
-        atomicAdd(&R->appended[S.ele_dest], n);
-        atomicAdd(&R->appended[S.pos_dest], n);
-    }
-}
-
-// block-wide: every thread calls it (n_tiles is uniform)
-template <bool MASSIVE>
-__device__ __forceinline__ void sfp_scan_group(const sfp_run_dev* __restrict__ R, const sfp_group_dev& G,
-                                               long long n_tiles, unsigned int* s_wh, uint4* s_wv) {
-    const long long n_super = (n_tiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE;
-    if (n_super == 0) return;
-    const long long per = (n_super + blockDim.x - 1) / blockDim.x;
-    const long long s0 = min(n_super, (long long)threadIdx.x * per), s1 = min(n_super, s0 + per);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // this thread's run of super-tiles as one scan element
-    unsigned int h = 0;
-    uint4 v{0u, 0u, 0u, 0u};
-    for (long long s = s0; s < s1; ++s) {
-        int si;
-        bool hd;
-        sfp_super_info(R, G, s, si, hd);
-        if (hd) {
-            h = 1;
-            v = uint4{0u, 0u, 0u, 0u};
-        }
-        v = sfp::u4_add(v, sfp::u4_one(R->seg[si].channel, G.super_cnt[s]));
-    }
-    seg_scan_warp(h, v);
-    __syncthreads();  // the previous user of s_wh / s_wv is done
-    if (lane == 31) {
-        s_wh[warp] = h;
-        s_wv[warp] = v;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
-        unsigned int wh = lane < nw ? s_wh[lane] : 0u;
-        uint4 wv = lane < nw ? s_wv[lane] : uint4{0u, 0u, 0u, 0u};
-        seg_scan_warp(wh, wv);
-        unsigned int eh = __shfl_up_sync(0xffffffffu, wh, 1);
-        uint4 ev = shfl_up_u4(wv, 1);
-        if (lane == 0) {
-            eh = 0u;
-            ev = uint4{0u, 0u, 0u, 0u};
-        }
-        if (lane < nw) {
-            s_wh[lane] = eh;
-            s_wv[lane] = ev;
-        }
-    }
-    __syncthreads();
-    // exclusive value of this thread: earlier warps, then earlier lanes of this warp
-    unsigned int lh = __shfl_up_sync(0xffffffffu, h, 1);
-    uint4 lv = shfl_up_u4(v, 1);
-    if (lane == 0) {
-        lh = 0u;
-        lv = uint4{0u, 0u, 0u, 0u};
-    }
-    uint4 run = lh ? lv : sfp::u4_add(s_wv[warp], lv);
-    int cur = -1;
-    unsigned long long acc = 0ull;
-    for (long long s = s0; s < s1; ++s) {
-        int si;
-        bool hd;
-        sfp_super_info(R, G, s, si, hd);
-        if (hd) run = uint4{0u, 0u, 0u, 0u};
-        const int ch = R->seg[si].channel;
-        G.super_pre[s] = (long long)sfp::u4_get(run, ch);
-        const unsigned int c = G.super_cnt[s];
-        run = sfp::u4_add(run, sfp::u4_one(ch, c));
-        if (si != cur) {
-            if (cur >= 0) sfp_add_appends<MASSIVE>(R, cur, acc);
-            cur = si;
-            acc = 0ull;
-        }
-        acc += c;
-    }
-    if (cur >= 0) sfp_add_appends<MASSIVE>(R, cur, acc);
-}
-
-extern "C" __global__ void __launch_bounds__(1024) sfp_scan_kernel(const sfp_run_dev* __restrict__ R) {
-    __shared__ unsigned int s_wh[32];
-    __shared__ uint4 s_wv[32];
-    __shared__ int s_short;
-    const sfp_step_state* st = R->st;
-    if (st->skip) return;
-    if (R->any_rad) sfp_scan_group<true>(R, R->mg, st->n_mtiles, s_wh, s_wv);
-    if (R->any_bw) sfp_scan_group<false>(R, R->pg, st->n_ptiles, s_wh, s_wv);
-    if (threadIdx.x == 0) s_short = 0;
-    __syncthreads();  // every append count is in
-    // exact room check: the appends kernel writes nothing unless every
-    // destination holds its children; otherwise the step waits for the host
-    for (int c = threadIdx.x; c < R->n_dseg; c += blockDim.x) {
-        const int d = R->dseg[c];
-        if (R->n_buf_step[d] + (long long)R->appended[d] > R->seg[d].capacity) atomicExch(&s_short, 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && s_short) {
-        R->st->append_wait = 1;
-        R->st->halted = 1;
-    }
+    sfp_tail(R, tail, busy, s_tab);
 }
 
 // ---------------------------------------------------------------------------
@@ -1448,11 +1566,12 @@ __device__ __forceinline__ void sfp_write_pair_child(const sfp_segment& D, long 
 
 template <int FORM>
 __device__ __forceinline__ void sfp_write_photon(const sfp_run_dev* __restrict__ R, const sfp_segment& S, long long i,
-                                                 long long rank, long long pre, const double* __restrict__ P, double t,
-                                                 double dt, double lag) {
+                                                 long long rank, long long pre, const double* __restrict__ P,
+                                                 const sfp_step_view& V, double dt) {
     using namespace sfp;
+    const double t = V.t, lag = V.lag;
     const sfp_segment& D = R->seg[S.photon_dest];
-    const long long slot = R->n_buf_step[S.photon_dest] + pre + rank;
+    const long long slot = V.n_buf[S.photon_dest] + pre + rank;
     double x = S.x[i], y = S.y[i], z = S.z[i];
     double ux = S.ux[i], uy = S.uy[i], uz = S.uz[i];
     const double d = S.delta[i];
@@ -1504,8 +1623,9 @@ __device__ __forceinline__ void sfp_write_photon(const sfp_run_dev* __restrict__
 
 template <int FORM>
 __device__ __forceinline__ void sfp_write_pair(const sfp_run_dev* __restrict__ R, const sfp_segment& S, long long i,
-                                               long long rank, long long pre, const double* __restrict__ P, double t,
-                                               double dt, double lag) {
+                                               long long rank, long long pre, const double* __restrict__ P,
+                                               const sfp_step_view& V, double dt) {
+    const double t = V.t, lag = V.lag;
     const double d = S.delta[i];
     double px = S.x[i], py = S.y[i], pz = S.z[i];
     const double pux = S.ux[i], puy = S.uy[i], puz = S.uz[i];
@@ -1518,28 +1638,30 @@ __device__ __forceinline__ void sfp_write_pair(const sfp_run_dev* __restrict__ R
         S.z[i] = pz;
     }
     S.pruned[i] = 1;
-    const long long be = R->n_buf_step[S.ele_dest] + pre + rank;
-    const long long bp = R->n_buf_step[S.pos_dest] + pre + rank;
+    const long long be = V.n_buf[S.ele_dest] + pre + rank;
+    const long long bp = V.n_buf[S.pos_dest] + pre + rank;
     sfp_write_pair_child<FORM>(R->seg[S.ele_dest], be, P, px, py, pz, d * pux, d * puy, d * puz, t, dt);
     const double d2 = 1.0 - d;
     sfp_write_pair_child<FORM>(R->seg[S.pos_dest], bp, P, px, py, pz, d2 * pux, d2 * puy, d2 * puz, t, dt);
 }
 
 template <int FORM, bool MASSIVE>
-__device__ __forceinline__ void sfp_append_tile(const sfp_run_dev* __restrict__ R, const sfp_group_dev& G, int PT,
-                                                long long tile, unsigned int c, unsigned short* list, double t,
-                                                double dt, double lag) {
+__device__ __forceinline__ void sfp_append_tile(const sfp_run_dev* __restrict__ R, const sfp_group_dev& G,
+                                                const sfp_step_view& V, long long tile, unsigned int c,
+                                                unsigned short* list, double dt) {
     using namespace sfp;
+    const int PT = MASSIVE ? V.mtile : V.ptile;
+    const long long* start = MASSIVE ? V.m_start : V.p_start;
     const int lane = threadIdx.x & 31;
     const long long s = tile / SFP_SUPER_TILE;
     unsigned int part = 0u;
     for (long long k = s * SFP_SUPER_TILE + lane; k < tile; k += 32) part += G.tile_cnt[k];
     const long long pre = G.super_pre[s] + (long long)warp_sum(part);
-    const int pos = sfp_find_group_pos(G.tile_start, G.n_seg, tile);
+    const int pos = sfp_find_group_pos(start, G.n_seg, tile);
     const sfp_segment& S = R->seg[G.seg[pos]];
     const double* __restrict__ P = sfp_field_params(R->inst[S.instance]);
-    const long long N = R->n_buf_step[G.seg[pos]];
-    const long long base = (tile - G.tile_start[pos]) * (long long)PT;
+    const long long N = V.n_buf[G.seg[pos]];
+    const long long base = (tile - start[pos]) * (long long)PT;
     const int len = (int)min(N - base, (long long)PT);  // the tile's particles
     // the tile's marked particles, in index order: lane q covers 16 flags per pass
     unsigned int n = 0u;
@@ -1571,8 +1693,8 @@ __device__ __forceinline__ void sfp_append_tile(const sfp_run_dev* __restrict__ 
         const unsigned int j = j0 + lane;
         if (j < n) {
             const long long i = base + list[j];
-            if (MASSIVE) sfp_write_photon<FORM>(R, S, i, j, pre, P, t, dt, lag);
-            else sfp_write_pair<FORM>(R, S, i, j, pre, P, t, dt, lag);
+            if (MASSIVE) sfp_write_photon<FORM>(R, S, i, j, pre, P, V, dt);
+            else sfp_write_pair<FORM>(R, S, i, j, pre, P, V, dt);
         }
     }
     __syncwarp();  // the list is read before the next tile rewrites it
@@ -1582,16 +1704,16 @@ template <int FORM>
 __device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__ R) {
     __shared__ unsigned short s_list[SFP_TILE / 32][SFP_TILE_MAX];
     const sfp_step_state* st = R->st;
-    if (st->skip || st->append_wait) return;
-    const long long nm = R->any_rad ? st->n_mtiles : 0, np = R->any_bw ? st->n_ptiles : 0;
-    const int mt = st->mtile, pt = st->ptile;
+    if (st->skip || st->halted) return;
+    const sfp_step_view V = sfp_view(R, st->cur ^ 1);  // the step whose events were scanned
+    const long long nm = R->any_rad ? V.n_mtiles : 0, np = R->any_bw ? V.n_ptiles : 0;
     const long long n_all = nm + np;
-    const double t = st->t;
+    const unsigned int busy_blocks = sfp_busy_blocks(n_all, gridDim.x);
+    if (blockIdx.x >= busy_blocks) return;
     const double dt = R->dt;
-    const double lag = (double)(st->step - st->pos_epoch);  // photon positions: steps since stored
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    const long long nw = ((long long)busy_blocks * blockDim.x) >> 5;
     // warp gw owns tiles gw, gw + nw, gw + 2 nw, ...: tiles with events
     // (every massive tile in a cascade, a few photon tiles) spread over all
     // warps instead of queueing behind one warp per 32 neighbours
@@ -1606,8 +1728,8 @@ __device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__
             busy &= busy - 1u;
             const long long tg = gw + (j0 + b) * nw;
             const unsigned int c = __shfl_sync(0xffffffffu, mc, b);
-            if (tg < nm) sfp_append_tile<FORM, true>(R, R->mg, mt, tg, c, s_list[warp], t, dt, lag);
-            else sfp_append_tile<FORM, false>(R, R->pg, pt, tg - nm, c, s_list[warp], t, dt, lag);
+            if (tg < nm) sfp_append_tile<FORM, true>(R, R->mg, V, tg, c, s_list[warp], dt);
+            else sfp_append_tile<FORM, false>(R, R->pg, V, tg - nm, c, s_list[warp], dt);
         }
     }
 }
@@ -1618,23 +1740,23 @@ __device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__
 // sfp_photon_..._t (any tile length: the steps of small populations)
 #define SFP_MASSIVE_KERNEL(FORM_S, QED_S, FORM, QED, STAGES, MINB)                                             \
     extern "C" __global__ void __launch_bounds__(SFP_TILE, MINB)                                              \
-        sfp_massive_##FORM_S##_##QED_S##_s##STAGES##_b##MINB(const sfp_run_dev* __restrict__ R) {             \
-        sfp_massive_body<FORM, QED, STAGES, true>(R);                                                        \
+        sfp_massive_##FORM_S##_##QED_S##_s##STAGES##_b##MINB(const sfp_run_dev* __restrict__ R, int tail) {   \
+        sfp_massive_body<FORM, QED, STAGES, true>(R, tail);                                                        \
     }
 #define SFP_PHOTON_KERNEL(FORM_S, QED_S, FORM, QED, STAGES, MINB)                                              \
     extern "C" __global__ void __launch_bounds__(SFP_TILE, MINB)                                              \
-        sfp_photon_##FORM_S##_##QED_S##_s##STAGES##_b##MINB(const sfp_run_dev* __restrict__ R) {              \
-        sfp_photon_body<FORM, QED, STAGES, true>(R);                                                         \
+        sfp_photon_##FORM_S##_##QED_S##_s##STAGES##_b##MINB(const sfp_run_dev* __restrict__ R, int tail) {              \
+        sfp_photon_body<FORM, QED, STAGES, true>(R, tail);                                                         \
     }
 #define SFP_MASSIVE_KERNEL_T(FORM_S, QED_S, FORM, QED, STAGES, MINB)                                           \
     extern "C" __global__ void __launch_bounds__(SFP_TILE, MINB)                                              \
-        sfp_massive_##FORM_S##_##QED_S##_s##STAGES##_b##MINB##_t(const sfp_run_dev* __restrict__ R) {         \
-        sfp_massive_body<FORM, QED, STAGES, false>(R);                                                       \
+        sfp_massive_##FORM_S##_##QED_S##_s##STAGES##_b##MINB##_t(const sfp_run_dev* __restrict__ R, int tail) {         \
+        sfp_massive_body<FORM, QED, STAGES, false>(R, tail);                                                       \
     }
 #define SFP_PHOTON_KERNEL_T(FORM_S, QED_S, FORM, QED, STAGES, MINB)                                            \
     extern "C" __global__ void __launch_bounds__(SFP_TILE, MINB)                                              \
-        sfp_photon_##FORM_S##_##QED_S##_s##STAGES##_b##MINB##_t(const sfp_run_dev* __restrict__ R) {          \
-        sfp_photon_body<FORM, QED, STAGES, false>(R);                                                        \
+        sfp_photon_##FORM_S##_##QED_S##_s##STAGES##_b##MINB##_t(const sfp_run_dev* __restrict__ R, int tail) {          \
+        sfp_photon_body<FORM, QED, STAGES, false>(R, tail);                                                        \
     }
 
 // ---------------------------------------------------------------------------

@@ -85,8 +85,8 @@ class Ensemble(object):
 
     def _launches_per_step(self):
         ps = self.species
-        return (1 + any(p.m != 0 for p in ps) + any(p.m == 0 for p in ps)
-                + 2 * any(p.bw or p.radiating for p in ps))
+        return (any(p.m != 0 for p in ps) + any(p.m == 0 for p in ps)
+                + any(p.bw or p.radiating for p in ps))
 
     def _begin(self):
         for p in self.species:

@@ -520,12 +520,12 @@ class Simulation(object):
         return out, before, [p.N_buffered for p in self.all_particles]
 
     def _launches_per_step(self):
-        """libsfp kernels one step launches: bookkeeping + the massive and
-        photon kernels that have species to work on + scan and appends when
-        a species emits photons or creates pairs."""
+        """libsfp kernels one step launches: the massive and photon kernels
+        that have species to work on + appends when a species emits photons or
+        creates pairs (a call launches one bookkeeping kernel besides)."""
         ps = self.all_particles
-        return (1 + any(p.m != 0 for p in ps) + any(p.m == 0 for p in ps)
-                + 2 * any(p.bw or p.radiating for p in ps))
+        return (any(p.m != 0 for p in ps) + any(p.m == 0 for p in ps)
+                + any(p.bw or p.radiating for p in ps))
 
     def _loop(self, run, nstep, call_back):
         L = _lib.load()
