@@ -215,6 +215,11 @@ int sfp_run_pending_need(sfp_run *r, int64_t *need);
  * fold its appends and advance t / step.  Asynchronous on the run's stream. */
 int sfp_run_resume(sfp_run *r, void *stream);
 int sfp_run_destroy(sfp_run *r);
+/* Destroyed runs leave their device blocks (bookkeeping, and the scratch
+ * copies of photons that a call of several steps makes, 25 bytes per photon,
+ * only where at least twice that is free) for later runs, at most 1 GiB in
+ * all.  This gives the blocks above 32 MiB back to the driver. */
+int sfp_release_cached(void);
 
 /* ---- learned photon-energy sampler (no counterpart in the reference) ------
  * An MLP (log10 chi, u) -> delta, 2 -> 64 -> 64 -> 64 -> 1 with SiLU, that can

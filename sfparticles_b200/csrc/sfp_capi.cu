@@ -802,6 +802,8 @@ int sfp_inv_gamma(const double* ux, const double* uy, const double* uz, double* 
 #define SFP_T_P_MINB 3
 // a group of more particles than this has SFP_TILE_MAX-long tiles at every
 // step (the tile rule), so the long-tile kernels may run it
+// photon segments of a run that may keep a store of hot photons
+#define SFP_HOT_MAX_SEGS 1024
 #define SFP_LONG_TILE_POP ((long long)(SFP_TILE_MAX / 2) * SFP_TILE_TARGET)
 
 struct sfp_group_host {
@@ -814,14 +816,16 @@ struct sfp_group_host {
 // run's bookkeeping is one block of a few hundred KB: as seventeen
 // cudaMalloc / cudaFree calls, a stream and two events it cost 1.2 ms per
 // run (create 0.7, destroy 0.45; several times that on a busy host), against
-// 4 ms for 32 steps of 1e6 particles.  Bounded: at most kPoolBlocks blocks
+// 4 ms for 32 steps of 1e6 particles.  A run's store of hot photons is a
+// second block, of 25 bytes per photon.  Bounded: at most kPoolBlocks blocks
 // and kPoolBytes bytes, and as many streams, over all devices; the rest goes
-// back to the driver at once, and everything does when an allocation fails.
-// A run gives its block and stream back only once its stream is idle, so no
-// work in flight can reach them; the lists are under one lock.
+// back to the driver at once, blocks above kPoolKeep when a Simulation or
+// Ensemble ends (sfp_release_cached), and every block when an allocation
+// fails.  A run gives its blocks and stream back only once its stream is
+// idle, so no work in flight can reach them; the lists are under one lock.
 namespace {
 
-constexpr size_t kPoolBlocks = 8, kPoolBytes = 32u << 20;
+constexpr size_t kPoolBlocks = 8, kPoolBytes = 1u << 30, kPoolKeep = 32u << 20;
 
 struct run_block {
     int dev = 0;
@@ -833,6 +837,7 @@ struct run_stream {
     cudaStream_t s = nullptr;
     cudaEvent_t in = nullptr, out = nullptr;
 };
+constexpr size_t kBlock0 = 1u << 18;
 std::mutex g_pool_mu;
 std::vector<run_block> g_blocks;
 std::vector<run_stream> g_streams;
@@ -849,7 +854,7 @@ bool block_get(size_t bytes, run_block* out) {
         std::lock_guard<std::mutex> g(g_pool_mu);
         size_t best = g_blocks.size();
         for (size_t k = 0; k < g_blocks.size(); ++k)
-            if (g_blocks[k].dev == dev && g_blocks[k].bytes >= bytes &&
+            if (g_blocks[k].dev == dev && g_blocks[k].bytes >= bytes && g_blocks[k].bytes / 4 <= std::max(bytes, kBlock0) &&
                 (best == g_blocks.size() || g_blocks[k].bytes < g_blocks[best].bytes))
                 best = k;
         if (best < g_blocks.size()) {
@@ -858,8 +863,9 @@ bool block_get(size_t bytes, run_block* out) {
             return true;
         }
     }
-    size_t n = 1u << 18;
-    while (n < bytes) n *= 2;
+    size_t n = kBlock0;
+    while (n < bytes && n < kPoolKeep) n *= 2;
+    n = std::max(n, bytes);
     out->dev = dev;
     out->bytes = n;
     if (cudaMalloc(&out->p, n) == cudaSuccess) return true;
@@ -874,6 +880,14 @@ bool block_get(size_t bytes, run_block* out) {
     if (cudaMalloc(&out->p, bytes) == cudaSuccess) return true;
     cudaGetLastError();
     out->p = nullptr;
+    return false;
+}
+
+bool block_cached(size_t bytes) {
+    const int dev = device_now();
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    for (const run_block& b : g_blocks)
+        if (b.dev == dev && b.bytes >= bytes && b.bytes / 4 <= std::max(bytes, kBlock0)) return true;
     return false;
 }
 
@@ -936,6 +950,13 @@ struct sfp_run {
     cudaKernel_t k_massive = nullptr, k_photon = nullptr, k_appends = nullptr, k_book = nullptr;
     cudaKernel_t k_massive_t = nullptr, k_photon_t = nullptr;  // any tile length
     cudaKernel_t k_sync = nullptr, k_epoch = nullptr;           // photon positions written out
+    cudaKernel_t k_hot = nullptr, k_hot_build = nullptr;        // hot photons (rejection sampling)
+    run_block hot_block;                                        // their store
+    long long hot_room = 0;                                     // entries it holds
+    long long hot_refused = 0;                                  // entries that found no memory
+    long long *d_hot_start = nullptr, *d_hot_cap = nullptr;
+    int grid_h = 0;
+    bool hot_f64 = false;
     int grid_m = 0, grid_p = 0, grid_a = 0, grid_mt = 0, grid_pt = 0;
     size_t smem_m = 0, smem_p = 0, smem_mt = 0, smem_pt = 0, smem_end = 0;
     std::vector<long long> nb_lo;  // lower bounds of the device's n_buffered (it only grows between reads)
@@ -1127,6 +1148,7 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     r->mod = m;
     r->n_seg = n_seg;
     r->n_inst = n_inst;
+    r->hot_f64 = f64;
     r->segs.assign(seg, seg + n_seg);
     r->insts.assign(inst, inst + n_inst);
     bool any_spin = false;
@@ -1255,6 +1277,11 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     ALLOC(h.st, sizeof(sfp_step_state));
     ALLOC(r->d, sizeof(sfp_run_dev));
     ALLOC(r->d_keys, sizeof(r->keys));
+    ALLOC(r->d_hot_start, n_seg * sizeof(long long));
+    ALLOC(r->d_hot_cap, n_seg * sizeof(long long));
+    ALLOC(h.hot.count, n_seg * sizeof(unsigned long long));
+    h.hot.start = r->d_hot_start;
+    h.hot.cap = r->d_hot_cap;
     float* pb;
     ALLOC(pb, 2 * SFP_PAIR_BOUND_BINS * sizeof(float));
     h.pair_bound = pb;
@@ -1306,6 +1333,13 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     for (size_t* q : {&r->smem_m, &r->smem_p, &r->smem_mt, &r->smem_pt}) *q = std::max(*q, r->smem_end);
     if ((rc = run_alloc_tiles(r))) return cleanup(rc);
     if ((rc = run_upload(r, inst, n_buffered))) return cleanup(rc);
+    if (cfg->qed == SFP_QED_REJECTION && h.any_bw && h.pg.n_seg <= SFP_HOT_MAX_SEGS) {
+        if ((rc = module_kernel(m, f64 ? "sfp_hot_fp64" : "sfp_hot_fp32", &r->k_hot)) ||
+            (rc = module_kernel(m, f64 ? "sfp_hot_build_fp64" : "sfp_hot_build_fp32", &r->k_hot_build)))
+            return cleanup(rc);
+        // the hot kernel keeps its tile map where the photon kernel has its ring
+        r->smem_p = std::max(r->smem_p, (size_t)h.ring_off + (h.pg.n_seg + 1) * sizeof(long long));
+    }
     const size_t cap = 200 * 1024;
     if (r->smem_m > cap || r->smem_p > cap || r->smem_mt > cap || r->smem_pt > cap)
         return cleanup(fail(SFP_EINVAL, "QED tables and copy rings too large for shared memory"));
@@ -1323,6 +1357,11 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     r->grid_mt = persistent_grid(r->k_massive_t, r->smem_mt, t_minb);
     r->grid_pt = persistent_grid(r->k_photon_t, r->smem_pt, SFP_T_P_MINB);
     r->grid_a = persistent_grid(r->k_appends, 0, 2);
+    if (r->k_hot) {
+        if (raise_dynamic_smem((const void*)r->k_hot, r->smem_p) != cudaSuccess)
+            return cleanup(fail(SFP_ECUDA, "cannot raise dynamic shared memory"));
+        r->grid_h = persistent_grid(r->k_hot, r->smem_p, 2);
+    }
     *out = r;
     return SFP_OK;
 }
@@ -1371,7 +1410,7 @@ struct cfield_guard {
 };
 
 // flags of the end of a step (sfp_step.cuh: SFP_PREP ... SFP_SCAN)
-enum { PREP = 1, PREP_M = 2, PREP_P = 4, FOLD = 8, SCAN = 16 };
+enum { PREP = 1, PREP_M = 2, PREP_P = 4, FOLD = 8, SCAN = 16, HOT = 32 };
 
 // the bookkeeping of a call's first step (PREP), or the fold of a resumed one
 static int launch_book(sfp_run* r, int flags) {
@@ -1387,8 +1426,10 @@ static int prep_flags(bool mlong, bool plong) { return PREP | (mlong ? PREP_M : 
 // step and prepares the next one.  ev (6 events) brackets the massive, the
 // photon and the appends kernels when given.
 // mlong / plong: the group's steps all have SFP_TILE_MAX-long tiles, run by
-// the autotuned long-tile kernel; else by the any-tile kernel
-static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, bool plong) {
+// the autotuned long-tile kernel; else by the any-tile kernel.  hot: the call
+// has a store of hot photons; the full photon kernel behind it runs the steps
+// after the store has run out of room (it leaves at once before)
+static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, bool plong, bool hot) {
     const bool has_m = !r->mg.seg.empty(), has_p = !r->pg.seg.empty(), has_a = !r->dseg.empty();
     // the bookkeeping checks the tiles that the next launches assume
     int end = FOLD | prep_flags(mlong, plong) | (has_a ? SCAN : 0);
@@ -1406,6 +1447,8 @@ static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, 
     if (ev) SFP_CUDA(cudaEventRecord(ev[2], s));
     if (has_p) {
         void* a[] = {&r->d, &end};
+        if (hot)
+            SFP_CUDA(cudaLaunchKernel((const void*)r->k_hot, dim3(r->grid_h), dim3(SFP_TILE_HOST), a, r->smem_p, s));
         if (plong)
             SFP_CUDA(cudaLaunchKernel((const void*)r->k_photon, dim3(r->grid_p), dim3(SFP_TILE_HOST), a, r->smem_p, s));
         else
@@ -1422,6 +1465,86 @@ static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, 
     return SFP_OK;
 }
 
+// Hot photons: a call of at least HOT_MIN_STEPS steps whose photon group is
+// large keeps a store of them.  Building it reads every photon's momentum
+// (25 bytes), half of what one step of the full kernel reads, so it pays from
+// the second step on where few photons are hot and from the fourth where half
+// are.  Below the long-tile population a step is bound by latency, not by the
+// photons it reads.
+constexpr int64_t HOT_MIN_STEPS = 4;
+
+// room for the store at the current counts (5/8 of a segment's photons, new
+// ones included); false: the call does without (no memory to spare: the store
+// takes at most half of what is free)
+static bool hot_store(sfp_run* r, cudaStream_t caller) {
+    if (!r->k_hot) return false;
+    // (a caller that captures its stream gets launches only)
+    cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(caller, &cap_st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (cap_st != cudaStreamCaptureStatusNone) return false;
+    const bool f64 = r->k_hot && r->hot_f64;
+    std::vector<long long> start(r->n_seg, 0), cap(r->n_seg, 0);
+    long long n = 0;
+    for (int s : r->pg.seg) {
+        const long long nb = r->nb_lo[s];
+        if (r->segs[s].capacity >= 0xFFFFFFFFll) return false;  // entries hold 32-bit indices
+        start[s] = n;
+        cap[s] = r->segs[s].bw && r->segs[s].push ? (nb / 8 * 5 + 65536 + 63) / 64 * 64 : 0;
+        n += cap[s];
+    }
+    const size_t each = f64 ? 52 : 40;
+    if (n > r->hot_room) {
+        if (r->hot_refused && n >= r->hot_refused) return false;
+        const long long room = r->hot_room ? n + n / 2 : n + n / 8;
+        const size_t bytes = (size_t)room * each;
+        if (r->hot_block.p) {
+            if (cudaStreamSynchronize(r->s) != cudaSuccess) return false;  // earlier calls still use it
+            block_put(r->hot_block);
+        }
+        r->hot_block = run_block();
+        r->hot_room = 0;
+        size_t free_b = 0, all_b = 0;
+        if (!block_cached(bytes) && (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || free_b / 2 < bytes)) {
+            r->hot_refused = n;
+            return false;
+        }
+        if (!block_get(bytes, &r->hot_block)) {
+            r->hot_refused = n;
+            return false;
+        }
+        r->hot_room = room;
+        char* p = static_cast<char*>(r->hot_block.p);
+        const size_t d8 = (size_t)room * 8, du = (size_t)room * (f64 ? 8 : 4);
+        sfp_hot_dev& H = r->h.hot;
+        H.x = reinterpret_cast<double*>(p);
+        H.y = reinterpret_cast<double*>(p + d8);
+        H.z = reinterpret_cast<double*>(p + 2 * d8);
+        H.ux = p + 3 * d8;
+        H.uy = p + 3 * d8 + du;
+        H.uz = p + 3 * d8 + 2 * du;
+        H.idx = reinterpret_cast<unsigned int*>(p + 3 * d8 + 3 * du);
+        if (cudaMemcpyAsync(r->d, &r->h, sizeof(sfp_run_dev), cudaMemcpyHostToDevice, r->s) != cudaSuccess) return false;
+    }
+    return cudaMemcpyAsync(r->d_hot_start, start.data(), r->n_seg * sizeof(long long), cudaMemcpyHostToDevice, r->s) ==
+               cudaSuccess &&
+           cudaMemcpyAsync(r->d_hot_cap, cap.data(), r->n_seg * sizeof(long long), cudaMemcpyHostToDevice, r->s) ==
+               cudaSuccess;
+}
+
+// the first launches of a call: the bookkeeping of its first step and, if the
+// call keeps a store of hot photons, that store
+static int launch_first(sfp_run* r, bool mlong, bool plong, bool hot) {
+    if (const int rc = launch_book(r, prep_flags(mlong, plong) | (hot ? HOT : 0))) return rc;
+    if (hot) {
+        void* a[] = {&r->d};
+        SFP_CUDA(cudaLaunchKernel((const void*)r->k_hot_build, dim3(4 * sm_count()), dim3(SFP_TILE_HOST), a, 0, r->s));
+    }
+    return SFP_OK;
+}
+
 int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
     if (!r) return fail(SFP_EINVAL, "sfp_run_steps: NULL run");
     if (nsteps <= 0) return SFP_OK;
@@ -1432,15 +1555,16 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
     if (const int rc0 = cg.put()) return rc0;
     int64_t done = 0;
     const bool ml = long_tiles(r, r->mg.seg), pl = long_tiles(r, r->pg.seg);
-    if (const int rc0 = launch_book(r, prep_flags(ml, pl))) return rc0;
+    const bool hot = pl && nsteps >= HOT_MIN_STEPS && hot_store(r, cs);
+    if (const int rc0 = launch_first(r, ml, pl, hot)) return rc0;
     if (graph_chunk > 0 && nsteps >= graph_chunk) {
-        const int key = graph_chunk * 4 + (ml ? 2 : 0) + (pl ? 1 : 0);
+        const int key = graph_chunk * 8 + (hot ? 4 : 0) + (ml ? 2 : 0) + (pl ? 1 : 0);
         auto it = r->graphs.find(key);
         if (it == r->graphs.end()) {
             cudaGraph_t g;
             SFP_CUDA(cudaStreamBeginCapture(r->s, cudaStreamCaptureModeThreadLocal));
             int rc = SFP_OK;
-            for (int k = 0; k < graph_chunk && rc == SFP_OK; ++k) rc = launch_unit(r, r->s, nullptr, ml, pl);
+            for (int k = 0; k < graph_chunk && rc == SFP_OK; ++k) rc = launch_unit(r, r->s, nullptr, ml, pl, hot);
             cudaError_t e = cudaStreamEndCapture(r->s, &g);
             if (rc) return rc;
             if (e != cudaSuccess) return fail(SFP_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -1453,7 +1577,7 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
         for (; done + graph_chunk <= nsteps; done += graph_chunk) SFP_CUDA(cudaGraphLaunch(it->second, r->s));
     }
     for (; done < nsteps; ++done) {
-        int rc = launch_unit(r, r->s, nullptr, ml, pl);
+        int rc = launch_unit(r, r->s, nullptr, ml, pl, hot);
         if (rc) return rc;
     }
     if (const int rc = cg.done()) return rc;
@@ -1475,8 +1599,9 @@ int sfp_run_steps_timed(sfp_run* r, int64_t nsteps, float* kernel_ms, void* stre
     for (auto& e : ev)
         if (cudaEventCreate(&e) != cudaSuccess) rc = fail(SFP_ECUDA, "cudaEventCreate");
     const bool ml = long_tiles(r, r->mg.seg), pl = long_tiles(r, r->pg.seg);
-    if (rc == SFP_OK) rc = launch_book(r, prep_flags(ml, pl));
-    for (int64_t k = 0; k < nsteps && rc == SFP_OK; ++k) rc = launch_unit(r, r->s, &ev[6 * k], ml, pl);
+    const bool hot = pl && hot_store(r, cs);
+    if (rc == SFP_OK) rc = launch_first(r, ml, pl, hot);
+    for (int64_t k = 0; k < nsteps && rc == SFP_OK; ++k) rc = launch_unit(r, r->s, &ev[6 * k], ml, pl, hot);
     if (rc == SFP_OK) rc = cg.done();
     if (rc == SFP_OK && cudaStreamSynchronize(r->s) != cudaSuccess) rc = fail(SFP_ECUDA, "synchronize");
     const bool has[3] = {!r->mg.seg.empty(), !r->pg.seg.empty(), !r->dseg.empty()};
@@ -1598,10 +1723,23 @@ int sfp_run_resume(sfp_run* r, void* stream) {
     return SFP_OK;
 }
 
+int sfp_release_cached(void) {
+    std::vector<run_block> old;
+    {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        std::vector<run_block> keep;
+        for (const run_block& b : g_blocks) (b.bytes > kPoolKeep ? old : keep).push_back(b);
+        g_blocks.swap(keep);
+    }
+    for (const run_block& b : old) cudaFree(b.p);
+    return SFP_OK;
+}
+
 int sfp_run_destroy(sfp_run* r) {
     if (!r) return SFP_OK;
     const bool idle = r->s && cudaStreamSynchronize(r->s) == cudaSuccess;
     for (auto& kv : r->graphs) cudaGraphExecDestroy(kv.second);
+    r->blocks.push_back(r->hot_block);
     for (const run_block& b : r->blocks) {
         if (idle) block_put(b);
         else cudaFree(b.p);

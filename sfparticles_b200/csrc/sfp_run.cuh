@@ -59,6 +59,8 @@ struct sfp_step_state {
     int halted;                 // sticky: a destination lacked room (host regrows, resumes)
     int error;                  // sticky device error (SFP_DEV_*)
     int blocks_done;            // blocks of the running launch that are done (sfp_last_block)
+    int hot_ok;                 // the running call's store of hot photons holds all of them
+    int pad0;
     int append_wait;            // the step in slot `cur` stopped before writing its children (no room)
     long long particle_steps;   // sum over executed steps of all N_buffered
     // Photons fly straight: a photon segment stores each position as of the
@@ -107,6 +109,21 @@ struct sfp_group_dev {
     int pad;
 };
 
+// The photons whose pair test can pass somewhere in the field (sfp_step.cuh,
+// "hot photons"), copied out of their segments for one sfp_run_steps call:
+// entries start[s] .. start[s] + count[s] - 1 are segment s's, each its
+// photon's index, stored position and momentum (float32 form: as float32,
+// all that its tests read).  A converted photon's entry gets index SFP_HOT_DEAD.
+#define SFP_HOT_DEAD 0xFFFFFFFFu
+struct sfp_hot_dev {
+    double *x, *y, *z;
+    void *ux, *uy, *uz;           // float or double
+    unsigned int* idx;
+    const long long* start;       // [n_seg]
+    const long long* cap;         // [n_seg] room of a segment's entries
+    unsigned long long* count;    // [n_seg]
+};
+
 struct sfp_run_dev {
     const sfp_segment* seg;
     const sfp_instance* inst;
@@ -143,6 +160,7 @@ struct sfp_run_dev {
     // photons whose pair test no draw can pass skip the draw; then its prefix
     // maximum (as many floats)
     const float* pair_bound;
+    sfp_hot_dev hot;              // x NULL: no store
 };
 
 // chi bins of the pair-rate bound: the float's exponent and 3 mantissa bits

@@ -123,6 +123,7 @@ def _release_cached_blocks():
     done once a run has ended, never between its chunks."""
     import torch
     if torch.cuda.is_available() and torch.cuda.is_initialized():
+        _lib.call("sfp_release_cached")
         torch.cuda.empty_cache()
         if hasattr(torch._C, "_host_emptyCache"):
             torch._C._host_emptyCache()
