@@ -800,11 +800,8 @@ int sfp_inv_gamma(const double* ux, const double* uy, const double* uz, double* 
 #define SFP_T_M_STAGES 2
 #define SFP_T_P_STAGES 3
 #define SFP_T_P_MINB 3
-// a group of more particles than this has SFP_TILE_MAX-long tiles at every
-// step (the tile rule), so the long-tile kernels may run it
 // photon segments of a run that may keep a store of hot photons
 #define SFP_HOT_MAX_SEGS 1024
-#define SFP_LONG_TILE_POP ((long long)(SFP_TILE_MAX / 2) * SFP_TILE_TARGET)
 
 struct sfp_group_host {
     std::vector<int> seg;
@@ -989,11 +986,11 @@ static int run_carve(sfp_run* r, size_t bytes, void** out) {
 // tile counters a group needs at full capacity: each segment's longest
 // tiles plus the padding up to the next multiple of a super-tile, and at
 // least what the shorter tiles of a small population take (at most
-// SFP_TILE_TARGET tiles plus one partial tile and the padding per segment)
+// SFP_TILE_TARGET_M tiles plus one partial tile and the padding per segment)
 static long long tiles_for(const sfp_run* r, const std::vector<int>& segs) {
     long long t = 0;
     for (int s : segs) t += (r->segs[s].capacity + SFP_TILE_MAX - 1) / SFP_TILE_MAX + SFP_SUPER_TILE_HOST;
-    const long long small = SFP_TILE_TARGET + (long long)segs.size() * (SFP_SUPER_TILE_HOST + 1);
+    const long long small = SFP_TILE_TARGET_M + (long long)segs.size() * (SFP_SUPER_TILE_HOST + 1);
     return (t > small ? t : small) + 1;
 }
 
@@ -1086,10 +1083,11 @@ static void note_counts(sfp_run* r, const long long* nb) {
 }
 
 // whether every step from here on gives the group SFP_TILE_MAX-long tiles
-static bool long_tiles(const sfp_run* r, const std::vector<int>& segs) {
+// (the tile rule), so that the long-tile kernels may run it
+static bool long_tiles(const sfp_run* r, const std::vector<int>& segs, long long target) {
     long long n = 0;
     for (int s : segs) n += r->nb_lo.empty() ? 0 : r->nb_lo[s];
-    return n > SFP_LONG_TILE_POP;
+    return n > (long long)(SFP_TILE_MAX / 2) * target;
 }
 
 static int run_upload(sfp_run* r, const sfp_instance* inst, const int64_t* n_buffered) {
@@ -1554,7 +1552,7 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
     cfield_guard cg(r);
     if (const int rc0 = cg.put()) return rc0;
     int64_t done = 0;
-    const bool ml = long_tiles(r, r->mg.seg), pl = long_tiles(r, r->pg.seg);
+    const bool ml = long_tiles(r, r->mg.seg, SFP_TILE_TARGET_M), pl = long_tiles(r, r->pg.seg, SFP_TILE_TARGET);
     const bool hot = pl && nsteps >= HOT_MIN_STEPS && hot_store(r, cs);
     if (const int rc0 = launch_first(r, ml, pl, hot)) return rc0;
     if (graph_chunk > 0 && nsteps >= graph_chunk) {
@@ -1598,7 +1596,7 @@ int sfp_run_steps_timed(sfp_run* r, int64_t nsteps, float* kernel_ms, void* stre
     int rc = SFP_OK;
     for (auto& e : ev)
         if (cudaEventCreate(&e) != cudaSuccess) rc = fail(SFP_ECUDA, "cudaEventCreate");
-    const bool ml = long_tiles(r, r->mg.seg), pl = long_tiles(r, r->pg.seg);
+    const bool ml = long_tiles(r, r->mg.seg, SFP_TILE_TARGET_M), pl = long_tiles(r, r->pg.seg, SFP_TILE_TARGET);
     const bool hot = pl && hot_store(r, cs);
     if (rc == SFP_OK) rc = launch_first(r, ml, pl, hot);
     for (int64_t k = 0; k < nsteps && rc == SFP_OK; ++k) rc = launch_unit(r, r->s, &ev[6 * k], ml, pl, hot);

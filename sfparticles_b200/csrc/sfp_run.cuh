@@ -25,18 +25,23 @@
 #pragma once
 #include "sfp_types.h"
 
-// Tile length.  Each step the bookkeeping kernel gives each group the
-// shortest power-of-two tile from SFP_TILE_MIN to SFP_TILE_MAX particles
-// that cuts its population into at most SFP_TILE_TARGET tiles: a large
-// population keeps 1024-particle tiles (32 sub-steps of the copy ring per
-// ticket), a small one is spread over every warp of the grid instead of
-// running a few long tiles serially.  Results do not depend on the tile:
-// draws are keyed by particle index and children are written in index
-// order.  The tile counters hold SFP_TILE_TARGET tiles plus the segments'
-// padding at least, so the rule always fits.
+// Tile length.  Each step the bookkeeping gives each group the shortest
+// power-of-two tile from SFP_TILE_MIN to SFP_TILE_MAX particles that cuts
+// its population into at most SFP_TILE_TARGET tiles (massive group:
+// SFP_TILE_TARGET_M): a large population keeps 1024-particle tiles (32
+// sub-steps of the copy ring per ticket), a small one is spread over every
+// warp of the grid instead of running a few long tiles serially.  An e+-
+// takes ten times a photon's work, so its tiles are shorter: 1e6 e- as 3900
+// tiles of 256 gave 3552 resident warps one or two each, half of the last
+// round idle; as 15600 tiles of 64, 64 -> 50 us (float32 form, rejection
+// sampling), 183 -> 122 us (spin, learned sampler).  Results do not depend on
+// the tile: draws are keyed by particle index and children are written in
+// index order.  The tile counters hold SFP_TILE_TARGET_M tiles plus the
+// segments' padding at least, so the rule always fits.
 #define SFP_TILE_MIN 32
 #define SFP_TILE_MAX 1024
 #define SFP_TILE_TARGET 4096
+#define SFP_TILE_TARGET_M 16384
 
 // what a step is planned with: its time and number, and each group's tiles
 struct sfp_step_plan {

@@ -709,12 +709,12 @@ SFP_DEVICE_INLINE long long sfp_group_map(const sfp_group_dev& G, const long lon
 
 // the group's tile of the next step (SFP_TILE_MIN..SFP_TILE_MAX, a power of
 // two) and its tile map; a map too long for the counters takes a longer tile
-SFP_DEVICE_INLINE long long sfp_group_plan(const sfp_group_dev& G, const long long* nb, long long* start, int& tile) {
+SFP_DEVICE_INLINE long long sfp_group_plan(const sfp_group_dev& G, const long long* nb, long long* start, long long target, int& tile) {
     long long n = 0;
     for (int j = threadIdx.x & 31; j < G.n_seg; j += 32) n += nb[G.seg[j]];
     n = sfp_warp_sum64(n);
     int sh = 5;  // SFP_TILE_MIN
-    while ((1 << sh) < SFP_TILE_MAX && ((long long)SFP_TILE_TARGET << sh) < n) ++sh;
+    while ((1 << sh) < SFP_TILE_MAX && (target << sh) < n) ++sh;
     long long tiles = sfp_group_map(G, nb, sh, start);
     while (tiles > G.max_tiles && (1 << sh) < SFP_TILE_MAX) tiles = sfp_group_map(G, nb, ++sh, start);
     tile = 1 << sh;
@@ -878,8 +878,8 @@ __device__ __forceinline__ void sfp_step_end(const sfp_run_dev* __restrict__ R, 
     if (warp < 2) {
         int tile = SFP_TILE_MAX;
         const long long tiles =
-            warp == 0 ? sfp_group_plan(R->mg, nb, R->mg.tile_start + slot * (nm + 1), tile)
-                      : sfp_group_plan(R->pg, nb, R->pg.tile_start + slot * (np + 1), tile);
+            warp == 0 ? sfp_group_plan(R->mg, nb, R->mg.tile_start + slot * (nm + 1), SFP_TILE_TARGET_M, tile)
+                      : sfp_group_plan(R->pg, nb, R->pg.tile_start + slot * (np + 1), SFP_TILE_TARGET, tile);
         if (lane == 0) {
             Q.tiles[warp] = tiles;
             Q.tile[warp] = tile;
@@ -1969,12 +1969,15 @@ __device__ __forceinline__ void sfp_write_pair(const sfp_run_dev* __restrict__ R
     sfp_write_pair_child<FORM>(R->seg[S.pos_dest], bp, P, px, py, pz, d2 * pux, d2 * puy, d2 * puz, t, dt);
 }
 
+// (a unit of U tiles: they follow one another in a segment, so it is one
+// tile of U times the length whose first tile is `tile`)
 template <int FORM, bool MASSIVE>
 __device__ __forceinline__ void sfp_append_tile(const sfp_run_dev* __restrict__ R, const sfp_group_dev& G,
                                                 const sfp_step_view& V, long long tile, unsigned int c,
-                                                unsigned short* list, double dt, bool hot) {
+                                                unsigned short* list, double dt, bool hot, int U) {
     using namespace sfp;
     const int PT = MASSIVE ? V.mtile : V.ptile;
+    const int UT = PT * U;  // the unit's particles
     const long long* start = MASSIVE ? V.m_start : V.p_start;
     const int lane = threadIdx.x & 31;
     const long long s = tile / SFP_SUPER_TILE;
@@ -1986,7 +1989,7 @@ __device__ __forceinline__ void sfp_append_tile(const sfp_run_dev* __restrict__ 
     const double* __restrict__ P = sfp_field_params(R->inst[S.instance]);
     const long long N = V.n_buf[G.seg[pos]];
     const long long base = (tile - start[pos]) * (long long)PT;
-    const int len = (int)min(N - base, (long long)PT);  // the tile's particles
+    const int len = (int)min(N - base, (long long)UT);  // the unit's particles
     // chi per gamma no photon exceeds here, where new photons may enter the store of hot ones
     const float cpg = MASSIVE && hot ? sfp_chi_per_gamma(P) : -1.0f;
     // the tile's marked particles, in index order: lane q covers 16 flags per pass
@@ -2041,22 +2044,31 @@ __device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)busy_blocks * blockDim.x) >> 5;
-    // warp gw owns tiles gw, gw + nw, gw + 2 nw, ...: tiles with events
-    // (every massive tile in a cascade, a few photon tiles) spread over all
+    // a unit of the massive group: as many tiles as leave one unit or more for
+    // every warp, SFP_TILE_MAX particles at most
+    int U = 1;
+    while ((nm / U) > nw && V.mtile * U < SFP_TILE_MAX && U < SFP_SUPER_TILE) U <<= 1;
+    const long long um = (nm + U - 1) / U, units = um + np;
+    // warp gw owns units gw, gw + nw, gw + 2 nw, ...: those with events
+    // (every massive one in a cascade, a few photon tiles) spread over all
     // warps instead of queueing behind one warp per 32 neighbours
-    for (long long j0 = 0; gw + j0 * nw < n_all; j0 += 32) {
+    for (long long j0 = 0; gw + j0 * nw < units; j0 += 32) {
         const long long mine = gw + (j0 + lane) * nw;
         unsigned int mc = 0u;
-        if (mine < nm) mc = R->mg.tile_cnt[mine];
-        else if (mine < n_all) mc = R->pg.tile_cnt[mine - nm];
+        if (mine < um) {
+            const long long t0 = mine * U, t1 = min(nm, t0 + U);
+            for (long long k = t0; k < t1; ++k) mc += R->mg.tile_cnt[k];
+        } else if (mine < units) {
+            mc = R->pg.tile_cnt[mine - um];
+        }
         unsigned int busy = __ballot_sync(0xffffffffu, mc != 0u);
         while (busy) {
             const int b = __ffs(busy) - 1;
             busy &= busy - 1u;
             const long long tg = gw + (j0 + b) * nw;
             const unsigned int c = __shfl_sync(0xffffffffu, mc, b);
-            if (tg < nm) sfp_append_tile<FORM, true>(R, R->mg, V, tg, c, s_list[warp], dt, hot);
-            else sfp_append_tile<FORM, false>(R, R->pg, V, tg - nm, c, s_list[warp], dt, hot);
+            if (tg < um) sfp_append_tile<FORM, true>(R, R->mg, V, tg * U, c, s_list[warp], dt, hot, U);
+            else sfp_append_tile<FORM, false>(R, R->pg, V, tg - um, c, s_list[warp], dt, hot, 1);
         }
     }
 }
