@@ -214,6 +214,13 @@ int sfp_run_pending_need(sfp_run *r, int64_t *need);
 /* finish a step stopped with appends_pending: write and push its children,
  * fold its appends and advance t / step.  Asynchronous on the run's stream. */
 int sfp_run_resume(sfp_run *r, void *stream);
+/* kernels that the run's step calls have launched so far (graph replays included) */
+int sfp_run_launches(sfp_run *r, int64_t *count);
+/* Small populations run several steps per launch, with barriers between the
+ * launch's blocks; a wait at one gives up after two seconds and sets the device
+ * error SFP_DEV_BARRIER.  This launches a step in which one block never
+ * arrives, to exercise that path; synchronous; the run is of no use after. */
+int sfp_run_barrier_withheld(sfp_run *r, void *stream);
 int sfp_run_destroy(sfp_run *r);
 /* Destroyed runs leave their device blocks (bookkeeping, and the scratch
  * copies of photons that a call of several steps makes, 25 bytes per photon,

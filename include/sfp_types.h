@@ -125,5 +125,6 @@ typedef struct sfp_run_state {
 #define SFP_DEV_OK 0
 #define SFP_DEV_CAPACITY 2 /* more tiles than the run's counters hold */
 #define SFP_DEV_TILE 3     /* a long-tile kernel met a step planned with shorter tiles */
+#define SFP_DEV_BARRIER 4  /* a grid barrier of the small-population kernel ran out of time */
 
 #endif

@@ -66,7 +66,8 @@ class RunConfig(ctypes.Structure):
 SFP_QED_REJECTION, SFP_QED_OPTICAL_DEPTH = 0, 1
 SFP_FORM_FP64, SFP_FORM_FP32 = 0, 1
 SFP_FIELD_PARAMS = 16
-DEV_ERRORS = {2: "tile table too small", 3: "a long-tile step kernel met a step planned with shorter tiles"}
+DEV_ERRORS = {2: "tile table too small", 3: "a long-tile step kernel met a step planned with shorter tiles",
+              4: "a grid barrier of the small-population kernel ran out of time"}
 
 _SIGS = {
     "sfp_version": ([], ctypes.c_char_p),
@@ -118,6 +119,8 @@ _SIGS = {
     "sfp_table_od": ([c_i32, c_d, P, c_i64, P, c_i64, P, P, P, P], c_i32),
     "sfp_run_destroy": ([P], c_i32),
     "sfp_release_cached": ([], c_i32),
+    "sfp_run_launches": ([P, P], c_i32),
+    "sfp_run_barrier_withheld": ([P, P], c_i32),
 }
 
 _lib = None

@@ -802,6 +802,8 @@ int sfp_inv_gamma(const double* ux, const double* uy, const double* uz, double* 
 #define SFP_T_P_MINB 3
 // photon segments of a run that may keep a store of hot photons
 #define SFP_HOT_MAX_SEGS 1024
+// segments of a run that may take the one-launch kernel (sfp_step.cuh)
+#define SFP_SMALL_SEGS 64
 
 struct sfp_group_host {
     std::vector<int> seg;
@@ -952,7 +954,11 @@ struct sfp_run {
     long long hot_room = 0;                                     // entries it holds
     long long hot_refused = 0;                                  // entries that found no memory
     long long *d_hot_start = nullptr, *d_hot_cap = nullptr;
+    int64_t launches = 0;                                       // kernels of its steps so far (graph replays too)
     int grid_h = 0;
+    cudaKernel_t k_steps = nullptr;  // several steps of a small population in one cooperative launch
+    int grid_s = 0;                  // its grid (0: the device runs no cooperative launches)
+    size_t smem_s = 0;
     bool hot_f64 = false;
     int grid_m = 0, grid_p = 0, grid_a = 0, grid_mt = 0, grid_pt = 0;
     size_t smem_m = 0, smem_p = 0, smem_mt = 0, smem_pt = 0, smem_end = 0;
@@ -1329,8 +1335,6 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     // the end of a step uses the event launches' shared memory
     r->smem_end = sizeof(sfp_end_smem);
     for (size_t* q : {&r->smem_m, &r->smem_p, &r->smem_mt, &r->smem_pt}) *q = std::max(*q, r->smem_end);
-    if ((rc = run_alloc_tiles(r))) return cleanup(rc);
-    if ((rc = run_upload(r, inst, n_buffered))) return cleanup(rc);
     if (cfg->qed == SFP_QED_REJECTION && h.any_bw && h.pg.n_seg <= SFP_HOT_MAX_SEGS) {
         if ((rc = module_kernel(m, f64 ? "sfp_hot_fp64" : "sfp_hot_fp32", &r->k_hot)) ||
             (rc = module_kernel(m, f64 ? "sfp_hot_build_fp64" : "sfp_hot_build_fp32", &r->k_hot_build)))
@@ -1338,6 +1342,15 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
         // the hot kernel keeps its tile map where the photon kernel has its ring
         r->smem_p = std::max(r->smem_p, (size_t)h.ring_off + (h.pg.n_seg + 1) * sizeof(long long));
     }
+    if (n_seg <= SFP_SMALL_SEGS) {
+        if ((rc = module_kernel(m, ("sfp_steps_" + fq).c_str(), &r->k_steps))) return cleanup(rc);
+        const size_t ring = std::max((size_t)SFP_T_M_STAGES * h.m_stage_bytes, (size_t)SFP_T_P_STAGES * ((6 + od) * 256 + 32));
+        h.small_ring = (int)ring;
+        h.small_end_off = (int)(((size_t)h.m_ring_off + warps * ring + 127) / 128 * 128);
+        r->smem_s = (size_t)h.small_end_off + sizeof(sfp_end_smem);
+    }
+    if ((rc = run_alloc_tiles(r))) return cleanup(rc);
+    if ((rc = run_upload(r, inst, n_buffered))) return cleanup(rc);
     const size_t cap = 200 * 1024;
     if (r->smem_m > cap || r->smem_p > cap || r->smem_mt > cap || r->smem_pt > cap)
         return cleanup(fail(SFP_EINVAL, "QED tables and copy rings too large for shared memory"));
@@ -1355,6 +1368,17 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     r->grid_mt = persistent_grid(r->k_massive_t, r->smem_mt, t_minb);
     r->grid_pt = persistent_grid(r->k_photon_t, r->smem_pt, SFP_T_P_MINB);
     r->grid_a = persistent_grid(r->k_appends, 0, 2);
+    if (r->k_steps) {
+        int coop = 0;
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_now());
+        if (coop && r->smem_s <= cap && raise_dynamic_smem((const void*)r->k_steps, r->smem_s) == cudaSuccess) {
+            int per_sm = 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)r->k_steps, SFP_TILE_HOST,
+                                                              r->smem_s) == cudaSuccess)
+                r->grid_s = sm_count() * per_sm;
+        }
+        cudaGetLastError();
+    }
     if (r->k_hot) {
         if (raise_dynamic_smem((const void*)r->k_hot, r->smem_p) != cudaSuccess)
             return cleanup(fail(SFP_ECUDA, "cannot raise dynamic shared memory"));
@@ -1408,13 +1432,18 @@ struct cfield_guard {
 };
 
 // flags of the end of a step (sfp_step.cuh: SFP_PREP ... SFP_SCAN)
-enum { PREP = 1, PREP_M = 2, PREP_P = 4, FOLD = 8, SCAN = 16, HOT = 32 };
+enum { PREP = 1, PREP_M = 2, PREP_P = 4, FOLD = 8, SCAN = 16, HOT = 32, SMALL = 64, SMALL_SHIFT = 8 };
 
 // the bookkeeping of a call's first step (PREP), or the fold of a resumed one
 static int launch_book(sfp_run* r, int flags) {
     void* a[] = {&r->d, &flags};
     SFP_CUDA(cudaLaunchKernel((const void*)r->k_book, dim3(1), dim3(256), a, r->smem_end, r->s));
+    ++r->launches;
     return SFP_OK;
+}
+
+static int step_launches(const sfp_run* r, bool hot) {
+    return !r->mg.seg.empty() + !r->pg.seg.empty() + !r->dseg.empty() + hot;
 }
 
 static int prep_flags(bool mlong, bool plong) { return PREP | (mlong ? PREP_M : 0) | (plong ? PREP_P : 0); }
@@ -1463,6 +1492,16 @@ static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, 
     return SFP_OK;
 }
 
+// whether the caller captures its stream (or cannot be asked)
+static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return c != cudaStreamCaptureStatusNone;
+}
+
 // Hot photons: a call of at least HOT_MIN_STEPS steps whose photon group is
 // large keeps a store of them.  Building it reads every photon's momentum
 // (25 bytes), half of what one step of the full kernel reads, so it pays from
@@ -1470,19 +1509,15 @@ static int launch_unit(sfp_run* r, cudaStream_t s, cudaEvent_t* ev, bool mlong, 
 // are.  Below the long-tile population a step is bound by latency, not by the
 // photons it reads.
 constexpr int64_t HOT_MIN_STEPS = 4;
+// steps of one launch of the one-launch kernel
+constexpr int64_t SMALL_STEPS = 256;
 
 // room for the store at the current counts (5/8 of a segment's photons, new
 // ones included); false: the call does without (no memory to spare: the store
 // takes at most half of what is free)
 static bool hot_store(sfp_run* r, cudaStream_t caller) {
     if (!r->k_hot) return false;
-    // (a caller that captures its stream gets launches only)
-    cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(caller, &cap_st) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (cap_st != cudaStreamCaptureStatusNone) return false;
+    if (capturing(caller)) return false;  // a captured call gets launches only
     const bool f64 = r->k_hot && r->hot_f64;
     std::vector<long long> start(r->n_seg, 0), cap(r->n_seg, 0);
     long long n = 0;
@@ -1539,6 +1574,41 @@ static int launch_first(sfp_run* r, bool mlong, bool plong, bool hot) {
     if (hot) {
         void* a[] = {&r->d};
         SFP_CUDA(cudaLaunchKernel((const void*)r->k_hot_build, dim3(4 * sm_count()), dim3(SFP_TILE_HOST), a, 0, r->s));
+        ++r->launches;
+    }
+    return SFP_OK;
+}
+
+// Whether a call's steps go to the one-launch kernel: runs with events whose
+// groups are small.  Beyond, the three launches' better occupancy (three blocks
+// per SM, tiles by ticket) counts for more than the gaps between them.  Step
+// times, three launches / one launch: rejection sampling, 6e5 e- 284 / 226 us
+// (float64 form) and 124 / 83 (float32), 1.5e6 e- 491 / 485 and 189 / 161;
+// optical depth, 1.25e5 e+- 498 / 410 and 222 / 186, 3.75e5 e+- 735 / 773 and
+// 329 / 349.  Without events (a push alone) a step is one launch in any case.
+constexpr long long SMALL_M_RS = 1 << 20, SMALL_M_OD = 1 << 18;
+
+static bool small_run(const sfp_run* r, bool mlong, bool plong) {
+    if (r->grid_s <= 0 || r->dseg.empty() || mlong || plong) return false;
+    long long m = 0;
+    for (int s : r->mg.seg) m += r->nb_lo[s];
+    return m <= (r->h.qed == SFP_QED_REJECTION ? SMALL_M_RS : SMALL_M_OD);
+}
+
+// nsteps steps of a small population (withhold: one block never arrives at the first barrier)
+static int launch_small(sfp_run* r, int64_t nsteps, bool withhold = false) {
+    const int warps = r->grid_s * (SFP_TILE_HOST / 32);
+    const int small = SMALL | (warps << SMALL_SHIFT);
+    if (const int rc = launch_book(r, PREP | small)) return rc;
+    int end = FOLD | PREP | (r->dseg.empty() ? 0 : SCAN) | small;
+    for (int64_t done = 0; done < nsteps;) {
+        int n = (int)std::min<int64_t>(nsteps - done, SMALL_STEPS), arg = withhold ? -n : n;
+        SFP_CUDA(cudaMemsetAsync(&r->h.st->barrier, 0, sizeof(unsigned int), r->s));
+        void* a[] = {&r->d, &arg, &end};
+        SFP_CUDA(cudaLaunchCooperativeKernel((const void*)r->k_steps, dim3(r->grid_s), dim3(SFP_TILE_HOST), a, r->smem_s,
+                                             r->s));
+        ++r->launches;
+        done += n;
     }
     return SFP_OK;
 }
@@ -1553,6 +1623,13 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
     if (const int rc0 = cg.put()) return rc0;
     int64_t done = 0;
     const bool ml = long_tiles(r, r->mg.seg, SFP_TILE_TARGET_M), pl = long_tiles(r, r->pg.seg, SFP_TILE_TARGET);
+    if (small_run(r, ml, pl)) {
+        if (const int rc0 = launch_small(r, nsteps)) return rc0;
+        if (const int rc0 = cg.done()) return rc0;
+        SFP_CUDA(cudaEventRecord(r->ev_out, r->s));
+        SFP_CUDA(cudaStreamWaitEvent(cs, r->ev_out, 0));
+        return SFP_OK;
+    }
     const bool hot = pl && nsteps >= HOT_MIN_STEPS && hot_store(r, cs);
     if (const int rc0 = launch_first(r, ml, pl, hot)) return rc0;
     if (graph_chunk > 0 && nsteps >= graph_chunk) {
@@ -1572,11 +1649,15 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
             if (e != cudaSuccess) return fail(SFP_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
             it = r->graphs.emplace(key, ge).first;
         }
-        for (; done + graph_chunk <= nsteps; done += graph_chunk) SFP_CUDA(cudaGraphLaunch(it->second, r->s));
+        for (; done + graph_chunk <= nsteps; done += graph_chunk) {
+            SFP_CUDA(cudaGraphLaunch(it->second, r->s));
+            r->launches += graph_chunk * step_launches(r, hot);
+        }
     }
     for (; done < nsteps; ++done) {
         int rc = launch_unit(r, r->s, nullptr, ml, pl, hot);
         if (rc) return rc;
+        r->launches += step_launches(r, hot);
     }
     if (const int rc = cg.done()) return rc;
     SFP_CUDA(cudaEventRecord(r->ev_out, r->s));
@@ -1600,6 +1681,7 @@ int sfp_run_steps_timed(sfp_run* r, int64_t nsteps, float* kernel_ms, void* stre
     const bool hot = pl && hot_store(r, cs);
     if (rc == SFP_OK) rc = launch_first(r, ml, pl, hot);
     for (int64_t k = 0; k < nsteps && rc == SFP_OK; ++k) rc = launch_unit(r, r->s, &ev[6 * k], ml, pl, hot);
+    r->launches += nsteps * step_launches(r, hot);
     if (rc == SFP_OK) rc = cg.done();
     if (rc == SFP_OK && cudaStreamSynchronize(r->s) != cudaSuccess) rc = fail(SFP_ECUDA, "synchronize");
     const bool has[3] = {!r->mg.seg.empty(), !r->pg.seg.empty(), !r->dseg.empty()};
@@ -1715,9 +1797,30 @@ int sfp_run_resume(sfp_run* r, void* stream) {
     if (const int rc = launch_book(r, FOLD)) return rc;
     void* a[] = {&r->d};
     SFP_CUDA(cudaLaunchKernel((const void*)r->k_appends, dim3(r->grid_a), dim3(SFP_TILE_HOST), a, 0, r->s));
+    ++r->launches;
     if (const int rc = cg.done()) return rc;
     SFP_CUDA(cudaEventRecord(r->ev_out, r->s));
     SFP_CUDA(cudaStreamWaitEvent(cs, r->ev_out, 0));
+    return SFP_OK;
+}
+
+int sfp_run_launches(sfp_run* r, int64_t* count) {
+    if (!r || !count) return fail(SFP_EINVAL, "sfp_run_launches: NULL argument");
+    *count = r->launches;
+    return SFP_OK;
+}
+
+int sfp_run_barrier_withheld(sfp_run* r, void* stream) {
+    if (!r) return fail(SFP_EINVAL, "sfp_run_barrier_withheld: NULL run");
+    if (r->grid_s < 2) return fail(SFP_EINVAL, "sfp_run_barrier_withheld: the run has no one-launch kernel");
+    cudaStream_t cs = as_stream(stream);
+    SFP_CUDA(cudaEventRecord(r->ev_in, cs));
+    SFP_CUDA(cudaStreamWaitEvent(r->s, r->ev_in, 0));
+    cfield_guard cg(r);
+    if (const int rc = cg.put()) return rc;
+    if (const int rc = launch_small(r, 1, true)) return rc;
+    if (const int rc = cg.done()) return rc;
+    SFP_CUDA(cudaStreamSynchronize(r->s));
     return SFP_OK;
 }
 

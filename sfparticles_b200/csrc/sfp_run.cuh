@@ -65,7 +65,7 @@ struct sfp_step_state {
     int error;                  // sticky device error (SFP_DEV_*)
     int blocks_done;            // blocks of the running launch that are done (sfp_last_block)
     int hot_ok;                 // the running call's store of hot photons holds all of them
-    int pad0;
+    unsigned int barrier;       // arrivals at the grid barriers of the running launch (sfp_steps_body)
     int append_wait;            // the step in slot `cur` stopped before writing its children (no room)
     long long particle_steps;   // sum over executed steps of all N_buffered
     // Photons fly straight: a photon segment stores each position as of the
@@ -145,6 +145,8 @@ struct sfp_run_dev {
     int m_stage_bytes;          // massive kernel: bytes per ring stage (the run's widest segment layout)
     int ring_off;               // photon kernel: byte offset of its copy ring in dynamic smem
     int mlp_off;                // massive kernel: byte offset of the network weights in dynamic smem
+    int small_ring;             // one-launch kernel: bytes of a warp's ring (at m_ring_off)
+    int small_end_off;          // one-launch kernel: byte offset of sfp_end_smem in dynamic smem
     int pad1;
     const int* dseg;            // [n_dseg]
     sfp_group_dev mg;           // massive group

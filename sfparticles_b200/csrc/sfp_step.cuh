@@ -149,11 +149,27 @@ SFP_DEVICE_INLINE sfp_pc32 push_consts32(const sfp_segment& S, double t, double 
     return K;
 }
 
+// The float32 push's sums of products have their roundings spelled out: which
+// product of a sum a compiler fuses depends on the code around it, so the same
+// source rounded differently in the group kernels, the appends kernel and the
+// one-launch kernel, and one float32 ulp of a momentum is enough to turn a
+// later event.  Now every kernel rounds alike (a b - c d: the second product is
+// rounded first).
+SFP_DEVICE_INLINE float diff_of_products(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+SFP_DEVICE_INLINE float gamma_push(double ux, double uy, double uz) {
+    const float fx = sfp32::d2f(ux), fy = sfp32::d2f(uy), fz = sfp32::d2f(uz);
+    const float u2 = __fmaf_rn(fz, fz, __fmaf_rn(fx, fx, __fmul_rn(fy, fy)));
+    if (u2 < (float)(sfp32::kGammaSplit * sfp32::kGammaSplit)) return sqrtf(1.0f + u2);
+    return sfp32::d2f(sqrt(((1.0 + ux * ux) + uy * uy) + uz * uz));
+}
+
+// CHILD: a push in the step of an event (emitters and new pairs, appends kernel)
+template <bool CHILD>
 SFP_DEVICE_INLINE void push_massive32(double& x, double& y, double& z, double& ux, double& uy, double& uz,
                                       double& sx, double& sy, double& sz, const sfp_segment& S,
                                       const double* __restrict__ P, const sfp_pc32& K) {
     const float hc = K.hc;
-    float g = sfp32::gamma_of(ux, uy, uz, false);
+    float g = gamma_push(ux, uy, uz);
     float fx = sfp32::d2f(ux), fy = sfp32::d2f(uy), fz = sfp32::d2f(uz);
     float a = __fdividef(hc, g);
     x += (double)(a * fx);
@@ -164,7 +180,9 @@ SFP_DEVICE_INLINE void push_massive32(double& x, double& y, double& z, double& u
     const float eps = K.eps;
     const float bq = K.bq;
     const float ex = eps * F[0], ey = eps * F[1], ez = eps * F[2];
-    const float umx = fx + ex, umy = fy + ey, umz = fz + ez;
+    const float umx = CHILD ? __fadd_rn(fx, ex) : __fmaf_rn(eps, F[0], fx);
+    const float umy = CHILD ? __fadd_rn(fy, ey) : __fmaf_rn(eps, F[1], fy);
+    const float umz = CHILD ? __fadd_rn(fz, ez) : __fmaf_rn(eps, F[2], fz);
     float gm;
     if (g < (float)sfp32::kGammaSplit) {
         gm = sqrtf(1.0f + umx * umx + umy * umy + umz * umz);
@@ -190,12 +208,13 @@ SFP_DEVICE_INLINE void push_massive32(double& x, double& y, double& z, double& u
     }
     // Boris (inline.py:4-36) as u += 2 eps E + u' x S
     const float Tx = bq * F[3] * igm, Ty = bq * F[4] * igm, Tz = bq * F[5] * igm;
-    const float upx = umx + (umy * Tz - umz * Ty), upy = umy + (umz * Tx - umx * Tz), upz = umz + (umx * Ty - umy * Tx);
+    const float upx = umx + diff_of_products(umy, Tz, umz, Ty), upy = umy + diff_of_products(umz, Tx, umx, Tz),
+                upz = umz + diff_of_products(umx, Ty, umy, Tx);
     const float f2 = __fdividef(2.0f, 1.0f + Tx * Tx + Ty * Ty + Tz * Tz);
-    ux += (double)(2.0f * ex + f2 * (upy * Tz - upz * Ty));
-    uy += (double)(2.0f * ey + f2 * (upz * Tx - upx * Tz));
-    uz += (double)(2.0f * ez + f2 * (upx * Ty - upy * Tx));
-    g = sfp32::gamma_of(ux, uy, uz, false);
+    ux += (double)__fadd_rn(2.0f * ex, f2 * diff_of_products(upy, Tz, upz, Ty));
+    uy += (double)__fadd_rn(2.0f * ey, f2 * diff_of_products(upz, Tx, upx, Tz));
+    uz += (double)__fadd_rn(2.0f * ez, f2 * diff_of_products(upx, Ty, upy, Tx));
+    g = gamma_push(ux, uy, uz);
     if (S.rr == SFP_RR_LL || (S.rr == SFP_RR_CLL && !S.spin)) {  // inline.py:104-123
         fx = sfp32::d2f(ux); fy = sfp32::d2f(uy); fz = sfp32::d2f(uz);
         const float chi = sfp32::chi_of(F, fx, fy, fz, g);
@@ -615,6 +634,9 @@ __device__ __forceinline__ int sfp_find_group_pos(const long long* __restrict__ 
 #define SFP_SCAN 16
 // (sfp_book_kernel) the call keeps a store of hot photons, which is built next
 #define SFP_HOT 32
+// the next step runs in the one-launch kernel, with flags >> SFP_SMALL_SHIFT warps
+#define SFP_SMALL 64
+#define SFP_SMALL_SHIFT 8
 
 // a step as its kernels see it
 struct sfp_step_view {
@@ -681,68 +703,104 @@ SFP_DEVICE_INLINE void seg_scan_warp(unsigned int& h, uint4& v) {
     }
 }
 
-// the group's tile map for tiles of 2^sh particles, by a warp, from the next
+// tiles of pt particles (a multiple of 32) that n particles take
+SFP_DEVICE_INLINE long long sfp_tiles_of(long long n, int pt) {
+    if ((n >> 31) == 0) return (long long)(((unsigned int)n + (unsigned int)pt - 1u) / (unsigned int)pt);
+    return (n + pt - 1) / pt;
+}
+
+// the group's tile map for tiles of pt particles, by a warp, from the next
 // step's counts nb: each segment's tiles start at a multiple of
 // SFP_SUPER_TILE; returns the number of tiles
-SFP_DEVICE_INLINE long long sfp_group_map(const sfp_group_dev& G, const long long* nb, int sh, long long* start) {
+SFP_DEVICE_INLINE long long sfp_group_map(const int* seg, int n_seg, const long long* nb, int pt, long long* start) {
     const int lane = threadIdx.x & 31;
     long long carry = 0, end = 0;
-    for (int j0 = 0; j0 < G.n_seg; j0 += 32) {
+    for (int j0 = 0; j0 < n_seg; j0 += 32) {
         const int j = j0 + lane;
-        const long long n = j < G.n_seg ? nb[G.seg[j]] : 0;
-        const long long t = (n + (1 << sh) - 1) >> sh;
+        const long long t = j < n_seg ? sfp_tiles_of(nb[seg[j]], pt) : 0;
         const long long own = (t + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE * SFP_SUPER_TILE;
         long long inc = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
+        __syncwarp();
+        for (int o = 1; o < 32 && o < n_seg - j0; o <<= 1) {
             const long long u = __shfl_up_sync(0xffffffffu, inc, o);
             if (lane >= o) inc += u;
         }
         const long long at = carry + inc - own;
-        if (j < G.n_seg) start[j] = at;
-        end = __shfl_sync(0xffffffffu, at + t, min(31, G.n_seg - 1 - j0));
-        carry += __shfl_sync(0xffffffffu, inc, 31);
+        if (j < n_seg) start[j] = at;
+        const int last = min(31, n_seg - 1 - j0);
+        __syncwarp();
+        end = __shfl_sync(0xffffffffu, at + t, last);
+        carry += __shfl_sync(0xffffffffu, inc, last);
     }
-    if (lane == 0) start[G.n_seg] = end;
+    if (lane == 0) start[n_seg] = end;
+    __syncwarp();
     return end;
 }
 
-// the group's tile of the next step (SFP_TILE_MIN..SFP_TILE_MAX, a power of
-// two) and its tile map; a map too long for the counters takes a longer tile
-SFP_DEVICE_INLINE long long sfp_group_plan(const sfp_group_dev& G, const long long* nb, long long* start, long long target, int& tile) {
+// a group's population, by a warp
+SFP_DEVICE_INLINE long long sfp_group_count(const int* seg, int n_seg, const long long* nb) {
     long long n = 0;
-    for (int j = threadIdx.x & 31; j < G.n_seg; j += 32) n += nb[G.seg[j]];
-    n = sfp_warp_sum64(n);
-    int sh = 5;  // SFP_TILE_MIN
-    while ((1 << sh) < SFP_TILE_MAX && (target << sh) < n) ++sh;
-    long long tiles = sfp_group_map(G, nb, sh, start);
-    while (tiles > G.max_tiles && (1 << sh) < SFP_TILE_MAX) tiles = sfp_group_map(G, nb, ++sh, start);
-    tile = 1 << sh;
-    return tiles;
+    for (int j = threadIdx.x & 31; j < n_seg; j += 32) n += nb[seg[j]];
+    __syncwarp();
+    for (int o = 1; o < 32 && o < n_seg; o <<= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    return __shfl_sync(0xffffffffu, n, 0);
 }
 
-__device__ __forceinline__ void sfp_step_end(const sfp_run_dev* __restrict__ R, int flags, sfp_end_smem& Q) {
+// the group's tile of the next step (SFP_TILE_MIN..SFP_TILE_MAX, a power of
+// two), for n particles in at most `target` tiles
+SFP_DEVICE_INLINE int sfp_tile_rule(long long n, long long target) {
+    int pt = SFP_TILE_MIN;
+    while (pt < SFP_TILE_MAX && pt * target < n) pt <<= 1;
+    return pt;
+}
+
+// The one-launch kernel's tiles: about one per warp, so that no warp takes a
+// second one while others are done.  A warp's 32 e+- take several times as long
+// as its 32 photons (weight), so the tiles' lengths are the shares of that
+// sum; both are multiples of 32, not powers of two (1e4 e- and 1.4e5 photons:
+// tiles of 32 and 64 left 13 % of the warps a second tile).  Weights measured:
+// rejection sampling 3 (1e5 e-, 1.2e6 photons, float32 form: 37.0 us a step,
+// with 5 38.4, with 8 39.9), optical depth 8 (1e5 e+-, 8e5 photons: 186 us,
+// with 5 203, with 3 236).
+SFP_DEVICE_INLINE int sfp_small_tile(long long m, long long p, int warps, bool massive, int weight) {
+    const long long work = weight * ((m + 31) >> 5) + ((p + 31) >> 5);  // in sub-steps of photons
+    const int share = (int)min((long long)(SFP_TILE_MAX / 32), (work + warps - 1) / warps);
+    const int sub = massive ? (share + weight - 1) / weight : share;
+    return 32 * (sub < 1 ? 1 : sub);
+}
+
+// What both halves of a step's end share: the counts and appends of every
+// segment, in shared memory (or the run's scratch)
+struct sfp_end_data {
+    sfp_end_seg* seg;
+    unsigned long long* app;
+    long long* nb;
+};
+SFP_DEVICE_INLINE sfp_end_data sfp_end_arrays(const sfp_run_dev* __restrict__ R, sfp_end_smem& Q) {
+    const bool held = R->n_seg <= SFP_END_SEGS;
+    return sfp_end_data{held ? Q.seg : R->end_seg, held ? Q.app : R->end_app, held ? Q.nb : R->end_nb};
+}
+
+// loads the step's counts, and (SFP_SCAN) scans its events; false if a
+// destination lacks room
+__device__ __forceinline__ bool sfp_end_scan(const sfp_run_dev* __restrict__ R, int flags, sfp_end_smem& Q) {
     sfp_step_state* st = R->st;
     const int n = R->n_seg, nm = R->mg.n_seg, np = R->pg.n_seg;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool held = n <= SFP_END_SEGS;
-    sfp_end_seg* const seg = held ? Q.seg : R->end_seg;
-    unsigned long long* const app = held ? Q.app : R->end_app;
-    long long* const nb = held ? Q.nb : R->end_nb;
-    const int cur = st->cur, slot = (flags & SFP_FOLD) ? cur ^ 1 : cur;
-    const sfp_step_plan now = st->plan[cur];
-    const bool go = !(st->halted || st->error || st->append_wait);
+    const sfp_end_data E = sfp_end_arrays(R, Q);
+    sfp_end_seg* const seg = E.seg;
+    unsigned long long* const app = E.app;
+    long long* const nb = E.nb;
+    const int cur = st->cur;
+    const long long n_mtiles = st->plan[cur].n_mtiles, n_ptiles = st->plan[cur].n_ptiles;
     const long long *m_start = R->mg.tile_start + cur * (nm + 1), *p_start = R->pg.tile_start + cur * (np + 1);
     const long long* n_buf = R->n_buf_step + cur * n;
     __syncthreads();  // the dynamic shared memory's earlier users are done
     if (threadIdx.x == 0) Q.lacks = 0;
-    const int nsm = (int)((now.n_mtiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE);
-    const int nsp = (int)((now.n_ptiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE);
-    long long ps = 0;
+    const int nsm = (int)((n_mtiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE);
+    const int nsp = (int)((n_ptiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE);
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const long long at = (flags & SFP_FOLD) ? n_buf[k] : __ldcg(&R->n_buffered[k]);
-        ps += at;
-        nb[k] = at;
+        nb[k] = (flags & SFP_FOLD) ? n_buf[k] : __ldcg(&R->n_buffered[k]);
         app[k] = (flags & (SFP_FOLD | SFP_SCAN)) == SFP_FOLD ? __ldcg(&R->appended[k]) : 0ull;
         if (flags & SFP_SCAN) {  // entry k of the massive group's segments, then the photon group's
             const bool massive = k < nm;
@@ -793,6 +851,7 @@ __device__ __forceinline__ void sfp_step_end(const sfp_run_dev* __restrict__ R, 
                 v = sfp::u4_add(v, sfp::u4_one(seg[j].channel, s == s0 ? c0 : count(s)));
             }
         }
+        __syncwarp();  // the lanes' runs differ in length: together again before the shuffles
         seg_scan_warp(h, v);
         if (lane == 31) {
             Q.wh[warp] = h;
@@ -848,21 +907,67 @@ __device__ __forceinline__ void sfp_step_end(const sfp_run_dev* __restrict__ R, 
                 st->append_wait = 1;
                 st->halted = 1;
             }
-            return;
+            return false;
         }
     }
+    return true;
+}
+
+// folds the step (SFP_FOLD) and prepares the next one (SFP_PREP); nb and app
+// as sfp_end_scan left them.  small: the tiles of the one-launch kernel, whose
+// warps it names, or 0
+__device__ __forceinline__ void sfp_end_plan(const sfp_run_dev* __restrict__ R, int flags, sfp_end_smem& Q, int small) {
+    sfp_step_state* st = R->st;
+    const int n = R->n_seg, nm = R->mg.n_seg, np = R->pg.n_seg;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const sfp_end_data E = sfp_end_arrays(R, Q);
+    unsigned long long* const app = E.app;
+    long long* const nb = E.nb;
+    const int cur = st->cur, slot = (flags & SFP_FOLD) ? cur ^ 1 : cur;
+    const double t = (flags & SFP_FOLD) ? st->plan[cur].t + R->dt : st->t;
+    const long long step = (flags & SFP_FOLD) ? st->plan[cur].step + 1 : st->step;
+    const bool go = !(st->halted || st->error || st->append_wait);
     if (flags & SFP_FOLD) {
-        ps = sfp_warp_sum64(ps);
-        if (lane == 0) Q.ps[warp] = ps;
+        long long ps = 0;
         for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            ps += nb[k];
             nb[k] += (long long)app[k];
             R->n_buffered[k] = nb[k];
             R->appended[k] = 0ull;
         }
-        __syncthreads();
+        __syncwarp();
+        ps = sfp_warp_sum64(ps);
+        if (lane == 0) Q.ps[warp] = ps;
     }
-    const double t = (flags & SFP_FOLD) ? now.t + R->dt : st->t;
-    const long long step = (flags & SFP_FOLD) ? now.step + 1 : st->step;
+    __syncthreads();
+    if ((flags & SFP_PREP) && go && warp < 2) {
+        const int* seg_m = R->mg.seg;
+        const int* seg_p = R->pg.seg;
+        const bool massive = warp == 0;
+        const int* seg = massive ? seg_m : seg_p;
+        const int ns = massive ? nm : np;
+        long long* start = massive ? R->mg.tile_start + slot * (nm + 1) : R->pg.tile_start + slot * (np + 1);
+        const long long most = massive ? R->mg.max_tiles : R->pg.max_tiles;
+        int pt;
+        if (small)
+            pt = sfp_small_tile(sfp_group_count(seg_m, nm, nb), sfp_group_count(seg_p, np, nb), small, massive,
+                                R->qed == SFP_QED_REJECTION ? 3 : 8);
+        else
+            pt = sfp_tile_rule(sfp_group_count(seg, ns, nb), massive ? SFP_TILE_TARGET_M : SFP_TILE_TARGET);
+        // a map too long for the counters takes a longer tile
+        long long tiles = sfp_group_map(seg, ns, nb, pt, start);
+        while (tiles > most && pt < SFP_TILE_MAX) {
+            pt = min(2 * pt, SFP_TILE_MAX);
+            tiles = sfp_group_map(seg, ns, nb, pt, start);
+        }
+        if (lane == 0) {
+            Q.tiles[warp] = tiles;
+            Q.tile[warp] = pt;
+        }
+    }
+    if ((flags & SFP_PREP) && go)
+        for (int k = threadIdx.x; k < n; k += blockDim.x) R->n_buf_step[slot * n + k] = nb[k];
+    __syncthreads();
     if (threadIdx.x == 0) {
         if (flags & SFP_FOLD) {
             long long all = 0;
@@ -875,18 +980,6 @@ __device__ __forceinline__ void sfp_step_end(const sfp_run_dev* __restrict__ R, 
         if ((flags & SFP_PREP) && !go) st->skip = 1;
     }
     if (!(flags & SFP_PREP) || !go) return;
-    if (warp < 2) {
-        int tile = SFP_TILE_MAX;
-        const long long tiles =
-            warp == 0 ? sfp_group_plan(R->mg, nb, R->mg.tile_start + slot * (nm + 1), SFP_TILE_TARGET_M, tile)
-                      : sfp_group_plan(R->pg, nb, R->pg.tile_start + slot * (np + 1), SFP_TILE_TARGET, tile);
-        if (lane == 0) {
-            Q.tiles[warp] = tiles;
-            Q.tile[warp] = tile;
-        }
-    }
-    for (int k = threadIdx.x; k < n; k += blockDim.x) R->n_buf_step[slot * n + k] = nb[k];
-    __syncthreads();
     const long long m_tiles = Q.tiles[0], p_tiles = Q.tiles[1];
     const int mt = Q.tile[0], pt = Q.tile[1];
     int error = SFP_DEV_OK;
@@ -916,6 +1009,10 @@ __device__ __forceinline__ void sfp_step_end(const sfp_run_dev* __restrict__ R, 
     const long long zp = (p_tiles + SFP_SUPER_TILE - 1) / SFP_SUPER_TILE;
     for (long long k = threadIdx.x; k < zm; k += blockDim.x) R->mg.super_cnt[k] = 0u;
     for (long long k = threadIdx.x; k < zp; k += blockDim.x) R->pg.super_cnt[k] = 0u;
+}
+
+__device__ __forceinline__ void sfp_step_end(const sfp_run_dev* __restrict__ R, int flags, sfp_end_smem& Q) {
+    if (sfp_end_scan(R, flags, Q)) sfp_end_plan(R, flags, Q, (flags & SFP_SMALL) ? flags >> SFP_SMALL_SHIFT : 0);
 }
 
 extern "C" __global__ void __launch_bounds__(256) sfp_book_kernel(const sfp_run_dev* __restrict__ R, int flags) {
@@ -1132,7 +1229,7 @@ __device__ __forceinline__ unsigned int sfp_massive_tile(const sfp_run_dev* __re
             reinterpret_cast<double*>(D[NC + 1])[e] = delta;
         }
         if (FORM == SFP_FORM_FP64) push_massive(x, y, z, ux, uy, uz, sx, sy, sz, S, P, t, dt);
-        else push_massive32(x, y, z, ux, uy, uz, sx, sy, sz, S, P, K32);
+        else push_massive32<false>(x, y, z, ux, uy, uz, sx, sy, sz, S, P, K32);
         if (!ev && alive && push) {
             reinterpret_cast<double*>(D[0])[e] = x;
             reinterpret_cast<double*>(D[1])[e] = y;
@@ -1331,9 +1428,9 @@ __device__ __forceinline__ unsigned int sfp_pair_batch(const sfp_run_dev* __rest
             x = q.x[lane], y = q.y[lane], z = q.z[lane];
             ux = q.ux[lane], uy = q.uy[lane], uz = q.uz[lane];
         } else {  // the row again (indices only in the float64 form's queue)
-            x = reinterpret_cast<const double*>(D[0])[e], y = reinterpret_cast<const double*>(D[1])[e];
-            z = reinterpret_cast<const double*>(D[2])[e], ux = reinterpret_cast<const double*>(D[3])[e];
-            uy = reinterpret_cast<const double*>(D[4])[e], uz = reinterpret_cast<const double*>(D[5])[e];
+            x = __ldcg(reinterpret_cast<const double*>(D[0]) + e), y = __ldcg(reinterpret_cast<const double*>(D[1]) + e);
+            z = __ldcg(reinterpret_cast<const double*>(D[2]) + e), ux = __ldcg(reinterpret_cast<const double*>(D[3]) + e);
+            uy = __ldcg(reinterpret_cast<const double*>(D[4]) + e), uz = __ldcg(reinterpret_cast<const double*>(D[5]) + e);
         }
     }
     if (S.push) photon_shift<FORM>(x, y, z, ux, uy, uz, dt, lag);  // the stored position advanced to t
@@ -1365,6 +1462,130 @@ __device__ __forceinline__ void sfp_pair_enqueue(sfp_pair_queue<STATE>& q, unsig
         q.uy[k] = uy;
         q.uz[k] = uz;
     }
+}
+
+// one tile of photons (`left` particles of its segment from its first on);
+// returns its events
+template <int FORM, int QED, int STAGES, bool LONG>
+__device__ __forceinline__ unsigned int sfp_photon_tile(const sfp_run_dev* __restrict__ R, const sfp_qed_smem& T,
+                                                        const float* s_pb, const float* s_pbmax, const sfp_segment& S,
+                                                        char** desc, unsigned char* ring,
+                                                        sfp_pair_queue<FORM == SFP_FORM_FP32>& q, int PT,
+                                                        long long base, long long left, double t, double dt,
+                                                        unsigned int step, double lag) {
+    using namespace sfp;
+    constexpr int OD = QED == SFP_QED_OPTICAL_DEPTH ? 1 : 0;
+    constexpr bool QUEUE = QED == SFP_QED_REJECTION;
+    constexpr int NC = 6 + OD;
+    constexpr int SB = sfp_ring<NC>::STAGE_BYTES;
+    constexpr bool QSTATE = FORM == SFP_FORM_FP32;  // the queue holds the kept photons' state
+    const int lane = threadIdx.x & 31;
+    char* const* D = desc;
+    const sfp_instance& I = R->inst[S.instance];
+    const double* __restrict__ P = sfp_field_params(I);
+    const float cpg = QUEUE ? sfp_chi_per_gamma(P) : 0.0f;  // chi per gamma no photon exceeds here
+            // LONG: 32 sub-steps of 32 with compile-time bounds; else sub-steps up
+            // to the tile's last photon (`len`: the tile length or fewer at a
+            // segment's end)
+            const int len = LONG ? SFP_TILE_MAX : (int)min(left, (long long)PT);
+            const bool bw = S.bw != 0, push = S.push != 0;
+            __syncwarp();  // the previous tile's lanes are done with its descriptor, stages and queue
+            if (lane < NC + 2) desc[lane] = sfp_desc_slot<QED, false>(S, lane, base);
+            __syncwarp();
+            unsigned int cnt = 0, qn = 0;
+            const bool full = LONG ? left >= (long long)SFP_TILE_MAX : len == PT;
+            // full long tiles of the float32 form without optical depth: each
+            // lane's three component copies (components 2k + lane/16, k = 0..2)
+            // read from per-tile pointers held in registers, lanes 0-1 copy the
+            // flags; no descriptor reads per stage.  (The float64 form and the
+            // any-tile kernel have no registers to spare for them.)
+            constexpr bool REGPTR = FORM == SFP_FORM_FP32 && !OD && LONG;
+            const char* q0 = nullptr;
+            const char* q1 = nullptr;
+            const char* q2 = nullptr;
+            if (REGPTR && full) {
+                const int h = lane >> 4, o = 16 * (lane & 15);
+                q0 = D[h] + o;
+                q1 = D[2 + h] + o;
+                q2 = D[4 + h] + o;
+            }
+            auto issue = [&](int sb, unsigned char* dst) {
+                if (REGPTR && full) {
+                    const unsigned int off = (unsigned int)sb * 256u;
+                    sfp::cp_async16(dst + lane * 16, q0 + off, 16u);
+                    sfp::cp_async16(dst + (lane + 32) * 16, q1 + off, 16u);
+                    sfp::cp_async16(dst + (lane + 64) * 16, q2 + off, 16u);
+                    if (lane < 2) sfp::cp_async16(dst + (lane + 96) * 16, D[NC] + sb * 32 + 16 * lane, 16u);
+                    sfp::cp_async_commit();
+                } else if (full) {
+                    sfp_ring_issue_full<NC, OD>(D, sb, dst, lane);
+                } else {
+                    sfp_ring_issue<NC, OD>(D, sb, LONG ? left : (long long)len, dst, lane);
+                }
+            };
+    #pragma unroll
+            for (int k = 0; k < STAGES - 1; ++k) {
+                if (LONG || 32 * k < len) issue(k, ring + k * SB);
+                else cp_async_commit();  // a short tile: nothing to fetch, the group count stays
+            }
+    #pragma unroll 1
+            for (int sub = 0; LONG ? sub < SFP_TILE_MAX / 32 : 32 * sub < len; ++sub) {
+                __syncwarp();  // every lane has read the stage about to be refilled
+                const int nsub = sub + STAGES - 1;
+                if (LONG ? nsub < SFP_TILE_MAX / 32 : 32 * nsub < len) issue(nsub, ring + (nsub % STAGES) * SB);
+                else cp_async_commit();
+                cp_async_wait<STAGES - 1>();
+                __syncwarp();  // the stage of `sub` is complete for the whole warp
+                const unsigned char* stg = ring + (sub % STAGES) * SB;
+                const double* sd = reinterpret_cast<const double*>(stg);
+                const int e = sub * 32 + lane;  // photon index from the tile's first
+                const long long i = base + e;
+                const bool alive = (LONG ? e < left : e < len) && stg[NC * 256 + lane] == 0;
+                double x = sd[lane], y = sd[32 + lane], z = sd[64 + lane];
+                double ux = sd[96 + lane], uy = sd[128 + lane], uz = sd[160 + lane];
+                // the step's push is carried by the epoch (pos_epoch), so a photon
+                // that does not convert stores nothing
+                if (QUEUE) {
+                    // from its energy alone, whether a photon's pair test can pass
+                    // anywhere in the field; those that can go, with their stored
+                    // state, to the queue, where the position at t, the field and
+                    // the rate bound are evaluated for full warps
+                    const bool keep = alive & bw & push & sfp_pair_reachable<FORM>(cpg, s_pbmax, ux, uy, uz, dt);
+                    // kept photons fill the queue; a full queue is tested at once and
+                    // the sub-step's remaining kept photons start the next one
+                    const unsigned int kb = __ballot_sync(0xffffffffu, keep);
+                    const unsigned int slot = qn + __popc(kb & ((1u << lane) - 1u)), nk = __popc(kb);
+                    if (keep && slot < 32u) sfp_pair_enqueue(q, slot, e, x, y, z, ux, uy, uz);
+                    if (qn + nk >= 32u) {
+                        __syncwarp();  // the queue entries are written
+                        cnt += sfp_pair_batch<FORM, QSTATE>(R, T, s_pb, S, I, P, D, q, 32u, base, t, dt, step, lag);
+                        __syncwarp();  // every lane has read its entry
+                        if (keep && slot >= 32u) sfp_pair_enqueue(q, slot - 32u, e, x, y, z, ux, uy, uz);
+                        qn = qn + nk - 32u;
+                    } else {
+                        qn += nk;
+                    }
+                } else {
+                    double tau = OD ? sd[192 + lane] : 0.0;
+                    bool ev = false;
+                    double delta = 0.0;
+                    if (push) photon_shift<FORM>(x, y, z, ux, uy, uz, dt, lag);  // the position at t
+                    if (alive && bw)
+                        ev = sfp_pair_event<FORM, QED>(R, T, S, I, P, x, y, z, ux, uy, uz, t, step, i, tau, delta);
+                    if (ev) {
+                        // converted photons are pruned, not pushed (cpu.py:190); marked until their pairs are written
+                        reinterpret_cast<unsigned char*>(D[NC])[e] = SFP_MARK;
+                        reinterpret_cast<double*>(D[NC + 1])[e] = delta;
+                    }
+                    if (OD && alive && bw && D[6]) reinterpret_cast<double*>(D[6])[e] = tau;
+                    cnt += __popc(__ballot_sync(0xffffffffu, ev));
+                }
+            }
+            if (QUEUE && qn) {  // the tile's last kept photons
+                __syncwarp();
+                cnt += sfp_pair_batch<FORM, QSTATE>(R, T, s_pb, S, I, P, D, q, qn, base, t, dt, step, lag);
+            }
+    return cnt;
 }
 
 template <int FORM, int QED, int STAGES, bool LONG>
@@ -1405,7 +1626,6 @@ __device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ 
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char* ring = reinterpret_cast<unsigned char*>(s_tab) + R->ring_off + (size_t)warp * STAGES * SB;
-    char* const* D = s_desc[warp];
     sfp_pair_queue<QSTATE>& q = s_q[QUEUE ? warp : 0];
 
     int tk = 0;
@@ -1415,10 +1635,6 @@ __device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ 
         if (lane == 0) tk = atomicAdd(&st->pticket, 1);  // next ticket, in flight during this tile
         const int pos = sfp_find_group_pos(V.p_start, R->pg.n_seg, tile);
         const int si = R->pg.seg[pos];
-        const sfp_segment& S = R->seg[si];
-        const sfp_instance& I = R->inst[S.instance];
-        const double* __restrict__ P = sfp_field_params(I);
-        const float cpg = QUEUE ? sfp_chi_per_gamma(P) : 0.0f;  // chi per gamma no photon exceeds here
         const long long N = V.n_buf[si];
         const long long base = (tile - V.p_start[pos]) * (long long)PT;
         if (base >= N) {  // alignment padding between segments: no photons
@@ -1426,108 +1642,8 @@ __device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ 
             tile = __shfl_sync(0xffffffffu, tk, 0);
             continue;
         }
-        // LONG: 32 sub-steps of 32 with compile-time bounds; else sub-steps up
-        // to the tile's last photon (`len`: the tile length or fewer at a
-        // segment's end)
-        const long long left = N - base;
-        const int len = LONG ? SFP_TILE_MAX : (int)min(left, (long long)PT);
-        const bool bw = S.bw != 0, push = S.push != 0;
-        __syncwarp();  // the previous tile's lanes are done with its descriptor, stages and queue
-        if (lane < NC + 2) s_desc[warp][lane] = sfp_desc_slot<QED, false>(S, lane, base);
-        __syncwarp();
-        unsigned int cnt = 0, qn = 0;
-        const bool full = LONG ? left >= (long long)SFP_TILE_MAX : len == PT;
-        // full long tiles of the float32 form without optical depth: each
-        // lane's three component copies (components 2k + lane/16, k = 0..2)
-        // read from per-tile pointers held in registers, lanes 0-1 copy the
-        // flags; no descriptor reads per stage.  (The float64 form and the
-        // any-tile kernel have no registers to spare for them.)
-        constexpr bool REGPTR = FORM == SFP_FORM_FP32 && !OD && LONG;
-        const char* q0 = nullptr;
-        const char* q1 = nullptr;
-        const char* q2 = nullptr;
-        if (REGPTR && full) {
-            const int h = lane >> 4, o = 16 * (lane & 15);
-            q0 = D[h] + o;
-            q1 = D[2 + h] + o;
-            q2 = D[4 + h] + o;
-        }
-        auto issue = [&](int sb, unsigned char* dst) {
-            if (REGPTR && full) {
-                const unsigned int off = (unsigned int)sb * 256u;
-                sfp::cp_async16(dst + lane * 16, q0 + off, 16u);
-                sfp::cp_async16(dst + (lane + 32) * 16, q1 + off, 16u);
-                sfp::cp_async16(dst + (lane + 64) * 16, q2 + off, 16u);
-                if (lane < 2) sfp::cp_async16(dst + (lane + 96) * 16, D[NC] + sb * 32 + 16 * lane, 16u);
-                sfp::cp_async_commit();
-            } else if (full) {
-                sfp_ring_issue_full<NC, OD>(D, sb, dst, lane);
-            } else {
-                sfp_ring_issue<NC, OD>(D, sb, LONG ? left : (long long)len, dst, lane);
-            }
-        };
-#pragma unroll
-        for (int k = 0; k < STAGES - 1; ++k) {
-            if (LONG || 32 * k < len) issue(k, ring + k * SB);
-            else cp_async_commit();  // a short tile: nothing to fetch, the group count stays
-        }
-#pragma unroll 1
-        for (int sub = 0; LONG ? sub < SFP_TILE_MAX / 32 : 32 * sub < len; ++sub) {
-            __syncwarp();  // every lane has read the stage about to be refilled
-            const int nsub = sub + STAGES - 1;
-            if (LONG ? nsub < SFP_TILE_MAX / 32 : 32 * nsub < len) issue(nsub, ring + (nsub % STAGES) * SB);
-            else cp_async_commit();
-            cp_async_wait<STAGES - 1>();
-            __syncwarp();  // the stage of `sub` is complete for the whole warp
-            const unsigned char* stg = ring + (sub % STAGES) * SB;
-            const double* sd = reinterpret_cast<const double*>(stg);
-            const int e = sub * 32 + lane;  // photon index from the tile's first
-            const long long i = base + e;
-            const bool alive = (LONG ? e < left : e < len) && stg[NC * 256 + lane] == 0;
-            double x = sd[lane], y = sd[32 + lane], z = sd[64 + lane];
-            double ux = sd[96 + lane], uy = sd[128 + lane], uz = sd[160 + lane];
-            // the step's push is carried by the epoch (pos_epoch), so a photon
-            // that does not convert stores nothing
-            if (QUEUE) {
-                // from its energy alone, whether a photon's pair test can pass
-                // anywhere in the field; those that can go, with their stored
-                // state, to the queue, where the position at t, the field and
-                // the rate bound are evaluated for full warps
-                const bool keep = alive & bw & push & sfp_pair_reachable<FORM>(cpg, s_pbmax, ux, uy, uz, dt);
-                // kept photons fill the queue; a full queue is tested at once and
-                // the sub-step's remaining kept photons start the next one
-                const unsigned int kb = __ballot_sync(0xffffffffu, keep);
-                const unsigned int slot = qn + __popc(kb & ((1u << lane) - 1u)), nk = __popc(kb);
-                if (keep && slot < 32u) sfp_pair_enqueue(q, slot, e, x, y, z, ux, uy, uz);
-                if (qn + nk >= 32u) {
-                    __syncwarp();  // the queue entries are written
-                    cnt += sfp_pair_batch<FORM, QSTATE>(R, T, s_pb, S, I, P, D, q, 32u, base, t, dt, step, lag);
-                    __syncwarp();  // every lane has read its entry
-                    if (keep && slot >= 32u) sfp_pair_enqueue(q, slot - 32u, e, x, y, z, ux, uy, uz);
-                    qn = qn + nk - 32u;
-                } else {
-                    qn += nk;
-                }
-            } else {
-                double tau = OD ? sd[192 + lane] : 0.0;
-                bool ev = false;
-                double delta = 0.0;
-                if (push) photon_shift<FORM>(x, y, z, ux, uy, uz, dt, lag);  // the position at t
-                if (alive && bw)
-                    ev = sfp_pair_event<FORM, QED>(R, T, S, I, P, x, y, z, ux, uy, uz, t, step, i, tau, delta);
-                if (ev) {
-                    // converted photons are pruned, not pushed (cpu.py:190); marked until their pairs are written
-                    reinterpret_cast<unsigned char*>(D[NC])[e] = SFP_MARK;
-                    reinterpret_cast<double*>(D[NC + 1])[e] = delta;
-                }
-                if (OD && alive && bw && D[6]) reinterpret_cast<double*>(D[6])[e] = tau;
-                cnt += __popc(__ballot_sync(0xffffffffu, ev));
-            }
-        }
-        if (QUEUE && qn) {  // the tile's last kept photons
-            __syncwarp();
-            cnt += sfp_pair_batch<FORM, QSTATE>(R, T, s_pb, S, I, P, D, q, qn, base, t, dt, step, lag);
-        }
+        const unsigned int cnt = sfp_photon_tile<FORM, QED, STAGES, LONG>(
+            R, T, s_pb, s_pbmax, R->seg[si], s_desc[warp], ring, q, PT, base, N - base, t, dt, step, lag);
         if (lane == 0) {
             R->pg.tile_cnt[tile] = cnt;
             if (cnt) atomicAdd(&R->pg.super_cnt[tile / SFP_SUPER_TILE], cnt);
@@ -1853,7 +1969,7 @@ __device__ __forceinline__ void sfp_write_pair_child(const sfp_segment& D, long 
     if (D.push) {
         double sx = 0.0, sy = 0.0, sz = 0.0;
         if (FORM == SFP_FORM_FP64) push_massive(x, y, z, ux, uy, uz, sx, sy, sz, D, P, t, dt);
-        else push_massive32(x, y, z, ux, uy, uz, sx, sy, sz, D, P, push_consts32(D, t, dt));
+        else push_massive32<true>(x, y, z, ux, uy, uz, sx, sy, sz, D, P, push_consts32(D, t, dt));
     }
     D.x[slot] = x;
     D.y[slot] = y;
@@ -1878,9 +1994,9 @@ __device__ __forceinline__ void sfp_write_photon(const sfp_run_dev* __restrict__
     const double t = V.t, lag = V.lag;
     const sfp_segment& D = R->seg[S.photon_dest];
     const long long slot = V.n_buf[S.photon_dest] + pre + rank;
-    double x = S.x[i], y = S.y[i], z = S.z[i];
-    double ux = S.ux[i], uy = S.uy[i], uz = S.uz[i];
-    const double d = S.delta[i];
+    double x = __ldcg(S.x + i), y = __ldcg(S.y + i), z = __ldcg(S.z + i);
+    double ux = __ldcg(S.ux + i), uy = __ldcg(S.uy + i), uz = __ldcg(S.uz + i);
+    const double d = __ldcg(S.delta + i);
     double cx = x, cy = y, cz = z;
     const double cux = d * ux, cuy = d * uy, cuz = d * uz;
     // the child is pushed in its creation step (simulation.py:117-121): at
@@ -1915,19 +2031,20 @@ __device__ __forceinline__ void sfp_write_photon(const sfp_run_dev* __restrict__
     }
     if (S.rr == SFP_RR_PHOTON) {
         const double f = 1.0 - d;
-        ux = ux * f;
-        uy = uy * f;
-        uz = uz * f;
+        // (a product of its own, not fused into the push: every kernel rounds alike)
+        ux = __dmul_rn(ux, f);
+        uy = __dmul_rn(uy, f);
+        uz = __dmul_rn(uz, f);
     }
     if (S.push) {
         double sx = 0.0, sy = 0.0, sz = 0.0;
         if (S.spin) {
-            sx = S.sx[i];
-            sy = S.sy[i];
-            sz = S.sz[i];
+            sx = __ldcg(S.sx + i);
+            sy = __ldcg(S.sy + i);
+            sz = __ldcg(S.sz + i);
         }
         if (FORM == SFP_FORM_FP64) push_massive(x, y, z, ux, uy, uz, sx, sy, sz, S, P, t, dt);
-        else push_massive32(x, y, z, ux, uy, uz, sx, sy, sz, S, P, push_consts32(S, t, dt));
+        else push_massive32<true>(x, y, z, ux, uy, uz, sx, sy, sz, S, P, push_consts32(S, t, dt));
         S.x[i] = x;
         S.y[i] = y;
         S.z[i] = z;
@@ -1950,9 +2067,9 @@ __device__ __forceinline__ void sfp_write_pair(const sfp_run_dev* __restrict__ R
                                                long long rank, long long pre, const double* __restrict__ P,
                                                const sfp_step_view& V, double dt) {
     const double t = V.t, lag = V.lag;
-    const double d = S.delta[i];
-    double px = S.x[i], py = S.y[i], pz = S.z[i];
-    const double pux = S.ux[i], puy = S.uy[i], puz = S.uz[i];
+    const double d = __ldcg(S.delta + i);
+    double px = __ldcg(S.x + i), py = __ldcg(S.y + i), pz = __ldcg(S.z + i);
+    const double pux = __ldcg(S.ux + i), puy = __ldcg(S.uy + i), puz = __ldcg(S.uz + i);
     // the converted photon at t, written out: it is pruned, and pruned
     // photons keep their stored position (no later advance)
     if (S.push) {
@@ -1964,9 +2081,11 @@ __device__ __forceinline__ void sfp_write_pair(const sfp_run_dev* __restrict__ R
     S.pruned[i] = 1;
     const long long be = V.n_buf[S.ele_dest] + pre + rank;
     const long long bp = V.n_buf[S.pos_dest] + pre + rank;
-    sfp_write_pair_child<FORM>(R->seg[S.ele_dest], be, P, px, py, pz, d * pux, d * puy, d * puz, t, dt);
+    sfp_write_pair_child<FORM>(R->seg[S.ele_dest], be, P, px, py, pz, __dmul_rn(d, pux), __dmul_rn(d, puy),
+                               __dmul_rn(d, puz), t, dt);
     const double d2 = 1.0 - d;
-    sfp_write_pair_child<FORM>(R->seg[S.pos_dest], bp, P, px, py, pz, d2 * pux, d2 * puy, d2 * puz, t, dt);
+    sfp_write_pair_child<FORM>(R->seg[S.pos_dest], bp, P, px, py, pz, __dmul_rn(d2, pux), __dmul_rn(d2, puy),
+                               __dmul_rn(d2, puz), t, dt);
 }
 
 // (a unit of U tiles: they follow one another in a segment, so it is one
@@ -1982,8 +2101,8 @@ __device__ __forceinline__ void sfp_append_tile(const sfp_run_dev* __restrict__ 
     const int lane = threadIdx.x & 31;
     const long long s = tile / SFP_SUPER_TILE;
     unsigned int part = 0u;
-    for (long long k = s * SFP_SUPER_TILE + lane; k < tile; k += 32) part += G.tile_cnt[k];
-    const long long pre = G.super_pre[s] + (long long)warp_sum(part);
+    for (long long k = s * SFP_SUPER_TILE + lane; k < tile; k += 32) part += __ldcg(&G.tile_cnt[k]);
+    const long long pre = __ldcg(&G.super_pre[s]) + (long long)warp_sum(part);
     const int pos = sfp_find_group_pos(start, G.n_seg, tile);
     const sfp_segment& S = R->seg[G.seg[pos]];
     const double* __restrict__ P = sfp_field_params(R->inst[S.instance]);
@@ -1999,10 +2118,10 @@ __device__ __forceinline__ void sfp_append_tile(const sfp_run_dev* __restrict__ 
         const unsigned char* f = S.pruned + base + e0;
         unsigned int m = 0u;
         if (e0 + 16 <= len) {
-            m = marks16(*reinterpret_cast<const uint4*>(f));
+            m = marks16(__ldcg(reinterpret_cast<const uint4*>(f)));
         } else {
             for (int b = 0; b < 16; ++b)
-                if (e0 + b < len && f[b] == SFP_MARK) m |= 1u << b;
+                if (e0 + b < len && __ldcg(f + b) == SFP_MARK) m |= 1u << b;
         }
         const unsigned int k = __popc(m);
         const unsigned int inc = warp_incl_scan(k);
@@ -2029,25 +2148,17 @@ __device__ __forceinline__ void sfp_append_tile(const sfp_run_dev* __restrict__ 
     __syncwarp();  // the list is read before the next tile rewrites it
 }
 
+// the step of view V: children of every unit dealt to warp gw of nw
 template <int FORM>
-__device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__ R) {
-    __shared__ unsigned short s_list[SFP_TILE / 32][SFP_TILE_MAX];
-    const sfp_step_state* st = R->st;
-    if (st->skip || st->halted) return;
-    const sfp_step_view V = sfp_view(R, st->cur ^ 1);  // the step whose events were scanned
+__device__ __forceinline__ void sfp_append_units(const sfp_run_dev* __restrict__ R, const sfp_step_view& V,
+                                                 unsigned short* list, long long gw, long long nw, double dt,
+                                                 bool hot) {
+    const int lane = threadIdx.x & 31;
     const long long nm = R->any_rad ? V.n_mtiles : 0, np = R->any_bw ? V.n_ptiles : 0;
-    const long long n_all = nm + np;
-    const unsigned int busy_blocks = sfp_busy_blocks(n_all, gridDim.x);
-    if (blockIdx.x >= busy_blocks) return;
-    const bool hot = st->hot_ok != 0;
-    const double dt = R->dt;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)busy_blocks * blockDim.x) >> 5;
     // a unit of the massive group: as many tiles as leave one unit or more for
     // every warp, SFP_TILE_MAX particles at most
     int U = 1;
-    while ((nm / U) > nw && V.mtile * U < SFP_TILE_MAX && U < SFP_SUPER_TILE) U <<= 1;
+    while (nm / U > nw && V.mtile * U * 2 <= SFP_TILE_MAX && U < SFP_SUPER_TILE) U <<= 1;
     const long long um = (nm + U - 1) / U, units = um + np;
     // warp gw owns units gw, gw + nw, gw + 2 nw, ...: those with events
     // (every massive one in a cascade, a few photon tiles) spread over all
@@ -2057,9 +2168,9 @@ __device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__
         unsigned int mc = 0u;
         if (mine < um) {
             const long long t0 = mine * U, t1 = min(nm, t0 + U);
-            for (long long k = t0; k < t1; ++k) mc += R->mg.tile_cnt[k];
+            for (long long k = t0; k < t1; ++k) mc += __ldcg(&R->mg.tile_cnt[k]);
         } else if (mine < units) {
-            mc = R->pg.tile_cnt[mine - um];
+            mc = __ldcg(&R->pg.tile_cnt[mine - um]);
         }
         unsigned int busy = __ballot_sync(0xffffffffu, mc != 0u);
         while (busy) {
@@ -2067,9 +2178,200 @@ __device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__
             busy &= busy - 1u;
             const long long tg = gw + (j0 + b) * nw;
             const unsigned int c = __shfl_sync(0xffffffffu, mc, b);
-            if (tg < um) sfp_append_tile<FORM, true>(R, R->mg, V, tg * U, c, s_list[warp], dt, hot, U);
-            else sfp_append_tile<FORM, false>(R, R->pg, V, tg - um, c, s_list[warp], dt, hot, 1);
+            if (tg < um) sfp_append_tile<FORM, true>(R, R->mg, V, tg * U, c, list, dt, hot, U);
+            else sfp_append_tile<FORM, false>(R, R->pg, V, tg - um, c, list, dt, hot, 1);
         }
+    }
+}
+
+template <int FORM>
+__device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__ R) {
+    __shared__ unsigned short s_list[SFP_TILE / 32][SFP_TILE_MAX];
+    const sfp_step_state* st = R->st;
+    if (st->skip || st->halted) return;
+    const sfp_step_view V = sfp_view(R, st->cur ^ 1);  // the step whose events were scanned
+    const long long n_all = (R->any_rad ? V.n_mtiles : 0) + (R->any_bw ? V.n_ptiles : 0);
+    const unsigned int busy_blocks = sfp_busy_blocks(n_all, gridDim.x);
+    if (blockIdx.x >= busy_blocks) return;
+    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nw = ((long long)busy_blocks * blockDim.x) >> 5;
+    sfp_append_units<FORM>(R, V, s_list[threadIdx.x >> 5], gw, nw, R->dt, st->hot_ok != 0);
+}
+
+// ---------------------------------------------------------------------------
+// Small populations: several steps in one launch (a cooperative one, every
+// block resident).  A step of 1e4 e- spent 53 us in three launches of which
+// no block had more than a few tiles: launch gaps (2 us each), tables staged
+// anew (2-4 us each), and the rest one tile's chain of dependent operations.
+// Here the tables are staged once, and a step is: every warp's tiles of both
+// groups; a grid barrier (2 us); the event scan in block 0; a barrier; the
+// children, while block 0 plans the next step; a barrier.  Particles, flags
+// and counts that other blocks write are read past L1 (cp.async.cg, __ldcg).
+// A barrier gives up after SFP_BARRIER_NS: the step's error is set and every
+// block returns.  Step times against three launches, float64 / float32 form:
+// 1e3 e- 49 -> 31 / 34 -> 22 us, 1e4 63 -> 40 / 41 -> 23, 1e5 151 -> 95 /
+// 73 -> 37.
+// ---------------------------------------------------------------------------
+#define SFP_BARRIER_NS 2000000000ull  // 400 times the longest launch of the populations it serves
+// segments of a run that may take this kernel
+#define SFP_SMALL_SEGS 64
+
+__device__ __forceinline__ unsigned long long sfp_clock_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// all blocks of the launch; `round` counts the barriers of the launch from 1.
+// False (in every thread of the block) once the wait has run out.
+__device__ __forceinline__ bool sfp_grid_barrier(sfp_step_state* st, unsigned int round) {
+    __shared__ int s_in;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned int want = round * gridDim.x;
+        __threadfence();
+        atomicAdd(&st->barrier, 1u);
+        int in = 1;
+        unsigned int v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->barrier) : "memory");
+        if (v < want) {
+            const unsigned long long t0 = sfp_clock_ns();
+            for (unsigned int k = 1; v < want; ++k) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->barrier) : "memory");
+                if ((k & 255u) == 0u && v < want && sfp_clock_ns() - t0 > SFP_BARRIER_NS) {
+                    in = 0;
+                    break;
+                }
+            }
+        }
+        if (!in) st->error = SFP_DEV_BARRIER;
+        __threadfence();
+        s_in = in;
+    }
+    __syncthreads();
+    return s_in != 0;
+}
+
+// the massive group's tile as a function of its own: compiled by itself, it
+// rounds as it does in the group kernels
+template <int FORM, int QED, bool SPIN>
+__device__ __noinline__ unsigned int sfp_massive_tile_call(const sfp_run_dev* __restrict__ R, const sfp_qed_smem& T,
+                                                           const sfp_mlp::Smem& M, const sfp_segment& S, char** desc,
+                                                           unsigned char* ring, int SB, int PT, long long base,
+                                                           long long left, double t, double dt, unsigned int step) {
+    return sfp_massive_tile<FORM, QED, 2, SPIN, false>(R, T, M, S, desc, ring, SB, PT, base, left, t, dt, step);
+}
+
+template <int FORM, int QED>
+__device__ __forceinline__ void sfp_steps_body(const sfp_run_dev* __restrict__ R, int nsteps, int end) {
+    using namespace sfp;
+    if (nsteps < 0) {  // a test of the barrier's time limit: the last block never arrives
+        if (blockIdx.x == gridDim.x - 1) return;
+        nsteps = -nsteps;
+    }
+    constexpr int OD = QED == SFP_QED_OPTICAL_DEPTH ? 1 : 0;
+    constexpr bool QUEUE = QED == SFP_QED_REJECTION;
+    constexpr int NW = SFP_TILE / 32;
+    extern __shared__ __align__(16) double s_tab[];
+    __shared__ char* s_desc[NW][6 + OD + 3 + 2];
+    __shared__ sfp_pair_queue<FORM == SFP_FORM_FP32> s_q[QUEUE ? NW : 1];
+    __shared__ float s_pb[QUEUE ? SFP_PAIR_BOUND_BINS : 1];
+    __shared__ float s_pbmax[QUEUE ? SFP_PAIR_BOUND_BINS : 1];
+    __shared__ long long s_start[2][SFP_SMALL_SEGS + 1], s_nbuf[SFP_SMALL_SEGS];
+    __shared__ sfp_step_plan s_plan;
+    __shared__ int s_cur, s_stop;
+    sfp_step_state* st = R->st;
+    const double dt = R->dt;
+    const sfp_qed_smem T = sfp_stage_tables<FORM, QED>(R, s_tab);
+    sfp_mlp::Smem& M = *reinterpret_cast<sfp_mlp::Smem*>(reinterpret_cast<unsigned char*>(s_tab) + R->mlp_off);
+    if (OD && R->mlp_params) sfp_mlp::stage(M, R->mlp_params);
+    if (QUEUE)
+        for (int k = threadIdx.x; k < SFP_PAIR_BOUND_BINS; k += blockDim.x) {
+            s_pb[k] = R->pair_bound[k];
+            s_pbmax[k] = R->pair_bound[SFP_PAIR_BOUND_BINS + k];
+        }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char* const ring = reinterpret_cast<unsigned char*>(s_tab) + R->m_ring_off + (size_t)warp * R->small_ring;
+    sfp_end_smem& Q = *reinterpret_cast<sfp_end_smem*>(reinterpret_cast<unsigned char*>(s_tab) + R->small_end_off);
+    const long long gw = (long long)warp * gridDim.x + blockIdx.x, nw = (long long)NW * gridDim.x;
+    unsigned int round = 0;
+    for (int k = 0; k < nsteps; ++k) {
+        // the step's plan, written by block 0 (or by the launch before)
+        if (threadIdx.x == 0) {
+            s_stop = __ldcg(&st->skip) | __ldcg(&st->halted) | __ldcg(&st->error);
+            s_cur = __ldcg(&st->cur);
+        }
+        __syncthreads();
+        if (s_stop) return;
+        const int cur = s_cur;
+        if (threadIdx.x == 0) {
+            const sfp_step_plan& p = st->plan[cur];
+            s_plan.t = __ldcg(&p.t);
+            s_plan.step = __ldcg(&p.step);
+            s_plan.n_mtiles = __ldcg(&p.n_mtiles);
+            s_plan.n_ptiles = __ldcg(&p.n_ptiles);
+            s_plan.mtile = __ldcg(&p.mtile);
+            s_plan.ptile = __ldcg(&p.ptile);
+        }
+        for (int j = threadIdx.x; j < R->mg.n_seg; j += blockDim.x)
+            s_start[0][j] = __ldcg(R->mg.tile_start + cur * (R->mg.n_seg + 1) + j);
+        for (int j = threadIdx.x; j < R->pg.n_seg; j += blockDim.x)
+            s_start[1][j] = __ldcg(R->pg.tile_start + cur * (R->pg.n_seg + 1) + j);
+        for (int j = threadIdx.x; j < R->n_seg; j += blockDim.x) s_nbuf[j] = __ldcg(R->n_buf_step + cur * R->n_seg + j);
+        __syncthreads();
+        sfp_step_view V;
+        V.t = s_plan.t;
+        V.step = s_plan.step;
+        V.lag = (double)(s_plan.step - st->pos_epoch);
+        V.n_mtiles = s_plan.n_mtiles;
+        V.n_ptiles = s_plan.n_ptiles;
+        V.mtile = s_plan.mtile;
+        V.ptile = s_plan.ptile;
+        V.m_start = s_start[0];
+        V.p_start = s_start[1];
+        V.n_buf = s_nbuf;
+        for (long long w = gw; w < V.n_mtiles + V.n_ptiles; w += nw) {
+            const bool massive = w < V.n_mtiles;
+            const sfp_group_dev& G = massive ? R->mg : R->pg;
+            const long long tile = massive ? w : w - V.n_mtiles;
+            const long long* start = massive ? V.m_start : V.p_start;
+            const int pos = sfp_find_group_pos(start, G.n_seg, tile);
+            const int si = G.seg[pos];
+            const sfp_segment& S = R->seg[si];
+            const int PT = massive ? V.mtile : V.ptile;
+            const long long base = (tile - start[pos]) * (long long)PT;
+            const long long left = V.n_buf[si] - base;
+            unsigned int cnt = 0;
+            if (left > 0) {  // else: alignment padding between segments
+                if (!massive)
+                    cnt = sfp_photon_tile<FORM, QED, 3, false>(R, T, s_pb, s_pbmax, S, s_desc[warp], ring,
+                                                               s_q[QUEUE ? warp : 0], PT, base, left, V.t, dt,
+                                                               (unsigned int)V.step, V.lag);
+                else if (S.spin)
+                    cnt = sfp_massive_tile_call<FORM, QED, true>(R, T, M, S, s_desc[warp], ring, R->m_stage_bytes,
+                                                                      PT, base, left, V.t, dt, (unsigned int)V.step);
+                else
+                    cnt = sfp_massive_tile_call<FORM, QED, false>(R, T, M, S, s_desc[warp], ring, R->m_stage_bytes,
+                                                                       PT, base, left, V.t, dt, (unsigned int)V.step);
+            }
+            if (lane == 0) {
+                G.tile_cnt[tile] = cnt;
+                if (cnt) atomicAdd(&G.super_cnt[tile / SFP_SUPER_TILE], cnt);
+            }
+        }
+        if (!sfp_grid_barrier(st, ++round)) return;
+        if (blockIdx.x == 0) sfp_end_scan(R, end, Q);
+        if (!sfp_grid_barrier(st, ++round)) return;
+        if (threadIdx.x == 0) s_stop = __ldcg(&st->halted);
+        __syncthreads();
+        if (s_stop) return;  // no room: the host resumes the step
+        // the children, while block 0 plans the next step
+        if (blockIdx.x == 0)
+            sfp_end_plan(R, end, Q, (int)nw);
+        else
+            sfp_append_units<FORM>(R, V, reinterpret_cast<unsigned short*>(ring), (long long)warp * (gridDim.x - 1) + blockIdx.x - 1,
+                                   (long long)NW * (gridDim.x - 1), dt, false);
+        if (!sfp_grid_barrier(st, ++round)) return;
     }
 }
 
@@ -2138,6 +2440,15 @@ extern "C" __global__ void __launch_bounds__(32) sfp_epoch_kernel(const sfp_run_
 extern "C" __global__ void __launch_bounds__(SFP_TILE, 2) sfp_appends_fp64(const sfp_run_dev* __restrict__ R) {
     sfp_appends_body<SFP_FORM_FP64>(R);
 }
+#if defined(SFP_STEP_QED_RS)
+extern "C" __global__ void __launch_bounds__(SFP_TILE, 2) sfp_steps_fp64_rs(const sfp_run_dev* __restrict__ R, int nsteps, int end) {
+    sfp_steps_body<SFP_FORM_FP64, SFP_QED_REJECTION>(R, nsteps, end);
+}
+#else
+extern "C" __global__ void __launch_bounds__(SFP_TILE, 2) sfp_steps_fp64_od(const sfp_run_dev* __restrict__ R, int nsteps, int end) {
+    sfp_steps_body<SFP_FORM_FP64, SFP_QED_OPTICAL_DEPTH>(R, nsteps, end);
+}
+#endif
 extern "C" __global__ void __launch_bounds__(256) sfp_sync_positions_fp64(const sfp_run_dev* __restrict__ R) {
     sfp_sync_positions_body<SFP_FORM_FP64>(R);
 }
@@ -2168,6 +2479,15 @@ SFP_PHOTON_KERNEL_T(fp64, od, SFP_FORM_FP64, SFP_QED_OPTICAL_DEPTH, 3, 3)
 extern "C" __global__ void __launch_bounds__(SFP_TILE, 3) sfp_appends_fp32(const sfp_run_dev* __restrict__ R) {
     sfp_appends_body<SFP_FORM_FP32>(R);
 }
+#if defined(SFP_STEP_QED_RS)
+extern "C" __global__ void __launch_bounds__(SFP_TILE, 2) sfp_steps_fp32_rs(const sfp_run_dev* __restrict__ R, int nsteps, int end) {
+    sfp_steps_body<SFP_FORM_FP32, SFP_QED_REJECTION>(R, nsteps, end);
+}
+#else
+extern "C" __global__ void __launch_bounds__(SFP_TILE, 2) sfp_steps_fp32_od(const sfp_run_dev* __restrict__ R, int nsteps, int end) {
+    sfp_steps_body<SFP_FORM_FP32, SFP_QED_OPTICAL_DEPTH>(R, nsteps, end);
+}
+#endif
 extern "C" __global__ void __launch_bounds__(256) sfp_sync_positions_fp32(const sfp_run_dev* __restrict__ R) {
     sfp_sync_positions_body<SFP_FORM_FP32>(R);
 }

@@ -26,7 +26,7 @@ from typing import Sequence
 from . import _lib, program
 from .particles import _device, _stream_ptr
 from .simulation import (MIN_ROOM, Simulation, _release_cached_blocks, attach_position_sync, detach_position_sync,
-                         observe_rates, plan_chunk, resolve_pending, sync_positions)
+                         launches_since, observe_rates, plan_chunk, resolve_pending, sync_positions)
 
 
 class Ensemble(object):
@@ -83,11 +83,6 @@ class Ensemble(object):
             base += len(sim.all_particles)
         return segs
 
-    def _launches_per_step(self):
-        ps = self.species
-        return (any(p.m != 0 for p in ps) + any(p.m == 0 for p in ps)
-                + any(p.bw or p.radiating for p in ps))
-
     def _begin(self):
         for p in self.species:
             p._to_gpu()
@@ -116,6 +111,7 @@ class Ensemble(object):
                   ctypes.byref(run))
         self._run = run
         self._keep = (mod, params)
+        self._launched = 0  # the run's launches counted so far
         self._ps_base = self.particle_steps
         attach_position_sync(self, allp)
 
@@ -172,7 +168,7 @@ class Ensemble(object):
             _lib.check(L.sfp_run_steps(self._run, chunk, self.graph_chunk if chunk >= self.graph_chunk else 0,
                                        _stream_ptr()), "sfp_run_steps")
             self._pos_dirty = True
-            self.kernel_launches += self._launches_per_step() * chunk + 1
+            self.kernel_launches += launches_since(self, self._run)
             done = self._sync_state(st, nbuf)
             halted = bool(st.halted)
             if halted:
@@ -204,7 +200,7 @@ class Ensemble(object):
             _lib.check(L.sfp_run_steps_timed(self._run, 1, ms, _stream_ptr()), "sfp_run_steps_timed")
             self._pos_dirty = True
             _lib.check(L.sfp_run_read_state(self._run, ctypes.byref(st), nbuf, _stream_ptr()), "read_state")
-            self.kernel_launches += self._launches_per_step() + 1
+            self.kernel_launches += launches_since(self, self._run)
             if st.error or (st.halted and not st.appends_pending):
                 raise _lib.SFPError("timed step did not complete")
             if st.appends_pending:  # finish the step; its appends kernel was not timed

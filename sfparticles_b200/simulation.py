@@ -158,6 +158,14 @@ def sync_positions(owner, species):
             p._touch()
 
 
+def launches_since(owner, run) -> int:
+    """Kernels the run has launched since the last count."""
+    n = ctypes.c_int64(0)
+    _lib.check(_lib.load().sfp_run_launches(run, ctypes.byref(n)), "sfp_run_launches")
+    new, owner._launched = int(n.value) - owner._launched, int(n.value)
+    return new
+
+
 def observe_rates(species, before, steps, rates):
     """Update the append rates from the counts before and after `steps` steps."""
     if steps <= 0:
@@ -444,6 +452,7 @@ class Simulation(object):
                   ctypes.byref(run))
         self._run = run
         self._keep = (mod, params)
+        self._launched = 0  # the run's launches counted so far
         self._ps_base = self.particle_steps  # the device counter restarts with the run
         attach_position_sync(self, self.all_particles)
 
@@ -504,7 +513,7 @@ class Simulation(object):
             _lib.check(L.sfp_run_steps_timed(self._run, 1, ms, _stream_ptr()), "sfp_run_steps_timed")
             self._pos_dirty = True
             _lib.check(L.sfp_run_read_state(self._run, ctypes.byref(st), nbuf, _stream_ptr()), "read_state")
-            self.kernel_launches += self._launches_per_step() + 1
+            self.kernel_launches += launches_since(self, self._run)
             if st.error or (st.halted and not st.appends_pending):
                 raise _lib.SFPError("timed step did not complete")
             if st.appends_pending:  # finish the step; its appends kernel was not timed
@@ -519,14 +528,6 @@ class Simulation(object):
         self.step = int(st.step)
         self.t = float(st.t)
         return out, before, [p.N_buffered for p in self.all_particles]
-
-    def _launches_per_step(self):
-        """libsfp kernels one step launches: the massive and photon kernels
-        that have species to work on + appends when a species emits photons or
-        creates pairs (a call launches one bookkeeping kernel besides)."""
-        ps = self.all_particles
-        return (any(p.m != 0 for p in ps) + any(p.m == 0 for p in ps)
-                + any(p.bw or p.radiating for p in ps))
 
     def _loop(self, run, nstep, call_back):
         L = _lib.load()
@@ -558,7 +559,7 @@ class Simulation(object):
             _lib.check(L.sfp_run_steps(run, chunk, self.graph_chunk if chunk >= self.graph_chunk else 0,
                                        _stream_ptr()), "sfp_run_steps")
             self._pos_dirty = True
-            self.kernel_launches += self._launches_per_step() * chunk + 1
+            self.kernel_launches += launches_since(self, run)
             done = self._sync_state(run, st, nbuf)
             halted = bool(st.halted)
             if halted:
