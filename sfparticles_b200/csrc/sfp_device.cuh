@@ -4,9 +4,14 @@
 // reference's 12 Numba kernels one for one) and by NVRTC into the
 // field-specialised fused step modules.  Nothing here allocates or launches.
 //
-// Each routine restates a reference routine (cited) in float64 with the same
-// operation order; nvcc/NVRTC may contract a*b+c into one FMA, which moves
-// results by <= 1 ulp per operation relative to the reference.
+// Each routine restates a reference routine (cited) in float64; nvcc/NVRTC
+// may contract a*b+c into one FMA, which moves results by <= 1 ulp per
+// operation relative to the reference.  Where the reference divides several
+// times by one quantity, takes a square root and divides by it, or raises to
+// the power 2/3, the same value is formed with one reciprocal, rsqrt or cbrt
+// (each within 1 ulp): on the GPU a float64 division is some twenty
+// instructions and pow two hundred, and they were most of what the float64
+// step executes.
 #pragma once
 #include "sfp_types.h"
 
@@ -158,27 +163,23 @@ SFP_DEVICE_INLINE void field_simple(const double* __restrict__ P, double x, doub
 
 // gaussian_laser_pulse, fields.py:152-168.
 // P = E0, k0, zR, w0, ctau, direction, x0, cep, cos(pol), sin(pol)
-SFP_DEVICE_INLINE void field_gaussian(const double* __restrict__ P, double x, double y, double z, double t,
-                                      double F[6]) {
-    const double E0 = P[0], k0 = P[1], zR = P[2], w0 = P[3], ctau = P[4], dir = P[5], x0 = P[6];
+
+#if defined(SFP_FIELD_TAIL)
+// Its value where |k0 xr| > kGaussTail kc, in the reference's own operations
+// (the per-op field kernel, whose values stand by themselves): there the
+// envelope exp(-(phi/kc)^2) is below exp(-49) in most of space and its relative
+// rounding error is that of its argument, up to 745 times 2^-53 per operation.
+// A step adds such a field to momenta that lose it whole.
+constexpr double kGaussTail = 8.0;
+SFP_DEVICE_INLINE void field_gaussian_tail(const double* __restrict__ P, double kx, double x, double r2, double F[6]) {
+    const double E0 = P[0], k0 = P[1], zR = P[2], w0 = P[3], ctau = P[4], dir = P[5];
     const double cep = P[7], cp = P[8], sp = P[9];
-    const double r2 = y * y + z * z;
-    // Far outside the pulse the envelope exp(-(phi/kc)^2) is exactly 0 in
-    // float64 ((phi/kc)^2 > 745.2).  |phi| >= |k0 xr| - k0 r2 / (4 zR) - pi/2,
-    // because |x| / (x^2 + zR^2) <= 1 / (2 zR) and |atan| < pi/2; once that
-    // bound exceeds sqrt(800) kc the field is 0 without evaluating atan, cos
-    // and the divisions (the formula gives +-0 there).  Multiplied by 4 zR > 0.
-    if (4.0 * zR * fabs(k0 * ((x - x0) - (dir * kC) * t)) - k0 * r2 - 6.2832 * zR >
-        4.0 * zR * kFieldCut64 * (k0 * ctau)) {
-        for (int k = 0; k < 6; ++k) F[k] = 0.0;
-        return;
-    }
     const double xz = x / zR;
     const double wx = w0 * sqrt(1.0 + xz * xz);
     const double zx = zR / x;
     const double Rx = x * (1.0 + zx * zx);
-    const double gouy = atan(x / zR);
-    const double phi = ((k0 * ((x - x0) - (dir * kC) * t)) + (((k0 * r2) / 2.0) / Rx)) - gouy;
+    const double gouy = atan(xz);
+    const double phi = __dadd_rn(kx, ((k0 * r2) / 2.0) / Rx) - gouy;
     const double kc = k0 * ctau;
     const double E = ((((E0 * cos(phi + cep)) * w0) / wx) * exp((-r2) / (wx * wx))) * exp((-(phi * phi)) / (kc * kc));
     const double Ey = E * cp, Ez = E * sp;
@@ -189,6 +190,53 @@ SFP_DEVICE_INLINE void field_gaussian(const double* __restrict__ P, double x, do
     F[4] = ((-Ez) / kC) * dir;
     F[5] = (Ey / kC) * dir;
 }
+#endif
+
+SFP_DEVICE_INLINE void field_gaussian(const double* __restrict__ P, double x, double y, double z, double t,
+                                      double F[6]) {
+    const double E0 = P[0], k0 = P[1], zR = P[2], w0 = P[3], ctau = P[4], dir = P[5], x0 = P[6];
+    const double cep = P[7], cp = P[8], sp = P[9];
+    const double r2 = y * y + z * z;
+    const double kx = __dmul_rn(k0, (x - x0) - (dir * kC) * t), kc = k0 * ctau;
+    // Far outside the pulse the envelope exp(-(phi/kc)^2) is exactly 0 in
+    // float64 ((phi/kc)^2 > 745.2).  |phi| >= |k0 xr| - k0 r2 / (4 zR) - pi/2,
+    // because |x| / (x^2 + zR^2) <= 1 / (2 zR) and |atan| < pi/2; once that
+    // bound exceeds sqrt(800) kc the field is 0 without evaluating atan, cos
+    // and the divisions (the formula gives +-0 there).  Multiplied by 4 zR > 0.
+    if (4.0 * zR * fabs(kx) - k0 * r2 - 6.2832 * zR > 4.0 * zR * kFieldCut64 * kc) {
+        for (int k = 0; k < 6; ++k) F[k] = 0.0;
+        return;
+    }
+#if defined(SFP_FIELD_TAIL)
+    if (fabs(kx) > kGaussTail * kc) {
+        field_gaussian_tail(P, kx, x, r2, F);
+        return;
+    }
+#endif
+    // with q = 1 + (x/zR)^2: w0/w = 1/sqrt(q), r^2/w^2 = (r/w0)^2/q and
+    // k0 r^2 / (2 x (1 + (zR/x)^2)) = k0/(2 zR^2) r^2 x / q, which the
+    // reference's form leaves undefined at x = 0.  The reciprocals of the
+    // parameters are the same for every particle (formed once per loop).
+    // 5e5 e- and 1.2e7 photons, rejection sampling: massive kernel 78 -> 51 us,
+    // hot photons 172 -> 113 us (with rsqrt, cbrt and one reciprocal in the push
+    // and the rates).
+    const double izR = 1.0 / zR, iw0 = 1.0 / w0, ikc = 1.0 / kc;
+    const double xz = x * izR;
+    const double rs = rsqrt(1.0 + xz * xz);
+    const double rq = rs * rs;
+    const double gouy = atan(xz);
+    const double curv = x == 0.0 ? __longlong_as_double(0x7ff8000000000000ll) : ((0.5 * k0 * izR) * r2) * (xz * rq);
+    const double phi = (kx + curv) - gouy;
+    const double rw = (iw0 * iw0) * r2, pk = phi * ikc;
+    const double E = ((E0 * cos(phi + cep)) * rs) * exp(-(rw * rq + pk * pk));
+    const double Ey = E * cp, Ez = E * sp;
+    F[0] = 0.0;
+    F[1] = Ey;
+    F[2] = Ez;
+    F[3] = 0.0;
+    F[4] = -Ez * (dir / kC);
+    F[5] = Ey * (dir / kC);
+}
 
 // focused_gaussian_laser_pulse, fields.py:211-263 (Salamin-type expansion
 // to eps^5).  P = E0, k0, zR, w0, ctau, direction, xfoc, x0, cep, cos(pol), sin(pol), eps
@@ -198,53 +246,54 @@ SFP_DEVICE_INLINE void field_focused(const double* __restrict__ P, double x, dou
     const double xfoc = P[6], x0 = P[7], cep = P[8], cp = P[9], sp = P[10], ep = P[11];
     x = dir * (x - xfoc);
     const double r2 = y * y + z * z;
-    const double xz = x / zR;
-    const double wx = w0 * sqrt(1.0 + xz * xz);
-    const double psiG = atan(x / zR);
-    const double psiR = (((k0 * x) * r2) / 2.0) / ((x * x) + (zR * zR));
+    // the parameters' reciprocals are the same for every particle
+    const double izR = 1.0 / zR, iw0 = 1.0 / w0, ikc = 1.0 / (k0 * ctau);
+    const double xz = x * izR;
+    const double eta = rsqrt(1.0 + xz * xz), eta2 = eta * eta;
+    const double psiG = atan(xz);
+    const double psiR = ((0.5 * k0 * izR) * r2) * (xz * eta2);  // k0 x r^2 / (2 (x^2 + zR^2))
     const double psiP = k0 * ((x - dir * x0) - kC * t);
-    const double psi = ((psiG + psiR) + psiP) + cep;
-    const double rho = sqrt(r2) / w0;
-    const double xi = y / w0;
-    const double nu = z / w0;
-    const double eta = 1.0 / sqrt(1.0 + xz * xz);
-    const double rho2 = ipow<2>(rho), rho4 = ipow<4>(rho), rho6 = ipow<6>(rho), rho8 = ipow<8>(rho);
-    const double kc = k0 * ctau;
-    const double pc = psi - cep;
-    const double E = (((E0 * w0) / wx) * exp((-r2) / (wx * wx))) * exp((-(pc * pc)) / (kc * kc));
-    const double S0 = sin(psi);
-    const double S2 = ipow<2>(eta) * sin(psi + 2.0 * psiG);
-    const double S3 = ipow<3>(eta) * sin(psi + 3.0 * psiG);
-    const double S4 = ipow<4>(eta) * sin(psi + 4.0 * psiG);
-    const double S5 = ipow<5>(eta) * sin(psi + 5.0 * psiG);
-    const double S6 = ipow<6>(eta) * sin(psi + 6.0 * psiG);
-    const double C1 = ipow<1>(eta) * cos(psi + 1.0 * psiG);
-    const double C2 = ipow<2>(eta) * cos(psi + 2.0 * psiG);
-    const double C3 = ipow<3>(eta) * cos(psi + 3.0 * psiG);
-    const double C4 = ipow<4>(eta) * cos(psi + 4.0 * psiG);
-    const double C5 = ipow<5>(eta) * cos(psi + 5.0 * psiG);
-    const double C6 = ipow<6>(eta) * cos(psi + 6.0 * psiG);
-    const double C7 = ipow<7>(eta) * cos(psi + 7.0 * psiG);
+    const double pc = (psiG + psiR) + psiP;
+    const double psi = pc + cep;
+    const double xi = y * iw0;
+    const double nu = z * iw0;
+    const double rho2 = r2 * (iw0 * iw0), rho4 = rho2 * rho2, rho6 = rho4 * rho2, rho8 = rho4 * rho4;
+    const double pk = pc * ikc;
+    const double E = (E0 * eta) * exp(-(rho2 * eta2 + pk * pk));
+    // C_n + i S_n = eta^n exp(i (psi + n psiG)): with cos psiG = eta and
+    // sin psiG = eta x/zR, each is the one before times eta^2 (1 + i x/zR),
+    // so one sincos serves all thirteen (1e6 e- with spin and the
+    // Landau-Lifshitz force: 119 -> 68 us a step)
+    double S0, C0;
+    sincos(psi, &S0, &C0);
+    const double a = eta2, b = eta2 * xz;
+    const double C1 = a * C0 - b * S0, S1 = a * S0 + b * C0;
+    const double C2 = a * C1 - b * S1, S2 = a * S1 + b * C1;
+    const double C3 = a * C2 - b * S2, S3 = a * S2 + b * C2;
+    const double C4 = a * C3 - b * S3, S4 = a * S3 + b * C3;
+    const double C5 = a * C4 - b * S4, S5 = a * S4 + b * C4;
+    const double C6 = a * C5 - b * S5, S6 = a * S5 + b * C5;
+    const double C7 = a * C6 - b * S6;
     const double e2 = ipow<2>(ep), e3 = ipow<3>(ep), e4 = ipow<4>(ep), e5 = ipow<5>(ep);
     const double xi2 = ipow<2>(xi);
-    const double exA = (((-C2) / 2.0) + rho2 * C3) - (rho4 * C4) / 4.0;
+    const double exA = (((-C2) * 0.5) + rho2 * C3) - (rho4 * C4) * 0.25;
     const double exB =
-        ((((-0.375 * C3) - (0.375 * rho2) * C4) + (1.0625 * rho4) * C5) - (0.375 * rho6) * C6) + (rho8 * C7) / 32.0;
+        ((((-0.375 * C3) - (0.375 * rho2) * C4) + (1.0625 * rho4) * C5) - (0.375 * rho6) * C6) + (rho8 * C7) * 0.03125;
     const double Ex_ = (E * xi) * (((ep * C1) + e3 * exA) + e5 * exB);
-    const double eyA = (xi2 * S2) - (rho4 * S3) / 4.0;
-    const double eyB = ((((S2 / 8.0) - (rho2 * S3) / 4.0) - ((rho2 * (rho2 - 16.0 * xi2)) * S4) / 16.0) -
-                        ((rho4 * (rho2 + 2.0 * xi2)) * S5) / 8.0) +
-                       (rho8 * S6) / 32.0;
+    const double eyA = (xi2 * S2) - (rho4 * S3) * 0.25;
+    const double eyB = ((((S2 * 0.125) - (rho2 * S3) * 0.25) - ((rho2 * (rho2 - 16.0 * xi2)) * S4) * 0.0625) -
+                        ((rho4 * (rho2 + 2.0 * xi2)) * S5) * 0.125) +
+                       (rho8 * S6) * 0.03125;
     const double Ey_ = E * ((S0 + e2 * eyA) + e4 * eyB);
-    const double Ez_ = ((E * xi) * nu) * ((e2 * S2) + e4 * ((rho2 * S4) - (rho4 * S5) / 4.0));
-    const double bxA = ((C2 / 2.0) + (rho2 * C3) / 2.0) - (rho4 * C4) / 4.0;
+    const double Ez_ = ((E * xi) * nu) * ((e2 * S2) + e4 * ((rho2 * S4) - (rho4 * S5) * 0.25));
+    const double bxA = ((C2 * 0.5) + (rho2 * C3) * 0.5) - (rho4 * C4) * 0.25;
     const double bxB =
-        ((((0.375 * C3) + (0.375 * rho2) * C4) + (0.1875 * rho4) * C5) - (rho6 * C6) / 4.0) + (rho8 * C7) / 32.0;
-    const double Bx_ = ((E / kC) * nu) * (((ep * C1) + e3 * bxA) + e5 * bxB);
-    const double bzA = ((rho2 * S2) / 2.0) - (rho4 * S3) / 4.0;
+        ((((0.375 * C3) + (0.375 * rho2) * C4) + (0.1875 * rho4) * C5) - (rho6 * C6) * 0.25) + (rho8 * C7) * 0.03125;
+    const double Bx_ = ((E * (1.0 / kC)) * nu) * (((ep * C1) + e3 * bxA) + e5 * bxB);
+    const double bzA = ((rho2 * S2) * 0.5) - (rho4 * S3) * 0.25;
     const double bzB =
-        (((((-S2) / 8.0) + (rho2 * S3) / 4.0) + (0.3125 * rho4) * S4) - (rho6 * S5) / 4.0) + (rho8 * S6) / 32.0;
-    const double Bz_ = (E / kC) * ((S0 + e2 * bzA) + e4 * bzB);
+        (((((-S2) * 0.125) + (rho2 * S3) * 0.25) + (0.3125 * rho4) * S4) - (rho6 * S5) * 0.25) + (rho8 * S6) * 0.03125;
+    const double Bz_ = (E * (1.0 / kC)) * ((S0 + e2 * bzA) + e4 * bzB);
     const double By_ = 0.0;
     F[0] = Ex_;
     F[1] = Ey_ * cp - Ez_ * sp;
@@ -261,10 +310,10 @@ SFP_DEVICE_INLINE void field_focused(const double* __restrict__ P, double x, dou
 // 1/gamma of a massive particle / 1/|u| of a photon, as the reference stores
 // it (particles.py:119,122; cpu.py:86,114,187)
 SFP_DEVICE_INLINE double inv_gamma_massive(double ux, double uy, double uz) {
-    return 1.0 / sqrt(((1.0 + ux * ux) + uy * uy) + uz * uz);
+    return rsqrt(((1.0 + ux * ux) + uy * uy) + uz * uz);
 }
 SFP_DEVICE_INLINE double inv_gamma_photon(double ux, double uy, double uz) {
-    return 1.0 / sqrt((ux * ux + uy * uy) + uz * uz);
+    return rsqrt((ux * ux + uy * uy) + uz * uz);
 }
 
 // cpu.py:5-19, one particle
@@ -283,7 +332,7 @@ SFP_DEVICE_INLINE double boris(double& ux, double& uy, double& uz, const double 
     const double uxm = ux + efactor * F[0];
     const double uym = uy + efactor * F[1];
     const double uzm = uz + efactor * F[2];
-    const double igm = 1.0 / sqrt(((1.0 + uxm * uxm) + uym * uym) + uzm * uzm);
+    const double igm = rsqrt(((1.0 + uxm * uxm) + uym * uym) + uzm * uzm);
     const double Tx = (bfactor * F[3]) * igm;
     const double Ty = (bfactor * F[4]) * igm;
     const double Tz = (bfactor * F[5]) * igm;
@@ -311,19 +360,22 @@ SFP_DEVICE_INLINE double boris_tbmt(double& ux, double& uy, double& uz, double& 
     const double uym = uy + efactor * Ey;
     const double uzm = uz + efactor * Ez;
     const double uB = (uxm * Bx + uym * By) + uzm * Bz;
-    const double gm = sqrt(((1.0 + uxm * uxm) + uym * uym) + uzm * uzm);
-    const double igm = 1.0 / gm;
+    const double g2m = ((1.0 + uxm * uxm) + uym * uym) + uzm * uzm;
+    const double igm = rsqrt(g2m);
+    const double gm = g2m * igm;
+    const double ig1 = 1.0 / (gm + 1.0);
     const double a1 = ae + igm;
-    const double a2 = (ae * gm) / (gm + 1.0);
-    const double a3 = ae + 1.0 / (gm + 1.0);
+    const double a2 = (ae * gm) * ig1;
+    const double a3 = ae + ig1;
     const double Bxe = (a1 * Bx - (a2 * uB) * uxm) - a3 * (uym * Ez - uzm * Ey);
     const double Bye = (a1 * By - (a2 * uB) * uym) - a3 * (uzm * Ex - uxm * Ez);
     const double Bze = (a1 * Bz - (a2 * uB) * uzm) - a3 * (uxm * Ey - uym * Ex);
     double Tx = bfactor * Bxe, Ty = bfactor * Bye, Tz = bfactor * Bze;
     const double T2 = (Tx * Tx + Ty * Ty) + Tz * Tz;
-    double Sx = (2.0 * Tx) / (1.0 + T2);
-    double Sy = (2.0 * Ty) / (1.0 + T2);
-    double Sz = (2.0 * Tz) / (1.0 + T2);
+    const double Tf1 = 2.0 / (1.0 + T2);
+    double Sx = Tf1 * Tx;
+    double Sy = Tf1 * Ty;
+    double Sz = Tf1 * Tz;
     const double s0x = sx, s0y = sy, s0z = sz;
     const double sxp = (s0x + s0y * Tz) - s0z * Ty;
     const double syp = (s0y + s0z * Tx) - s0x * Tz;
@@ -359,8 +411,8 @@ SFP_DEVICE_INLINE double ll_factor(double dt) {
 SFP_DEVICE_INLINE double ll_push(double& ux, double& uy, double& uz, double ig, double chi, double dt, bool quantum) {
     double factor = ll_factor(dt);
     if (quantum) {
-        const double g = pow((1.0 + (4.8 * (1.0 + chi)) * log(1.0 + 1.7 * chi)) + 2.44 * (chi * chi), -2.0 / 3.0);
-        factor = factor * g;
+        const double g = rcbrt((1.0 + (4.8 * (1.0 + chi)) * log(1.0 + 1.7 * chi)) + 2.44 * (chi * chi));
+        factor = factor * (g * g);
     }
     const double c2 = chi * chi;
     ux = ux + ((factor * c2) * ux) * ig;
@@ -388,27 +440,30 @@ SFP_DEVICE_INLINE double chi_of(const double F[6], double ux, double uy, double 
 // ---------------------------------------------------------------------------
 SFP_DEVICE_INLINE void ai_interp(double z, const double* __restrict__ iAt, const double* __restrict__ dAt, int zN,
                                  double zmax, double& iA, double& dA) {
-    const double dz = (zmax - 0.0) / (double)(zN - 1);
-    long long idx = (long long)((z - 0.0) / dz);
+    const double inv_dz = (double)(zN - 1) / zmax;  // the same for every particle
+    const double f = z * inv_dz;
+    int idx = (int)f;
     if (idx > zN - 2) idx = zN - 2;
-    const double zl = 0.0 + (double)idx * dz;
-    double k = (iAt[idx + 1] - iAt[idx]) / dz;
-    iA = iAt[idx] + k * (z - zl);
-    k = (dAt[idx + 1] - dAt[idx]) / dz;
-    dA = dAt[idx] + k * (z - zl);
+    const double w = f - (double)idx;
+    const double i0 = iAt[idx], d0 = dAt[idx];
+    iA = i0 + (iAt[idx + 1] - i0) * w;
+    dA = d0 + (dAt[idx + 1] - d0) * w;
 }
 
-// qed/rejection_sampling_tables.py:32-53; z beyond the table -> 0
+// The differential rates take z = b^(2/3) and sqrt(z) = b^(1/3), both from one
+// cube root; z beyond the table -> 0.
+// qed/rejection_sampling_tables.py:32-53
 SFP_DEVICE_INLINE double photon_rate(double chi_e, double delta, const double* iAt, const double* dAt, int zN,
                                      double zmax) {
     const double chi_gamma = delta * chi_e;
     const double chi_ep = chi_e - chi_gamma;
-    const double z = pow((chi_gamma / chi_e) / chi_ep, 2.0 / 3.0);
+    const double rz = cbrt(chi_gamma / (chi_e * chi_ep));
+    const double z = rz * rz;
     const double factor = (((-kAlpha) * kMe) * (kC * kC)) / kHbar;
     if (!(z <= zmax)) return 0.0;
     double iA, dA;
     ai_interp(z, iAt, dAt, zN, zmax, iA, dA);
-    return factor * (iA + (2.0 / z + chi_gamma * sqrt(z)) * dA);
+    return factor * (iA + (2.0 / z + chi_gamma * rz) * dA);
 }
 
 // qed/rejection_sampling_tables.py:56-78
@@ -416,12 +471,13 @@ SFP_DEVICE_INLINE double pair_rate(double chi_gamma, double delta, const double*
                                    double zmax) {
     const double chi_e = delta * chi_gamma;
     const double chi_ep = chi_gamma - chi_e;
-    const double z = pow((chi_gamma / chi_e) / chi_ep, 2.0 / 3.0);
+    const double rz = cbrt(chi_gamma / (chi_e * chi_ep));
+    const double z = rz * rz;
     const double factor = ((kAlpha * kMe) * (kC * kC)) / kHbar;
     if (!(z <= zmax)) return 0.0;
     double iA, dA;
     ai_interp(z, iAt, dAt, zN, zmax, iA, dA);
-    return factor * (iA + (2.0 / z - chi_gamma * sqrt(z)) * dA);
+    return factor * (iA + (2.0 / z - chi_gamma * rz) * dA);
 }
 
 // qed/rejection_sampling.py:73-89 with draws (r1, r2): returns event, sets delta
@@ -456,7 +512,7 @@ SFP_DEVICE_INLINE bool pair_event_rs(double chi, double ig, double dt, double r1
 // ---------------------------------------------------------------------------
 SFP_DEVICE_INLINE double od_row(double log_chi, const sfp_od_table& t) {
     if (log_chi > t.log_chi_max) log_chi = t.log_chi_max;
-    double idx = (log_chi - t.log_chi_min) / t.log_chi_delta;
+    double idx = (log_chi - t.log_chi_min) * (1.0 / t.log_chi_delta);
     if (idx > (double)(t.chi_N - 1)) idx = (double)(t.chi_N - 1);
     return idx;
 }
@@ -469,8 +525,7 @@ SFP_DEVICE_INLINE double od_interp1d(double chi, const sfp_od_table& t, const do
     if (idx > t.chi_N - 2) idx = t.chi_N - 2;
     if (log_chi > t.log_chi_max) log_chi = t.log_chi_max;
     const double left = t.log_chi_min + (double)idx * t.log_chi_delta;
-    const double k = (rate[idx + 1] - rate[idx]) / t.log_chi_delta;
-    return rate[idx] + k * (log_chi - left);
+    return rate[idx] + (rate[idx + 1] - rate[idx]) * ((log_chi - left) * (1.0 / t.log_chi_delta));
 }
 
 // _bisect_interp, qed/optical_depth_tables.py:69-112 (rows blended linearly in
@@ -483,15 +538,14 @@ SFP_DEVICE_INLINE double od_bisect(double chi, double r_uniform, const sfp_od_ta
     if (lo_i > t.chi_N - 2) lo_i = t.chi_N - 2;
     if (lo_i < 0) lo_i = 0;
     const long long hi_i = lo_i + 1;
-    const double chi_top = pow(10.0, t.log_chi_max);
+    const double chi_top = exp10(t.log_chi_max);
     if (chi > chi_top) chi = chi_top;
-    const double chi_low = pow(10.0, t.log_chi_min + (double)lo_i * t.log_chi_delta);
-    const double chi_high = pow(10.0, t.log_chi_min + (double)hi_i * t.log_chi_delta);
+    const double chi_low = exp10(t.log_chi_min + (double)lo_i * t.log_chi_delta);
+    const double chi_high = exp10(t.log_chi_min + (double)hi_i * t.log_chi_delta);
     const double* __restrict__ TL = t.cumulative + (size_t)lo_i * n;
     const double* __restrict__ TH = t.cumulative + (size_t)hi_i * n;
-    const double w = chi - chi_low;
-    const double span = chi_high - chi_low;
-#define SFP_ROWVAL(j) (__ldg(TL + (j)) + ((__ldg(TH + (j)) - __ldg(TL + (j))) / span) * w)
+    const double ws = (chi - chi_low) / (chi_high - chi_low);
+#define SFP_ROWVAL(j) (__ldg(TL + (j)) + (__ldg(TH + (j)) - __ldg(TL + (j))) * ws)
     const double ymin = SFP_ROWVAL(0);
     const double ymax = SFP_ROWVAL(n - 1);
     const double r = r_uniform * (ymax - ymin) + ymin;
@@ -510,8 +564,8 @@ SFP_DEVICE_INLINE double od_bisect(double chi, double r_uniform, const sfp_od_ta
     const double y1 = SFP_ROWVAL(di);
     const double y2 = SFP_ROWVAL(di + 1);
 #undef SFP_ROWVAL
-    const double dl = pow(10.0, t.log_delta_min + (double)di * t.log_delta_delta);
-    const double dr = pow(10.0, t.log_delta_min + (double)(di + 1) * t.log_delta_delta);
+    const double dl = exp10(t.log_delta_min + (double)di * t.log_delta_delta);
+    const double dr = exp10(t.log_delta_min + (double)(di + 1) * t.log_delta_delta);
     const double k = (dr - dl) / (y2 - y1);
     return dl + k * (r - y1);
 }

@@ -1149,10 +1149,13 @@ __device__ __forceinline__ void sfp_ring_issue_full(char* const* D, int sub, uns
 // ---------------------------------------------------------------------------
 template <int FORM, int QED, int STAGES, bool SPIN, bool LONG>
 __device__ __forceinline__ unsigned int sfp_massive_tile(const sfp_run_dev* __restrict__ R, const sfp_qed_smem& T,
-                                                         const sfp_mlp::Smem& M, const sfp_segment& S, char** desc,
+                                                         const sfp_mlp::Smem& M, const sfp_segment& S_in, char** desc,
                                                          unsigned char* ring, int SB, int PT, long long base,
                                                          long long left, double t, double dt, unsigned int step) {
     using namespace sfp;
+    // a copy: what depends on the segment alone (the float64 push's factors, two
+    // divisions) is formed once per tile, as no store can change it
+    const sfp_segment S = S_in;
     constexpr int OD = QED == SFP_QED_OPTICAL_DEPTH ? 1 : 0;
     constexpr int NC = 6 + OD + (SPIN ? 3 : 0);
     const int lane = threadIdx.x & 31;

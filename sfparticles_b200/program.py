@@ -55,7 +55,8 @@ def module_source(field_src: str, form, qed, n_const=None) -> str:
     seen = set()
     head = _inline('#include "sfp_types.h"\n#include "sfp_device.cuh"\n#include "sfp_device32.cuh"\n', seen)
     parts = [head, "// ---- field program ----\n", field_src]
-    if form is None:
+    if form is None:  # the field kernel alone: the reference's operations in a pulse's far tail too
+        parts.insert(0, "#define SFP_FIELD_TAIL 1\n")
         parts.append("#define SFP_WANT_FIELD_EVAL 1\n")
     else:
         parts.append(f"#define SFP_WANT_STEP 1\n#define SFP_STEP_FORM_{form.upper()} 1\n#define SFP_STEP_QED_{qed.upper()} 1\n")
