@@ -102,230 +102,288 @@ __global__ void k_mlp_samples(sfp_od_table t, unsigned long long seed, unsigned 
 }
 
 // ---------------------------------------------------------------- training
-// One block of 256 threads per SM; 64-sample tiles.  Thread (ty, tx) =
-// (tid / 16, tid % 16) owns samples ty + 16 a and units tx + 16 b
-// (a, b = 0..3) of every 64 x 64 tile product, and the weight-gradient
-// entries (j = tx + 16 b, i = ty + 16 a) of W1 and W2.
-constexpr int TS = 64;   // samples per tile
-constexpr int LD = H + 1;  // padded row stride of the smem matrices
+// One block per SM of three pipelines of 128 threads, each with its own
+// 32-sample tiles (the pipelines share the weights and meet at no barrier, so
+// one computes while another waits; a single pipeline of 256 threads and
+// 64-sample tiles left each scheduler two warps that waited for shared
+// memory half of the time).  Every product of 32 x 64 tiles gives thread
+// (ty, tx) = (tid / 16, tid % 16) a 4 x 4 piece: samples ty + 8 a with units
+// 4 tx + q (forward, and backward through a layer); the weight gradients,
+// 64 x 64, give it j = 4 tx + q, i = 8 ty + a.  All operands are read four
+// floats at a time (rows of 68 floats, so that the 16 columns a warp reads
+// fall on different banks): per step of the inner sum a warp takes 3
+// shared-memory wavefronts for its 16 multiply-adds; with single floats it
+// took 8.  Multiply-adds are packed in pairs.  65536 samples, the call with
+// its zeroing and the loss read back: 220 -> 151 us.
+constexpr int TS = 32;     // samples per tile
+constexpr int PIPES = 3;
+constexpr int PT = 128;    // threads of a pipeline
+constexpr int LD = H + 4;  // padded row stride of the smem matrices, 16-byte aligned rows
 
-struct TrainSmem {
-    float W1[H][LD], W2[H][LD];   // BF16-rounded forward weights
+// one pipeline's tile
+struct TrainTile {
     float A1[TS][LD], A2[TS][LD], A3[TS][LD];
     float D1[TS][LD], D2[TS][LD], D3[TS][LD];  // silu'(z), then dL/dz in place
-    float W0[H][2], b0[H], b1[H], b2[H], W3[H];
-    float x[TS][2], y[TS], dy[TS];
-    float gW0[H][2], gb0[H], gb1[H], gb2[H], gW3[H];
-    float gb3, b3;
-    double loss;
+    float x[TS][2], dy[TS];
 };
 
-// out[s][j] = sum_i W[j][i] in[s][i] + b[j]  ->  A = silu, D = silu'
-__device__ __forceinline__ void dense_fwd(const float (*W)[LD], const float* b, const float (*in)[LD],
+struct TrainSmem {
+    float W1[H][LD], W2[H][LD];   // BF16-rounded forward weights, W[unit][input]
+    float V1[H][LD], V2[H][LD];   // their transposes, V[input][unit]
+    float W0[H][2], b0[H], b1[H], b2[H], W3[H];
+    float b3, pad[3];
+    TrainTile tile[PIPES];
+};
+
+__device__ __forceinline__ void pipe_sync(int pipe) {
+    asm volatile("barrier.sync %0, %1;" ::"r"(1 + pipe), "n"(PT) : "memory");
+}
+__device__ __forceinline__ float4 f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float at4(const float4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
+
+// c0 += a0 x, c1 += a1 x as one packed multiply-add (each rounded as fmaf)
+__device__ __forceinline__ void fma2(float& c0, float& c1, float a0, float a1, float x) {
+    asm("{\n\t.reg .b64 c, a, b;\n\tmov.b64 c, {%0, %1};\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\t"
+        "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "+f"(c0), "+f"(c1)
+        : "f"(a0), "f"(a1), "f"(x));
+}
+
+// acc[a][q] += sum_k V[k][4 tx + q] in[ty + 8 a][k], in the order of k
+__device__ __forceinline__ void tile_product(const float (*V)[LD], const float (*in)[LD], float (&acc)[4][4], int ty,
+                                             int tx) {
+#pragma unroll
+    for (int k = 0; k < H; k += 4) {
+        float4 x[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) x[a] = f4(&in[ty + 8 * a][k]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float4 w = f4(&V[k + r][4 * tx]);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const float xa = at4(x[a], r);
+                fma2(acc[a][0], acc[a][1], w.x, w.y, xa);
+                fma2(acc[a][2], acc[a][3], w.z, w.w, xa);
+            }
+        }
+    }
+}
+
+// out[s][j] = sum_i W[j][i] in[s][i] + b[j]  ->  A = silu, D = silu'  (V: W's transpose)
+__device__ __forceinline__ void dense_fwd(const float (*V)[LD], const float* b, const float (*in)[LD],
                                           float (*A)[LD], float (*D)[LD], int ty, int tx) {
     float acc[4][4];
+    const float4 bias = f4(b + 4 * tx);
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[a][q] = b[tx + 16 * q];
-#pragma unroll 4
-    for (int i = 0; i < H; ++i) {
-        float xi[4], wi[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) xi[a] = in[ty + 16 * a][i];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) wi[q] = W[tx + 16 * q][i];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[a][q] = fmaf(wi[q], xi[a], acc[a][q]);
+    for (int a = 0; a < 4; ++a) {
+        acc[a][0] = bias.x;
+        acc[a][1] = bias.y;
+        acc[a][2] = bias.z;
+        acc[a][3] = bias.w;
     }
+    tile_product(V, in, acc, ty, tx);
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) silu_train(acc[a][q], A[ty + 16 * a][tx + 16 * q], D[ty + 16 * a][tx + 16 * q]);
+    for (int a = 0; a < 4; ++a) {
+        float4 act, der;
+        silu_train(acc[a][0], act.x, der.x);
+        silu_train(acc[a][1], act.y, der.y);
+        silu_train(acc[a][2], act.z, der.z);
+        silu_train(acc[a][3], act.w, der.w);
+        *reinterpret_cast<float4*>(&A[ty + 8 * a][4 * tx]) = act;
+        *reinterpret_cast<float4*>(&D[ty + 8 * a][4 * tx]) = der;
+    }
 }
 
 // backward through a 64 -> 64 layer: dZ (in Dout, per sample and output unit),
-// input activations Ain; accumulates gW (registers) and gb (smem); writes
-// dL/dz of the layer below into Din (Din *= W^T dZ).
+// input activations Ain; accumulates gW (registers) and gb (registers of the
+// threads of the first 64); writes dL/dz of the layer below into Din
+// (Din *= W^T dZ).
 __device__ __forceinline__ void dense_bwd(const float (*W)[LD], const float (*Dout)[LD], const float (*Ain)[LD],
-                                          float (*Din)[LD], float (&gW)[4][4], float* gb, int ty, int tx, int tid,
-                                          bool below) {
-    // weight gradient: gW[j][i] += sum_s dZ[s][j] Ain[s][i]   (j = tx + 16 q, i = ty + 16 a)
-#pragma unroll 4
+                                          float (*Din)[LD], float (&gW)[4][8], float (&gb)[4], int ty, int tx) {
+    // weight gradient: gW[j][i] += sum_s dZ[s][j] Ain[s][i]   (j = 4 tx + q, i = 8 ty + a);
+    // bias gradient: the threads of ty = 0 add their units' dZ
+#pragma unroll 8
     for (int s = 0; s < TS; ++s) {
-        float dz[4], ai[4];
+        const float4 dz = f4(&Dout[s][4 * tx]), ai = f4(&Ain[s][8 * ty]), aj = f4(&Ain[s][8 * ty + 4]);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) dz[q] = Dout[s][tx + 16 * q];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) ai[a] = Ain[s][ty + 16 * a];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int a = 0; a < 4; ++a) gW[q][a] = fmaf(dz[q], ai[a], gW[q][a]);
+        for (int q = 0; q < 4; ++q) {
+            fma2(gW[q][0], gW[q][1], ai.x, ai.y, at4(dz, q));
+            fma2(gW[q][2], gW[q][3], ai.z, ai.w, at4(dz, q));
+            fma2(gW[q][4], gW[q][5], aj.x, aj.y, at4(dz, q));
+            fma2(gW[q][6], gW[q][7], aj.z, aj.w, at4(dz, q));
+        }
+        if (ty == 0) {
+            gb[0] += dz.x;
+            gb[1] += dz.y;
+            gb[2] += dz.z;
+            gb[3] += dz.w;
+        }
     }
-    if (tid < H) {
-        float g = 0.0f;
-        for (int s = 0; s < TS; ++s) g += Dout[s][tid];
-        gb[tid] += g;
-    }
-    if (!below) return;
-    // dA_in[s][i] = sum_j W[j][i] dZ[s][j];  Din[s][i] = silu'(z_in) * dA_in   (s = ty + 16 a, i = tx + 16 q)
+    // dA_in[s][i] = sum_j W[j][i] dZ[s][j];  Din[s][i] = silu'(z_in) * dA_in   (s = ty + 8 a, i = 4 tx + q)
     float acc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[a][q] = 0.0f;
-#pragma unroll 4
-    for (int j = 0; j < H; ++j) {
-        float dz[4], wj[4];
+    tile_product(W, Dout, acc, ty, tx);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) dz[a] = Dout[ty + 16 * a][j];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) wj[q] = W[j][tx + 16 * q];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[a][q] = fmaf(wj[q], dz[a], acc[a][q]);
+    for (int a = 0; a < 4; ++a) {
+        float4* d = reinterpret_cast<float4*>(&Din[ty + 8 * a][4 * tx]);
+        float4 v = *d;
+        v.x *= acc[a][0];
+        v.y *= acc[a][1];
+        v.z *= acc[a][2];
+        v.w *= acc[a][3];
+        *d = v;
     }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) Din[ty + 16 * a][tx + 16 * q] *= acc[a][q];
 }
 
-__global__ void __launch_bounds__(256, 1) k_mlp_grad(const float* __restrict__ P, const float* __restrict__ feat,
+__global__ void __launch_bounds__(PIPES * PT, 1) k_mlp_grad(const float* __restrict__ P, const float* __restrict__ feat,
                                                      const float* __restrict__ target, long long n,
                                                      float* __restrict__ grad, double* __restrict__ loss) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    for (int k = tid; k < H * H; k += blockDim.x) {
-        S.W1[k / H][k % H] = bf16r(P[OW1 + k]);
-        S.W2[k / H][k % H] = bf16r(P[OW2 + k]);
+    const int pipe = threadIdx.x / PT, tid = threadIdx.x % PT, ty = tid >> 4, tx = tid & 15;
+    TrainTile& B = S.tile[pipe];
+    for (int k = threadIdx.x; k < H * H; k += blockDim.x) {
+        const float w1 = bf16r(P[OW1 + k]), w2 = bf16r(P[OW2 + k]);
+        S.W1[k / H][k % H] = w1;
+        S.W2[k / H][k % H] = w2;
+        S.V1[k % H][k / H] = w1;
+        S.V2[k % H][k / H] = w2;
     }
-    for (int k = tid; k < H; k += blockDim.x) {
+    for (int k = threadIdx.x; k < H; k += blockDim.x) {
         S.W0[k][0] = bf16r(P[OW0 + 2 * k]);
         S.W0[k][1] = bf16r(P[OW0 + 2 * k + 1]);
         S.b0[k] = P[OB0 + k];
         S.b1[k] = P[OB1 + k];
         S.b2[k] = P[OB2 + k];
         S.W3[k] = bf16r(P[OW3 + k]);
-        S.gW0[k][0] = S.gW0[k][1] = 0.0f;
-        S.gb0[k] = S.gb1[k] = S.gb2[k] = S.gW3[k] = 0.0f;
     }
-    if (tid == 0) {
-        S.b3 = P[OB3];
-        S.gb3 = 0.0f;
-        S.loss = 0.0;
+    if (threadIdx.x == 0) S.b3 = P[OB3];
+    // sums over samples that stay in registers: the output bias and the loss in
+    // the four threads of a sample's first, the outer layers' weights in thread
+    // (part, unit) over the samples 16 part .. + 15 of every tile
+    float gb3 = 0.0f, gW3 = 0.0f, gW00 = 0.0f, gW01 = 0.0f, gb0 = 0.0f;
+    double lsum = 0.0;
+    const int unit = tid & 63, s_first = 16 * (tid >> 6);
+    float gW1[4][8], gW2[4][8], gb1[4], gb2[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        gb1[q] = gb2[q] = 0.0f;
+#pragma unroll
+        for (int a = 0; a < 8; ++a) gW1[q][a] = gW2[q][a] = 0.0f;
     }
-    float gW1[4][4], gW2[4][4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int a = 0; a < 4; ++a) gW1[q][a] = gW2[q][a] = 0.0f;
     __syncthreads();
     const long long ntiles = (n + TS - 1) / TS;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    for (long long tile = (long long)blockIdx.x * PIPES + pipe; tile < ntiles; tile += (long long)gridDim.x * PIPES) {
         const long long s0 = tile * TS;
         if (tid < TS) {
             const long long i = s0 + tid;
             const bool ok = i < n;
-            S.x[tid][0] = ok ? feat[2 * i] : 0.0f;
-            S.x[tid][1] = ok ? feat[2 * i + 1] : 0.0f;
-            S.dy[tid] = ok ? target[i] : 0.0f;  // target, replaced by dL/dy below
+            B.x[tid][0] = ok ? feat[2 * i] : 0.0f;
+            B.x[tid][1] = ok ? feat[2 * i + 1] : 0.0f;
+            B.dy[tid] = ok ? target[i] : 0.0f;  // target, replaced by dL/dy below
         }
-        __syncthreads();
+        pipe_sync(pipe);
         // layer 0 (2 -> 64)
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int s = ty + 16 * a, j = tx + 16 * q;
-                const float z = fmaf(S.W0[j][0], S.x[s][0], fmaf(S.W0[j][1], S.x[s][1], S.b0[j]));
-                silu_train(z, S.A1[s][j], S.D1[s][j]);
+                const int s = ty + 8 * a, j = 4 * tx + q;
+                const float z = fmaf(S.W0[j][0], B.x[s][0], fmaf(S.W0[j][1], B.x[s][1], S.b0[j]));
+                silu_train(z, B.A1[s][j], B.D1[s][j]);
             }
-        __syncthreads();
-        dense_fwd(S.W1, S.b1, S.A1, S.A2, S.D2, ty, tx);
-        __syncthreads();
-        dense_fwd(S.W2, S.b2, S.A2, S.A3, S.D3, ty, tx);
-        __syncthreads();
+        pipe_sync(pipe);
+        dense_fwd(S.V1, S.b1, B.A1, B.A2, B.D2, ty, tx);
+        pipe_sync(pipe);
+        dense_fwd(S.V2, S.b2, B.A2, B.A3, B.D3, ty, tx);
+        pipe_sync(pipe);
         // layer 3 (64 -> 1): four threads per sample; loss sum (y - t)^2
         {
             const int s = tid >> 2, part = tid & 3;
             float y = 0.0f;
-            for (int j = part * 16; j < part * 16 + 16; ++j) y = fmaf(S.W3[j], S.A3[s][j], y);
+            for (int j = part * 16; j < part * 16 + 16; ++j) y = fmaf(S.W3[j], B.A3[s][j], y);
             y += __shfl_xor_sync(0xffffffffu, y, 1);
             y += __shfl_xor_sync(0xffffffffu, y, 2);
             __syncwarp();
             if (part == 0) {
                 y += S.b3;
                 const bool ok = s0 + s < n;
-                const float e = ok ? y - S.dy[s] : 0.0f;
-                S.y[s] = y;
-                S.dy[s] = 2.0f * e;
-                atomicAdd(&S.loss, (double)e * (double)e);
+                const float e = ok ? y - B.dy[s] : 0.0f;
+                B.dy[s] = 2.0f * e;
+                gb3 += 2.0f * e;
+                lsum += (double)e * (double)e;
             }
         }
-        __syncthreads();
+        pipe_sync(pipe);
         // layer 3 backward: gW3, gb3, dz3 = W3 dy silu'(z3)
-        if (tid < H) {
-            float g = 0.0f;
-            for (int s = 0; s < TS; ++s) g = fmaf(S.dy[s], S.A3[s][tid], g);
-            S.gW3[tid] += g;
-        }
-        if (tid == 0) {
-            float g = 0.0f;
-            for (int s = 0; s < TS; ++s) g += S.dy[s];
-            S.gb3 += g;
-        }
+#pragma unroll
+        for (int s = 0; s < 16; ++s) gW3 = fmaf(B.dy[s_first + s], B.A3[s_first + s][unit], gW3);
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int s = ty + 16 * a, j = tx + 16 * q;
-                S.D3[s][j] *= S.W3[j] * S.dy[s];
+                const int s = ty + 8 * a, j = 4 * tx + q;
+                B.D3[s][j] *= S.W3[j] * B.dy[s];
             }
-        __syncthreads();
-        dense_bwd(S.W2, S.D3, S.A2, S.D2, gW2, S.gb2, ty, tx, tid, true);
-        __syncthreads();
-        dense_bwd(S.W1, S.D2, S.A1, S.D1, gW1, S.gb1, ty, tx, tid, true);
-        __syncthreads();
+        pipe_sync(pipe);
+        dense_bwd(S.W2, B.D3, B.A2, B.D2, gW2, gb2, ty, tx);
+        pipe_sync(pipe);
+        dense_bwd(S.W1, B.D2, B.A1, B.D1, gW1, gb1, ty, tx);
+        pipe_sync(pipe);
         // layer 0 backward
-        if (tid < H) {
-            float g0 = 0.0f, g1 = 0.0f, gb = 0.0f;
-            for (int s = 0; s < TS; ++s) {
-                const float dz = S.D1[s][tid];
-                g0 = fmaf(dz, S.x[s][0], g0);
-                g1 = fmaf(dz, S.x[s][1], g1);
-                gb += dz;
-            }
-            S.gW0[tid][0] += g0;
-            S.gW0[tid][1] += g1;
-            S.gb0[tid] += gb;
+#pragma unroll
+        for (int s = 0; s < 16; ++s) {
+            const float dz = B.D1[s_first + s][unit];
+            gW00 = fmaf(dz, B.x[s_first + s][0], gW00);
+            gW01 = fmaf(dz, B.x[s_first + s][1], gW01);
+            gb0 += dz;
+        }
+        pipe_sync(pipe);
+    }
+    // the pipelines' weight gradients added up in the tiles' memory, then one
+    // set of atomics per block
+    __syncthreads();
+    float* const sum = reinterpret_cast<float*>(S.tile);
+    for (int p = 0; p < PIPES; ++p) {
+        if (pipe == p) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int a = 0; a < 8; ++a) {
+                    const int k = (4 * tx + q) * H + 8 * ty + a;
+                    sum[k] = p ? sum[k] + gW1[q][a] : gW1[q][a];
+                    sum[H * H + k] = p ? sum[H * H + k] + gW2[q][a] : gW2[q][a];
+                }
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int j = tx + 16 * q, i = ty + 16 * a;
-            atomicAdd(&grad[OW1 + j * H + i], gW1[q][a]);
-            atomicAdd(&grad[OW2 + j * H + i], gW2[q][a]);
-        }
-    for (int k = tid; k < H; k += blockDim.x) {
-        atomicAdd(&grad[OW0 + 2 * k], S.gW0[k][0]);
-        atomicAdd(&grad[OW0 + 2 * k + 1], S.gW0[k][1]);
-        atomicAdd(&grad[OB0 + k], S.gb0[k]);
-        atomicAdd(&grad[OB1 + k], S.gb1[k]);
-        atomicAdd(&grad[OB2 + k], S.gb2[k]);
-        atomicAdd(&grad[OW3 + k], S.gW3[k]);
+    for (int k = threadIdx.x; k < H * H; k += blockDim.x) {
+        atomicAdd(&grad[OW1 + k], sum[k]);
+        atomicAdd(&grad[OW2 + k], sum[H * H + k]);
     }
-    if (tid == 0) {
-        atomicAdd(&grad[OB3], S.gb3);
-        atomicAdd(loss, S.loss);
+    if (ty == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            atomicAdd(&grad[OB1 + 4 * tx + q], gb1[q]);
+            atomicAdd(&grad[OB2 + 4 * tx + q], gb2[q]);
+        }
+    }
+    atomicAdd(&grad[OW0 + 2 * unit], gW00);
+    atomicAdd(&grad[OW0 + 2 * unit + 1], gW01);
+    atomicAdd(&grad[OB0 + unit], gb0);
+    atomicAdd(&grad[OW3 + unit], gW3);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        gb3 += __shfl_xor_sync(0xffffffffu, gb3, o);
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    }
+    if ((tid & 31) == 0) {
+        atomicAdd(&grad[OB3], gb3);
+        atomicAdd(loss, lsum);
     }
 }
 
@@ -717,9 +775,9 @@ int sfp_mlp_grad(const float* params, const float* features, const float* target
         MLP_CUDA(cudaFuncSetAttribute((const void*)k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set = true;
     }
-    const long long tiles = (N + TS - 1) / TS;
-    const int grid = (int)(tiles < sm_count_here() ? tiles : sm_count_here());
-    k_mlp_grad<<<grid, 256, smem, reinterpret_cast<cudaStream_t>(stream)>>>(params, features, targets, N, grad, loss);
+    const long long tiles = (N + TS - 1) / TS, blocks = (tiles + PIPES - 1) / PIPES;
+    const int grid = (int)(blocks < sm_count_here() ? blocks : sm_count_here());
+    k_mlp_grad<<<grid, PIPES * PT, smem, reinterpret_cast<cudaStream_t>(stream)>>>(params, features, targets, N, grad, loss);
     MLP_CUDA(cudaGetLastError());
     return SFP_OK;
 }
