@@ -143,6 +143,16 @@ int sfp_update_tau(double *tau, const double *inv_gamma, const double *chi, doub
 int sfp_inv_gamma(const double *ux, const double *uy, const double *uz, double *inv_gamma, int64_t N, int massless,
                   void *stream);
 
+/* Grow the arrays of a species: dst[0:old_n] = src[0:old_n], and every byte of
+ * dst[old_n:new_n] = fill.  Elements of 1 or 8 bytes; dst and src disjoint. */
+typedef struct sfp_grow_array {
+    const void *src;
+    void *dst;
+    int32_t size; /* bytes of an element */
+    int32_t fill; /* byte of the new elements */
+} sfp_grow_array;
+int sfp_grow_arrays(const sfp_grow_array *arrays, int32_t n, int64_t old_n, int64_t new_n, void *stream);
+
 /* ---- fused step: Simulation.start (simulation.py:74-160) -------------------
  * A run owns the device bookkeeping of one or more instances whose species
  * buffers are described by segments (device pointers owned by the caller). */

@@ -35,6 +35,10 @@ class Segment(ctypes.Structure):
     ]
 
 
+class GrowArray(ctypes.Structure):
+    _fields_ = [("src", P), ("dst", P), ("size", c_i32), ("fill", c_i32)]
+
+
 class Instance(ctypes.Structure):
     _fields_ = [("seed", c_u64), ("field_params", P), ("first_seg", c_i32), ("n_seg", c_i32)]
 
@@ -95,6 +99,7 @@ _SIGS = {
     "sfp_photon_from_rejection_sampling": ([P, P, c_d, c_i64, P, P, P, P, c_u64, c_u32, c_u32, P], c_i32),
     "sfp_pair_from_rejection_sampling": ([P, P, c_d, c_i64, P, P, P, P, c_u64, c_u32, c_u32, P], c_i32),
     "sfp_update_tau": ([P, P, P, c_d, c_i64, P, P, P, P, c_u64, c_u32, c_u32, P], c_i32),
+    "sfp_grow_arrays": ([P, c_i32, c_i64, c_i64, P], c_i32),
     "sfp_inv_gamma": ([P, P, P, P, c_i64, c_i32, P], c_i32),
     "sfp_run_create": ([P, P, c_i32, P, c_i32, P, P, P], c_i32),
     "sfp_run_update": ([P, c_i32, P, P], c_i32),

@@ -271,6 +271,30 @@ __global__ void k_fei_scatter(const unsigned char* __restrict__ ev, long long N,
     }
 }
 
+// A species' arrays in larger ones, the new slots filled: one launch over all
+// of them (blockIdx.y is the array).  Used where the arrays are small and a
+// growth is bound by its launches: a copy and a fill for each of up to 17
+// arrays.  Each thread moves whole elements; loads and stores of a warp are
+// consecutive, and the sources need no more alignment than their elements.
+constexpr int kGrowArrays = 32;
+struct grow_list {
+    sfp_grow_array a[kGrowArrays];
+};
+
+__global__ void k_grow(grow_list L, long long old_n, long long new_n) {
+    const sfp_grow_array& A = L.a[blockIdx.y];
+    if (A.size == 8) {
+        const unsigned long long fill = A.fill ? 0x0101010101010101ull * (unsigned char)A.fill : 0ull;
+        const unsigned long long* src = static_cast<const unsigned long long*>(A.src);
+        unsigned long long* dst = static_cast<unsigned long long*>(A.dst);
+        GRID_STRIDE(i, new_n) dst[i] = i < old_n ? src[i] : fill;
+    } else {
+        const unsigned char* src = static_cast<const unsigned char*>(A.src);
+        unsigned char* dst = static_cast<unsigned char*>(A.dst);
+        GRID_STRIDE(i, new_n) dst[i] = i < old_n ? src[i] : (unsigned char)A.fill;
+    }
+}
+
 __global__ void k_create_photon(const double* __restrict__ xs, const double* __restrict__ ys,
                                 const double* __restrict__ zs, const double* __restrict__ uxs,
                                 const double* __restrict__ uys, const double* __restrict__ uzs, double* __restrict__ xd,
@@ -781,6 +805,22 @@ int sfp_inv_gamma(const double* ux, const double* uy, const double* uz, double* 
     RETURN_IF_EMPTY(N);
     k_inv_gamma<<<grid_for(N), kBlock, 0, as_stream(stream)>>>(ux, uy, uz, ig, N, massless);
     SFP_CHECK_LAUNCH();
+    return SFP_OK;
+}
+
+int sfp_grow_arrays(const sfp_grow_array* arrays, int32_t n, int64_t old_n, int64_t new_n, void* stream) {
+    if (!arrays || n < 0 || old_n < 0 || new_n < old_n) return fail(SFP_EINVAL, "sfp_grow_arrays: bad arguments");
+    for (int i = 0; i < n; ++i)
+        if (!arrays[i].dst || (!arrays[i].src && old_n) || (arrays[i].size != 1 && arrays[i].size != 8))
+            return fail(SFP_EINVAL, "sfp_grow_arrays: NULL array or an element size other than 1 or 8");
+    RETURN_IF_EMPTY(new_n);
+    for (int first = 0; first < n; first += kGrowArrays) {
+        grow_list L = {};
+        const int m = n - first < kGrowArrays ? n - first : kGrowArrays;
+        for (int i = 0; i < m; ++i) L.a[i] = arrays[first + i];
+        k_grow<<<dim3(grid_for(new_n), (unsigned int)m), kBlock, 0, as_stream(stream)>>>(L, old_n, new_n);
+        SFP_CHECK_LAUNCH();
+    }
     return SFP_OK;
 }
 
