@@ -200,8 +200,12 @@ int sfp_run_steps(sfp_run *r, int64_t nsteps, int graph_chunk, void *stream);
 /* like sfp_run_steps without graphs, with CUDA events recorded around the
  * kernels of every step on the run's stream; synchronous.
  * kernel_ms[3*i + k] is the duration of step i's massive (k=0) and photon
- * (k=1) kernels and of its scan + appends kernels (k=2); 0 for kernels the
- * run does not launch (3*nsteps entries). */
+ * (k=1) kernels and of its appends kernel (k=2); 0 for kernels the run does
+ * not launch (3*nsteps entries).  The event scan and the next step's
+ * bookkeeping run in the last block of the photon kernel (of the massive one
+ * in a run without photons).  Calls of four steps and more step a large
+ * photon population through a store of hot photons, as sfp_run_steps does;
+ * k=1 then is that kernel's time. */
 int sfp_run_steps_timed(sfp_run *r, int64_t nsteps, float *kernel_ms, void *stream);
 /* Photon positions are stored as of the run's position epoch: the step
  * kernels advance a photon's position in registers (photons fly straight,
@@ -226,6 +230,9 @@ int sfp_run_pending_need(sfp_run *r, int64_t *need);
 int sfp_run_resume(sfp_run *r, void *stream);
 /* kernels that the run's step calls have launched so far (graph replays included) */
 int sfp_run_launches(sfp_run *r, int64_t *count);
+/* synchronous: photons in the store of the last step call, of which its photon
+ * kernel read 40 bytes (float32 form; float64: 52) a step; 0 if it kept none */
+int sfp_run_hot_photons(sfp_run *r, int64_t *count);
 /* Small populations run several steps per launch, with barriers between the
  * launch's blocks; a wait at one gives up after two seconds and sets the device
  * error SFP_DEV_BARRIER.  This launches a step in which one block never

@@ -125,6 +125,7 @@ _SIGS = {
     "sfp_run_destroy": ([P], c_i32),
     "sfp_release_cached": ([], c_i32),
     "sfp_run_launches": ([P, P], c_i32),
+    "sfp_run_hot_photons": ([P, P], c_i32),
     "sfp_run_barrier_withheld": ([P, P], c_i32),
 }
 

@@ -4,10 +4,12 @@
 //     (the plugin boundary, sfparticles/particles.py:14-25);
 //   * NVRTC compilation / loading of field-specialised step modules;
 //   * step runs: device bookkeeping, persistent launches of the massive /
-//     photon / scan / appends kernels, CUDA graphs.
+//     photon / appends kernels, several steps per launch for small
+//     populations, a store of hot photons for large ones, CUDA graphs.
 //
 // Device memory of particle buffers belongs to the caller; a run allocates
-// only its own bookkeeping (segment tables, tile maps, event counters).
+// its bookkeeping (segment tables, tile maps, event counters) and, for calls
+// of several steps over many photons, the store of hot photons.
 #include <cuda_runtime.h>
 #include <nvrtc.h>
 
@@ -992,6 +994,7 @@ struct sfp_run {
     cudaKernel_t k_hot = nullptr, k_hot_build = nullptr;        // hot photons (rejection sampling)
     run_block hot_block;                                        // their store
     long long hot_room = 0;                                     // entries it holds
+    bool hot_last = false;                                      // the last call kept a store
     long long hot_refused = 0;                                  // entries that found no memory
     long long *d_hot_start = nullptr, *d_hot_cap = nullptr;
     int64_t launches = 0;                                       // kernels of its steps so far (graph replays too)
@@ -1664,6 +1667,7 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
     int64_t done = 0;
     const bool ml = long_tiles(r, r->mg.seg, SFP_TILE_TARGET_M), pl = long_tiles(r, r->pg.seg, SFP_TILE_TARGET);
     if (small_run(r, ml, pl)) {
+        r->hot_last = false;
         if (const int rc0 = launch_small(r, nsteps)) return rc0;
         if (const int rc0 = cg.done()) return rc0;
         SFP_CUDA(cudaEventRecord(r->ev_out, r->s));
@@ -1671,6 +1675,7 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
         return SFP_OK;
     }
     const bool hot = pl && nsteps >= HOT_MIN_STEPS && hot_store(r, cs);
+    r->hot_last = hot;
     if (const int rc0 = launch_first(r, ml, pl, hot)) return rc0;
     if (graph_chunk > 0 && nsteps >= graph_chunk) {
         const int key = graph_chunk * 8 + (hot ? 4 : 0) + (ml ? 2 : 0) + (pl ? 1 : 0);
@@ -1718,7 +1723,8 @@ int sfp_run_steps_timed(sfp_run* r, int64_t nsteps, float* kernel_ms, void* stre
     for (auto& e : ev)
         if (cudaEventCreate(&e) != cudaSuccess) rc = fail(SFP_ECUDA, "cudaEventCreate");
     const bool ml = long_tiles(r, r->mg.seg, SFP_TILE_TARGET_M), pl = long_tiles(r, r->pg.seg, SFP_TILE_TARGET);
-    const bool hot = pl && hot_store(r, cs);
+    const bool hot = pl && nsteps >= HOT_MIN_STEPS && hot_store(r, cs);
+    r->hot_last = hot;
     if (rc == SFP_OK) rc = launch_first(r, ml, pl, hot);
     for (int64_t k = 0; k < nsteps && rc == SFP_OK; ++k) rc = launch_unit(r, r->s, &ev[6 * k], ml, pl, hot);
     r->launches += nsteps * step_launches(r, hot);
@@ -1847,6 +1853,17 @@ int sfp_run_resume(sfp_run* r, void* stream) {
 int sfp_run_launches(sfp_run* r, int64_t* count) {
     if (!r || !count) return fail(SFP_EINVAL, "sfp_run_launches: NULL argument");
     *count = r->launches;
+    return SFP_OK;
+}
+
+int sfp_run_hot_photons(sfp_run* r, int64_t* count) {
+    if (!r || !count) return fail(SFP_EINVAL, "sfp_run_hot_photons: NULL argument");
+    *count = 0;
+    if (!r->hot_last) return SFP_OK;
+    std::vector<unsigned long long> c(r->n_seg, 0);
+    SFP_CUDA(cudaMemcpyAsync(c.data(), r->h.hot.count, r->n_seg * sizeof(c[0]), cudaMemcpyDeviceToHost, r->s));
+    SFP_CUDA(cudaStreamSynchronize(r->s));
+    for (int s : r->pg.seg) *count += (int64_t)c[s];
     return SFP_OK;
 }
 

@@ -1,5 +1,6 @@
-// sfp_step.cuh -- the fused particle step (one launch per kernel advances
-// every species of every instance by one step) plus its bookkeeping kernel.
+// sfp_step.cuh -- the fused particle step: every species of every instance by
+// one step in three launches (massive, photon, appends), or several steps in
+// one launch where the population is small (sfp_steps_body).
 //
 // Compiled by NVRTC together with a generated field program that defines
 //     SFP_DEVICE_INLINE void sfp_field_program(double x, double y, double z,
@@ -14,20 +15,25 @@
 //   5. pairs appended, converted photons pruned,
 //   6. every pushed particle -- children included -- pushed from t to t+dt:
 //      half position, fields at t+dt/2, Boris / Boris-TBMT (+LL/CLL), half position.
-// After the bookkeeping kernel a step is:
+// A call's first step is prepared by a one-block kernel (sfp_book_kernel); a
+// step is:
 //   massive -- 3; a particle with an event is marked and left as it was at t
 //              (its delta stored), every other one takes 6;
 //   photon  -- 2; a converted photon is marked (its delta stored), every
-//              other one takes 6;
-//   scan    -- the children's slots: per-tile event counts scanned in the
-//              reference's order;
+//              other one takes 6.  Calls of several steps with many photons
+//              visit only the photons that could convert, from a store of
+//              them (sfp_hot_*);
+//   step end, in the last block of the photon launch -- the children's slots:
+//              per-tile event counts scanned in the reference's order; the
+//              next step planned (sfp_step_end);
 //   appends -- 4 (child from the parent's state at t, then the parent's
 //              recoil and 6) and 5 (children pushed, 6), at those slots.
 // The massive and photon kernels touch disjoint memory: each writes only
 // below the start-of-step counts of its own group's buffers.  Appends are
 // ordered: a child gets the slot that the reference's find_event_index +
 // create_* would give it, so Philox streams keyed by slot are reproducible.
-// No kernel waits on another block.
+// Only the one-launch kernel's blocks wait on one another, at grid barriers of
+// a cooperative launch, each wait with a time limit (sfp_grid_barrier).
 #pragma once
 #include "sfp_device.cuh"
 #include "sfp_device32.cuh"
@@ -2379,7 +2385,7 @@ __device__ __forceinline__ void sfp_steps_body(const sfp_run_dev* __restrict__ R
 }
 
 // kernels: sfp_massive_<form>_<qed>_s<stages>_b<blocks>,
-// sfp_photon_<form>_<qed>_s<stages>_b<blocks>, sfp_scan_kernel, sfp_appends_<form>
+// sfp_photon_<form>_<qed>_s<stages>_b<blocks>, sfp_book_kernel, sfp_appends_<form>
 // (long-tile kernels) and sfp_massive_<form>_<qed>_s<stages>_b<blocks>_t,
 // sfp_photon_..._t (any tile length: the steps of small populations)
 #define SFP_MASSIVE_KERNEL(FORM_S, QED_S, FORM, QED, STAGES, MINB)                                             \

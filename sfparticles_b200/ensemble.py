@@ -183,10 +183,11 @@ class Ensemble(object):
             if done == 0 and not halted:
                 raise _lib.SFPError("the step made no progress")
 
-    def time_step_kernel(self, nstep: int):
+    def time_step_kernel(self, nstep: int, per_call: int = 1):
         """Advance `nstep` steps with eager launches and return, per step, the
-        CUDA-event durations [ms] of its (massive, photon, scan + appends)
-        kernels, with the buffered counts before and after."""
+        CUDA-event durations [ms] of its (massive, photon, appends)
+        kernels, with the buffered counts before and after (per_call as in
+        Simulation.time_step_kernel)."""
         if self._run is None:
             self._begin()
         L = _lib.load()
@@ -195,19 +196,21 @@ class Ensemble(object):
         st = _lib.RunState()
         nbuf = (ctypes.c_int64 * len(allp))()
         out = []
-        for _ in range(int(nstep)):
-            ms = (ctypes.c_float * 3)()
-            _lib.check(L.sfp_run_steps_timed(self._run, 1, ms, _stream_ptr()), "sfp_run_steps_timed")
+        end = self.step + int(nstep)
+        while self.step < end:
+            k, first = min(int(per_call), end - self.step), self.step
+            ms = (ctypes.c_float * (3 * k))()
+            _lib.check(L.sfp_run_steps_timed(self._run, k, ms, _stream_ptr()), "sfp_run_steps_timed")
             self._pos_dirty = True
             _lib.check(L.sfp_run_read_state(self._run, ctypes.byref(st), nbuf, _stream_ptr()), "read_state")
             self.kernel_launches += launches_since(self, self._run)
             if st.error or (st.halted and not st.appends_pending):
                 raise _lib.SFPError("timed step did not complete")
+            out += [tuple(float(v) for v in ms[3 * j:3 * j + 3]) for j in range(int(st.step) - first)]
             if st.appends_pending:  # finish the step; its appends kernel was not timed
                 resolve_pending(self._run, allp, lambda: self._update_run(counts=False))
                 _lib.check(L.sfp_run_read_state(self._run, ctypes.byref(st), nbuf, _stream_ptr()), "read_state")
-            else:
-                out.append((float(ms[0]), float(ms[1]), float(ms[2])))
+            self.step = int(st.step)
             for i, p in enumerate(allp):
                 p.N_buffered = int(nbuf[i])
                 p._touch()

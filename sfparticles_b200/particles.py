@@ -518,8 +518,9 @@ class Particles(object):
         GROW_TOGETHER bytes a growth is bound by its allocations and
         launches, three of them for each array (a run of the per-op engine
         from 5e4 electrons, 18 growths in 32 steps: 40.6 ms an array at a
-        time, 32 ms together); a larger one keeps to an array at a time, which needs the room of one array only beside the
-        species, and returns False here."""
+        time, 32 ms together).  A larger one keeps to an array at a time,
+        which needs the room of one array only beside the species; it returns
+        False here."""
         import torch
         sizes = [v.element_size() for v in self._arr.values()]
         steps = [(new * s + 255) // 256 * 256 for s in sizes]

@@ -9,18 +9,21 @@ generates QED events, appends photons then pairs, and pushes every pushed
 particle (children included) from t to t+dt (simulation.py:102-144);
 ``start`` ends by pruning and returning host arrays (simulation.py:158-161).
 
-Each step is a one-block bookkeeping launch followed by the massive kernel
-(e+-: emission events; emitters marked, every other particle pushed), the
-photon kernel (pair events; converted photons marked, the others pushed), a
-one-block scan of both kinds of event counts and the appends kernel (photon
+A step is three launches: the massive kernel (e+-: emission events; emitters
+marked, every other particle pushed), the photon kernel (pair events;
+converted photons marked, the others pushed; its last block scans both kinds
+of event counts and plans the next step) and the appends kernel (photon
 children, the emitters' recoil and push, e-/e+ children, all written in the
-reference's order and pushed); steps between progress reports / callbacks
-run back to back on the device, replayed from CUDA graphs, with no host
-synchronisation.  No kernel overruns a buffer: the scan compares each
-destination's room with the step's exact number of children before any is
-written, and if one lacks room the step waits; the host grows that buffer
-by the reference rule and resumes the step.  Between device chunks the host
-grows destinations ahead of the append rates it has seen, so waits are rare.
+reference's order and pushed).  Large photon populations are stepped through a
+store of the photons that could create a pair, built once per native call;
+small populations take many steps in one cooperative launch.  Steps between
+progress reports / callbacks run back to back on the device, replayed from
+CUDA graphs, with no host synchronisation.  No kernel overruns a buffer: the
+scan compares each destination's room with the step's exact number of children
+before any is written, and if one lacks room the step waits; the host grows
+that buffer by the reference rule and resumes the step.  Between device chunks
+the host grows destinations ahead of the append rates it has seen, so waits
+are rare.
 
 Extra keyword arguments (no reference counterpart):
   seed        -- 64-bit key of the Philox streams (default: random);
@@ -498,12 +501,14 @@ class Simulation(object):
             p._to_host()
         _release_cached_blocks()
 
-    def time_step_kernel(self, nstep: int):
+    def time_step_kernel(self, nstep: int, per_call: int = 1):
         """Advance `nstep` steps with eager launches and return, per step, the
-        CUDA-event durations [ms] of its (massive, photon, scan + appends)
+        CUDA-event durations [ms] of its (massive, photon, appends)
         kernels (recorded on the stream they run on; 0 for a kernel the run
         does not launch), with the buffered counts before and after.  A step
-        that waited for room is finished untimed and not reported."""
+        that waited for room is finished untimed and not reported.  per_call:
+        steps of one native call; from four on, a large photon population is
+        stepped through the call's store of hot photons, as in longer runs."""
         if getattr(self, "_run", None) is None:
             self._begin()
         before = [p.N_buffered for p in self.all_particles]
@@ -511,19 +516,21 @@ class Simulation(object):
         L = _lib.load()
         st = _lib.RunState()
         nbuf = (ctypes.c_int64 * len(self.all_particles))()
-        for _ in range(int(nstep)):
-            ms = (ctypes.c_float * 3)()
-            _lib.check(L.sfp_run_steps_timed(self._run, 1, ms, _stream_ptr()), "sfp_run_steps_timed")
+        end = self.step + int(nstep)
+        while self.step < end:
+            k, first = min(int(per_call), end - self.step), self.step
+            ms = (ctypes.c_float * (3 * k))()
+            _lib.check(L.sfp_run_steps_timed(self._run, k, ms, _stream_ptr()), "sfp_run_steps_timed")
             self._pos_dirty = True
             _lib.check(L.sfp_run_read_state(self._run, ctypes.byref(st), nbuf, _stream_ptr()), "read_state")
             self.kernel_launches += launches_since(self, self._run)
             if st.error or (st.halted and not st.appends_pending):
                 raise _lib.SFPError("timed step did not complete")
+            out += [tuple(float(v) for v in ms[3 * j:3 * j + 3]) for j in range(int(st.step) - first)]
             if st.appends_pending:  # finish the step; its appends kernel was not timed
                 resolve_pending(self._run, self.all_particles, lambda: self._update_run(self._run, counts=False))
                 _lib.check(L.sfp_run_read_state(self._run, ctypes.byref(st), nbuf, _stream_ptr()), "read_state")
-            else:
-                out.append((float(ms[0]), float(ms[1]), float(ms[2])))
+            self.step = int(st.step)
             for i, p in enumerate(self.all_particles):
                 p.N_buffered = int(nbuf[i])
                 p._touch()
