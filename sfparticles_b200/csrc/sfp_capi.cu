@@ -1555,55 +1555,68 @@ constexpr int64_t HOT_MIN_STEPS = 4;
 // steps of one launch of the one-launch kernel
 constexpr int64_t SMALL_STEPS = 256;
 
-// room for the store at the current counts (5/8 of a segment's photons, new
-// ones included); false: the call does without (no memory to spare: the store
-// takes at most half of what is free)
+// room for n entries of the store, with some to grow into, in at most half of
+// the memory that is free; false, and remembered, where that is not enough
+static bool hot_room(sfp_run* r, long long n) {
+    if (r->hot_refused && n >= r->hot_refused) return false;
+    const size_t each = r->hot_f64 ? 52 : 40;
+    const bool f64 = r->hot_f64;
+    const long long room = r->hot_room ? n + n / 2 : n + n / 8;
+    const size_t bytes = (size_t)room * each;
+    if (r->hot_block.p) {
+        if (cudaStreamSynchronize(r->s) != cudaSuccess) return false;  // earlier calls still use it
+        block_put(r->hot_block);
+    }
+    r->hot_block = run_block();
+    r->hot_room = 0;
+    size_t free_b = 0, all_b = 0;
+    if (!block_cached(bytes) && (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || free_b / 2 < bytes)) {
+        r->hot_refused = n;
+        return false;
+    }
+    if (!block_get(bytes, &r->hot_block)) {
+        r->hot_refused = n;
+        return false;
+    }
+    r->hot_room = room;
+    char* p = static_cast<char*>(r->hot_block.p);
+    const size_t d8 = (size_t)room * 8, du = (size_t)room * (f64 ? 8 : 4);
+    sfp_hot_dev& H = r->h.hot;
+    H.x = reinterpret_cast<double*>(p);
+    H.y = reinterpret_cast<double*>(p + d8);
+    H.z = reinterpret_cast<double*>(p + 2 * d8);
+    H.ux = p + 3 * d8;
+    H.uy = p + 3 * d8 + du;
+    H.uz = p + 3 * d8 + 2 * du;
+    H.idx = reinterpret_cast<unsigned int*>(p + 3 * d8 + 3 * du);
+    if (cudaMemcpyAsync(r->d, &r->h, sizeof(sfp_run_dev), cudaMemcpyHostToDevice, r->s) != cudaSuccess) return false;
+    return true;
+}
+
+// The store at the current counts: room for 5/8 of a segment's photons (new
+// ones included), which holds all hot ones in most scenes, or, where memory is
+// short, 3/8 or 1/4, which does late in a run, when most photons are soft: 1.4e9
+// photons of 256 collisions, one in six hot, 50 GB free: 5/8 would take 42 GB,
+// and a step over every photon takes 15.7 ms, through the store 4.9.  A store that
+// turns out too small is dropped by the kernel that fills it (hot_ok), and the
+// call steps every photon.  false: the call does without.
 static bool hot_store(sfp_run* r, cudaStream_t caller) {
     if (!r->k_hot) return false;
     if (capturing(caller)) return false;  // a captured call gets launches only
-    const bool f64 = r->k_hot && r->hot_f64;
     std::vector<long long> start(r->n_seg, 0), cap(r->n_seg, 0);
-    long long n = 0;
-    for (int s : r->pg.seg) {
-        const long long nb = r->nb_lo[s];
-        if (r->segs[s].capacity >= 0xFFFFFFFFll) return false;  // entries hold 32-bit indices
-        start[s] = n;
-        cap[s] = r->segs[s].bw && r->segs[s].push ? (nb / 8 * 5 + 65536 + 63) / 64 * 64 : 0;
-        n += cap[s];
+    bool have = false;
+    for (int eighths : {5, 3, 2}) {
+        long long n = 0;
+        for (int s : r->pg.seg) {
+            const long long nb = r->nb_lo[s];
+            if (r->segs[s].capacity >= 0xFFFFFFFFll) return false;  // entries hold 32-bit indices
+            start[s] = n;
+            cap[s] = r->segs[s].bw && r->segs[s].push ? (nb / 8 * eighths + 65536 + 63) / 64 * 64 : 0;
+            n += cap[s];
+        }
+        if ((have = n <= r->hot_room || hot_room(r, n))) break;
     }
-    const size_t each = f64 ? 52 : 40;
-    if (n > r->hot_room) {
-        if (r->hot_refused && n >= r->hot_refused) return false;
-        const long long room = r->hot_room ? n + n / 2 : n + n / 8;
-        const size_t bytes = (size_t)room * each;
-        if (r->hot_block.p) {
-            if (cudaStreamSynchronize(r->s) != cudaSuccess) return false;  // earlier calls still use it
-            block_put(r->hot_block);
-        }
-        r->hot_block = run_block();
-        r->hot_room = 0;
-        size_t free_b = 0, all_b = 0;
-        if (!block_cached(bytes) && (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || free_b / 2 < bytes)) {
-            r->hot_refused = n;
-            return false;
-        }
-        if (!block_get(bytes, &r->hot_block)) {
-            r->hot_refused = n;
-            return false;
-        }
-        r->hot_room = room;
-        char* p = static_cast<char*>(r->hot_block.p);
-        const size_t d8 = (size_t)room * 8, du = (size_t)room * (f64 ? 8 : 4);
-        sfp_hot_dev& H = r->h.hot;
-        H.x = reinterpret_cast<double*>(p);
-        H.y = reinterpret_cast<double*>(p + d8);
-        H.z = reinterpret_cast<double*>(p + 2 * d8);
-        H.ux = p + 3 * d8;
-        H.uy = p + 3 * d8 + du;
-        H.uz = p + 3 * d8 + 2 * du;
-        H.idx = reinterpret_cast<unsigned int*>(p + 3 * d8 + 3 * du);
-        if (cudaMemcpyAsync(r->d, &r->h, sizeof(sfp_run_dev), cudaMemcpyHostToDevice, r->s) != cudaSuccess) return false;
-    }
+    if (!have) return false;
     return cudaMemcpyAsync(r->d_hot_start, start.data(), r->n_seg * sizeof(long long), cudaMemcpyHostToDevice, r->s) ==
                cudaSuccess &&
            cudaMemcpyAsync(r->d_hot_cap, cap.data(), r->n_seg * sizeof(long long), cudaMemcpyHostToDevice, r->s) ==

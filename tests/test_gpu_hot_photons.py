@@ -101,3 +101,36 @@ def test_several_instances():
             assert np.array_equal(x, y)
     for e in ens:
         e.finish()
+
+
+# entries: 5/8, 3/8 and 1/4 of 8e6 photons, with 1/8 to grow into, take 228, 138 and 93 MB in the float32 form;
+# the store may take half of the free memory
+@pytest.mark.parametrize("free_mb,kept", [(2000, True), (360, True), (230, True), (120, False)])
+def test_store_where_memory_is_short(free_mb, kept):
+    import ctypes
+
+    import torch
+
+    from sfparticles_b200 import _lib
+    cuda_or_skip()
+    one, many = (_sim("fp32", _soft, n_ph=8_000_000) for _ in range(2))
+    for s in (one, many):
+        s.run_on_device(2)
+        s.reserve(STEPS)
+    for _ in range(STEPS):
+        one.run_on_device(1)
+    _lib.call("sfp_release_cached")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    room = torch.cuda.mem_get_info()[0] - free_mb * 1_000_000
+    filler = torch.empty(room, dtype=torch.uint8, device="cuda")
+    many.run_on_device(STEPS)
+    n = ctypes.c_int64()
+    _lib.call("sfp_run_hot_photons", many._run, ctypes.byref(n))
+    del filler
+    torch.cuda.empty_cache()
+    assert (n.value > 0) == kept
+    for x, y in zip(_arrays(one), _arrays(many)):
+        assert np.array_equal(x, y)
+    one.finish()
+    many.finish()
