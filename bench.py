@@ -62,9 +62,10 @@ BYTES_PAIR = 155    # pair event in the appends kernel: parent state + delta rea
 # one-kernel ncu capture of the collision window at 1e6 e- (photon kernel:
 # 2.38e7 photons, 1.17 GB of state, larger than L2, so traffic scales with
 # the units processed): 1.1695e9 read + 0.0036e9 written against 1.1680e9.
-# Only kernels whose state exceeds L2 in that capture are listed; the hot
-# photons' kernel has not been captured.
-NCU_TRAFFIC_RATIO = {"photon_full": (1.169452e9 + 3.648256e6) / 1.167978920e9}
+# Only kernels whose state exceeds L2 in that capture are listed.  The hot
+# photons' kernel (4.9e6 of 2.4e7 photons): 0.19606e9 read against 40 bytes of
+# each; what it writes are other kernels' lines leaving L2.
+NCU_TRAFFIC_RATIO = {"photon_full": (1.169452e9 + 3.648256e6) / 1.167978920e9, "photon": 1.0}
 
 WORKLOAD = "scaled cascade: 1e7 e- (gamma0 2000 +-1%, sigma_perp 1um, sigma_par 5um) x LP Gaussian a0=200 " \
            "(0.8um, w0 3um, 25fs FWHM), photons + pairs, dt=T0/100, 3000 steps"
@@ -1177,8 +1178,8 @@ def run_ours(args, rank, world):
     return dict(ms=ms, particle_steps=tot_ps, counts=counts, launches=launches, clocks=clk.summary(),
                 roofline={"bound": "hbm", "achieved": dk["achieved_gbs"], "peak": peak, "unit": "GB/s",
                           "frac": dk["achieved_gbs"] / peak, "peak_kind": peak_kind,
-                          "traffic": (dk["alg_bytes_per_launch"] * NCU_TRAFFIC_RATIO["photon_full"]
-                                      if dominant == "photon" and not hot else None),
+                          "traffic": (dk["alg_bytes_per_launch"] * NCU_TRAFFIC_RATIO["photon" if hot else "photon_full"]
+                                      if dominant == "photon" else None),
                           "traffic_note": "ncu DRAM bytes of a 1e6-electron capture scaled by units processed",
                           "kernel": dk["kernel"], "kernel_avg_ms": dk["avg_ms"],
                           "alg_bytes_per_launch": dk["alg_bytes_per_launch"], "launches_timed": args.roofline_steps,
