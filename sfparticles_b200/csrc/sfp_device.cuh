@@ -451,7 +451,8 @@ SFP_DEVICE_INLINE void ai_interp(double z, const double* __restrict__ iAt, const
 }
 
 // The differential rates take z = b^(2/3) and sqrt(z) = b^(1/3), both from one
-// cube root; z beyond the table -> 0.
+// cube root; z beyond the table -> 0, and b < 0 (chi below 0), whose power 2/3
+// is not a number, -> 0 too.
 // qed/rejection_sampling_tables.py:32-53
 SFP_DEVICE_INLINE double photon_rate(double chi_e, double delta, const double* iAt, const double* dAt, int zN,
                                      double zmax) {
@@ -460,7 +461,7 @@ SFP_DEVICE_INLINE double photon_rate(double chi_e, double delta, const double* i
     const double rz = cbrt(chi_gamma / (chi_e * chi_ep));
     const double z = rz * rz;
     const double factor = (((-kAlpha) * kMe) * (kC * kC)) / kHbar;
-    if (!(z <= zmax)) return 0.0;
+    if (!(z <= zmax) || rz < 0.0) return 0.0;
     double iA, dA;
     ai_interp(z, iAt, dAt, zN, zmax, iA, dA);
     return factor * (iA + (2.0 / z + chi_gamma * rz) * dA);
@@ -474,7 +475,7 @@ SFP_DEVICE_INLINE double pair_rate(double chi_gamma, double delta, const double*
     const double rz = cbrt(chi_gamma / (chi_e * chi_ep));
     const double z = rz * rz;
     const double factor = ((kAlpha * kMe) * (kC * kC)) / kHbar;
-    if (!(z <= zmax)) return 0.0;
+    if (!(z <= zmax) || rz < 0.0) return 0.0;
     double iA, dA;
     ai_interp(z, iAt, dAt, zN, zmax, iA, dA);
     return factor * (iA + (2.0 / z - chi_gamma * rz) * dA);
