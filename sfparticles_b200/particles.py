@@ -494,7 +494,8 @@ class Particles(object):
             self.buffer_size = new
             self._touch()
             return
-        for k, v in list(self._arr.items()):
+        for k in list(self._arr):  # (the names: a list of the arrays would hold every outgrown one to the end)
+            v = self._arr[k]
             if self._gpu:
                 import torch
                 t = torch.empty(new, dtype=v.dtype, device=v.device)
