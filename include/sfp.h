@@ -244,6 +244,14 @@ int sfp_run_destroy(sfp_run *r);
  * only where at least twice that is free) for later runs, at most 1 GiB in
  * all.  This gives the blocks above 32 MiB back to the driver. */
 int sfp_release_cached(void);
+/* Live runs keep the store of hot photons of their last call for the next one.
+ * This gives the stores of the current device's runs back to the driver, with
+ * the blocks that destroyed runs left; a run that is being called into, or
+ * whose stream is being captured, keeps its own.  Call it when an allocation
+ * fails: the next call of several steps makes a store again if there is room,
+ * and steps every photon if not, with the same results.  Synchronises the
+ * runs' streams.  freed (may be NULL): the bytes given back. */
+int sfp_release_stores(int64_t *freed);
 
 /* ---- learned photon-energy sampler (no counterpart in the reference) ------
  * An MLP (log10 chi, u) -> delta, 2 -> 64 -> 64 -> 64 -> 1 with SiLU, that can

@@ -124,6 +124,7 @@ _SIGS = {
     "sfp_table_od": ([c_i32, c_d, P, c_i64, P, c_i64, P, P, P, P], c_i32),
     "sfp_run_destroy": ([P], c_i32),
     "sfp_release_cached": ([], c_i32),
+    "sfp_release_stores": ([P], c_i32),
     "sfp_run_launches": ([P, P], c_i32),
     "sfp_run_hot_photons": ([P, P], c_i32),
     "sfp_run_barrier_withheld": ([P, P], c_i32),

@@ -1005,6 +1005,7 @@ struct sfp_run {
     bool hot_f64 = false;
     int grid_m = 0, grid_p = 0, grid_a = 0, grid_mt = 0, grid_pt = 0;
     size_t smem_m = 0, smem_p = 0, smem_mt = 0, smem_pt = 0, smem_end = 0;
+    std::mutex mu;  // held by the calls that use the store, and by the one that gives it back
     std::vector<long long> nb_lo;  // lower bounds of the device's n_buffered (it only grows between reads)
     cudaStream_t s = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
@@ -1017,6 +1018,10 @@ struct sfp_run {
     sfp_group_host mg, pg;
     std::vector<int> dseg;
 };
+
+// the live runs, whose stores sfp_release_stores may give back
+static std::mutex g_runs_mu;
+static std::vector<sfp_run*> g_runs;
 
 // `bytes` of the run's bookkeeping, 256-byte aligned, from its last block
 static int run_carve(sfp_run* r, size_t bytes, void** out) {
@@ -1427,6 +1432,10 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
             return cleanup(fail(SFP_ECUDA, "cannot raise dynamic shared memory"));
         r->grid_h = persistent_grid(r->k_hot, r->smem_p, 2);
     }
+    {
+        std::lock_guard<std::mutex> g(g_runs_mu);
+        g_runs.push_back(r);
+    }
     *out = r;
     return SFP_OK;
 }
@@ -1443,6 +1452,7 @@ int sfp_run_update(sfp_run* r, int n_seg, const sfp_segment* seg, const int64_t*
     int rc = validate_segments(r->n_inst, r->insts.data(), n_seg, seg);
     if (rc) return rc;
     r->segs.assign(seg, seg + n_seg);
+    std::lock_guard<std::mutex> own(r->mu);
     rc = run_alloc_tiles(r);
     if (rc) return rc;
     return run_upload(r, nullptr, n_buffered);
@@ -1672,6 +1682,7 @@ static int launch_small(sfp_run* r, int64_t nsteps, bool withhold = false) {
 int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
     if (!r) return fail(SFP_EINVAL, "sfp_run_steps: NULL run");
     if (nsteps <= 0) return SFP_OK;
+    std::lock_guard<std::mutex> own(r->mu);
     cudaStream_t cs = as_stream(stream);
     SFP_CUDA(cudaEventRecord(r->ev_in, cs));
     SFP_CUDA(cudaStreamWaitEvent(r->s, r->ev_in, 0));
@@ -1726,6 +1737,7 @@ int sfp_run_steps(sfp_run* r, int64_t nsteps, int graph_chunk, void* stream) {
 int sfp_run_steps_timed(sfp_run* r, int64_t nsteps, float* kernel_ms, void* stream) {
     if (!r || !kernel_ms) return fail(SFP_EINVAL, "sfp_run_steps_timed: NULL argument");
     if (nsteps <= 0) return SFP_OK;
+    std::lock_guard<std::mutex> own(r->mu);
     cudaStream_t cs = as_stream(stream);
     SFP_CUDA(cudaEventRecord(r->ev_in, cs));
     SFP_CUDA(cudaStreamWaitEvent(r->s, r->ev_in, 0));
@@ -1827,6 +1839,7 @@ int sfp_run_pending_need(sfp_run* r, int64_t* need) {
 
 int sfp_run_resume(sfp_run* r, void* stream) {
     if (!r) return fail(SFP_EINVAL, "sfp_run_resume: NULL run");
+    std::lock_guard<std::mutex> own(r->mu);
     sfp_step_state st;
     std::vector<long long> ns(2 * r->n_seg);
     std::vector<unsigned long long> ap(r->n_seg);
@@ -1872,6 +1885,7 @@ int sfp_run_launches(sfp_run* r, int64_t* count) {
 int sfp_run_hot_photons(sfp_run* r, int64_t* count) {
     if (!r || !count) return fail(SFP_EINVAL, "sfp_run_hot_photons: NULL argument");
     *count = 0;
+    std::lock_guard<std::mutex> own(r->mu);
     if (!r->hot_last) return SFP_OK;
     std::vector<unsigned long long> c(r->n_seg, 0);
     SFP_CUDA(cudaMemcpyAsync(c.data(), r->h.hot.count, r->n_seg * sizeof(c[0]), cudaMemcpyDeviceToHost, r->s));
@@ -1906,8 +1920,49 @@ int sfp_release_cached(void) {
     return SFP_OK;
 }
 
+// A run keeps its store between calls, as most of its calls would build one
+// of the same size; the species it steps may need that memory more.  A run
+// that another thread is calling into keeps its store (its mutex is taken), and
+// so does one whose stream a caller captures.
+int sfp_release_stores(int64_t* freed) {
+    if (freed) *freed = 0;
+    int64_t n = 0;
+    const int dev = device_now();
+    std::vector<run_block> old;
+    {
+        std::lock_guard<std::mutex> g(g_runs_mu);
+        for (sfp_run* r : g_runs) {
+            std::unique_lock<std::mutex> own(r->mu, std::try_to_lock);
+            if (!own.owns_lock() || !r->hot_block.p || r->rs.dev != dev || capturing(r->s)) continue;
+            // a stopped step's appends, resumed later, find no store
+            SFP_CUDA(cudaMemsetAsync(&r->h.st->hot_ok, 0, sizeof(int), r->s));
+            SFP_CUDA(cudaStreamSynchronize(r->s));
+            old.push_back(r->hot_block);
+            r->hot_block = run_block();
+            r->hot_room = 0;
+            r->hot_last = false;
+        }
+    }
+    {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        std::vector<run_block> keep;
+        for (const run_block& b : g_blocks) (b.dev == dev ? old : keep).push_back(b);
+        g_blocks.swap(keep);
+    }
+    for (const run_block& b : old) {
+        n += (int64_t)b.bytes;
+        cudaFree(b.p);
+    }
+    if (freed) *freed = n;
+    return SFP_OK;
+}
+
 int sfp_run_destroy(sfp_run* r) {
     if (!r) return SFP_OK;
+    {
+        std::lock_guard<std::mutex> g(g_runs_mu);
+        g_runs.erase(std::remove(g_runs.begin(), g_runs.end(), r), g_runs.end());
+    }
     const bool idle = r->s && cudaStreamSynchronize(r->s) == cudaSuccess;
     for (auto& kv : r->graphs) cudaGraphExecDestroy(kv.second);
     r->blocks.push_back(r->hot_block);

@@ -85,6 +85,21 @@ def _host_empty(shape, dtype):
 GROW_TOGETHER = 1 << 28
 
 
+def _with_room(allocate):
+    """allocate(), and once more where device memory runs out with the memory
+    that live runs hold for their own speed given back (their stores of hot
+    photons, which the next steps do without)."""
+    import torch
+    try:
+        return allocate()
+    except torch.OutOfMemoryError:
+        freed = ctypes.c_int64(0)
+        _lib.call("sfp_release_stores", ctypes.byref(freed))
+        if not freed.value:
+            raise
+    return allocate()
+
+
 def _random_seed() -> int:
     return int.from_bytes(os.urandom(8), "little")
 
@@ -207,14 +222,14 @@ class Particles(object):
         if self._gpu:
             import torch
             dt = torch.uint8 if name in _BOOL_ATTRS else torch.float64
-            self._arr[name] = torch.zeros(n, dtype=dt, device=_device())
+            self._arr[name] = _with_room(lambda: torch.zeros(n, dtype=dt, device=_device()))
         else:
             self._arr[name] = np.zeros(n, dtype=bool) if name in _BOOL_ATTRS else np.zeros(n)
 
     def _inv_gamma_from_u(self):
         if self._gpu:
             import torch
-            ig = torch.empty(self.buffer_size, dtype=torch.float64, device=_device())
+            ig = _with_room(lambda: torch.empty(self.buffer_size, dtype=torch.float64, device=_device()))
             if self.buffer_size:
                 _lib.call("sfp_inv_gamma", ctypes.c_void_p(self._arr["ux"].data_ptr()),
                           ctypes.c_void_p(self._arr["uy"].data_ptr()), ctypes.c_void_p(self._arr["uz"].data_ptr()),
@@ -263,7 +278,7 @@ class Particles(object):
         for k, v in list(self._arr.items()):
             a = np.ascontiguousarray(v, dtype=np.uint8 if k in _BOOL_ATTRS else np.float64)
             src.append(a)
-            self._arr[k] = torch.from_numpy(a).to(dev, non_blocking=True)
+            self._arr[k] = _with_room(lambda: torch.from_numpy(a).to(dev, non_blocking=True))
         torch.cuda.current_stream(dev).synchronize()
         del src
         self.__dict__["_gpu"] = True
@@ -498,7 +513,7 @@ class Particles(object):
             v = self._arr[k]
             if self._gpu:
                 import torch
-                t = torch.empty(new, dtype=v.dtype, device=v.device)
+                t = _with_room(lambda: torch.empty(new, dtype=v.dtype, device=v.device))
                 m = min(old, new)
                 t[:m] = v[:m]
                 if new > old:
@@ -530,7 +545,7 @@ class Particles(object):
                 v.device != dev or v.dtype not in (torch.float64, torch.uint8) or v.shape != (old,) or not v.is_contiguous()
                 for v in self._arr.values()):
             return False
-        block = torch.empty(sum(steps), dtype=torch.uint8, device=dev)
+        block = _with_room(lambda: torch.empty(sum(steps), dtype=torch.uint8, device=dev))
         jobs, grown, at = (_lib.GrowArray * len(steps))(), {}, 0
         for job, (k, v), size, step in zip(jobs, self._arr.items(), sizes, steps):
             t = block[at:at + new * size].view(v.dtype)
@@ -548,9 +563,9 @@ class Particles(object):
             import torch
             self._sync_positions()
             # the kept slots once, then one gather per array
-            idx = torch.nonzero(self._arr["_to_be_pruned"] == 0).flatten()
+            idx = _with_room(lambda: torch.nonzero(self._arr["_to_be_pruned"] == 0).flatten())
             for k, v in list(self._arr.items()):
-                self._arr[k] = torch.index_select(v, 0, idx)
+                self._arr[k] = _with_room(lambda: torch.index_select(v, 0, idx))
             N = int(idx.numel())
         else:
             keep = ~self._arr["_to_be_pruned"].astype(bool)

@@ -1,0 +1,120 @@
+"""The life of a run's store of hot photons: whether a call kept one, a store
+that newborn photons fill in the middle of a call, a step that waits for room
+while the store is live, memory that the species need more, memory that comes
+free again, and fields whose photons are all hot.  Whatever becomes of the
+store, the particles are those of single-step calls, bit for bit."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from gpu_helpers import cuda_or_skip
+from test_gpu_hot_photons import N, _arrays, _hard, _sim, _soft
+
+pytestmark = pytest.mark.gpu
+
+
+def _kept(sim):
+    from sfparticles_b200 import _lib
+    n = ctypes.c_int64(-1)
+    _lib.call("sfp_run_hot_photons", sim._run, ctypes.byref(n))
+    return n.value
+
+
+def _launches(sim):
+    from sfparticles_b200 import _lib
+    n = ctypes.c_int64(-1)
+    _lib.call("sfp_run_launches", sim._run, ctypes.byref(n))
+    return n.value
+
+
+def _same(a, b):
+    a, b = _arrays(a), _arrays(b)
+    assert [x.shape for x in a] == [x.shape for x in b]
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
+
+
+def _room(sim, slots):
+    """Free slots for every species, without the halts of a run that begins with full buffers."""
+    for p in sim.all_particles:
+        p._to_gpu()
+        p._resize(p.N_buffered + slots)
+
+
+class _LeaveFree:
+    """The device's memory taken but for `free` bytes."""
+
+    def __init__(self, free):
+        self.free = free
+
+    def __enter__(self):
+        import torch
+        from sfparticles_b200 import _lib
+        _lib.call("sfp_release_cached")
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        self.block = torch.empty(torch.cuda.mem_get_info()[0] - self.free, dtype=torch.uint8, device="cuda")
+
+    def __exit__(self, *a):
+        import torch
+        self.block = None
+        torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32"])
+@pytest.mark.parametrize("give_back", [False, True])
+def test_a_step_waits_for_room_while_the_store_is_live(form, give_back, monkeypatch):
+    cuda_or_skip()
+    from sfparticles_b200 import _lib, simulation
+    one, many = (_sim(form, _soft, n_e=100_000) for _ in range(2))
+    _room(one, 3_000_000)
+    _room(many, 30_000)
+    waits, resolve = [], simulation.resolve_pending
+
+    def resolved(run, species, update):
+        waits.append(_kept(many))
+        if give_back:  # the store's memory goes before the children are written
+            _lib.call("sfp_release_stores", None)
+            assert _kept(many) == 0
+        resolve(run, species, update)
+
+    for _ in range(24):
+        one.run_on_device(1)
+    monkeypatch.setattr(simulation, "resolve_pending", resolved)
+    many.run_on_device(24)
+    assert waits and waits[0] > 0  # steps ran through the store before the wait
+    _same(one, many)
+    for s in (one, many):
+        s.finish()
+
+
+@pytest.mark.parametrize("together", [False, True])
+def test_a_growth_that_fits_only_without_the_store(together, monkeypatch):
+    cuda_or_skip()
+    from sfparticles_b200 import particles
+    if together:
+        monkeypatch.setattr(particles, "GROW_TOGETHER", 1 << 30)
+    one, many = (_sim("fp32", _soft, n_ph=8_000_000) for _ in range(2))
+    for s in (one, many):
+        s.run_on_device(2)
+        s.reserve(20)
+    for _ in range(12):
+        one.run_on_device(1)
+    many.run_on_device(6)
+    assert _kept(many) > 0  # about 228 MB
+    pho = many.all_particles[2]
+    # 65 bytes a slot; the store holds about 228 MB
+    if together:  # the whole species anew
+        slots = pho.buffer_size
+        need = slots * 65
+    else:  # what it grows by, and one array beside it
+        slots = pho.buffer_size + 4_000_000
+        need = (slots - pho.buffer_size) * 65 + slots * 8
+    with _LeaveFree(need - 100_000_000):
+        pho._resize(slots)
+        many._update_run(many._run)
+    many.run_on_device(6)
+    _same(one, many)
+    for s in (one, many):
+        s.finish()
