@@ -7,6 +7,8 @@ from __future__ import annotations
 
 import numpy as np
 
+from .particles import _with_room
+
 
 def photon_energies(photons) -> np.ndarray:
     """Photon energies in units of m_e c^2 (|u| of each photon)."""
@@ -32,12 +34,15 @@ def photon_spectrum_device(photons, bins: int = 64, lo: float = 2.0, hi: float =
     n = photons.N_buffered
     if n == 0:
         return np.zeros(bins)
-    alive = photons._d("_to_be_pruned")[:n] == 0
-    ux, uy, uz = (photons._d(k)[:n] for k in ("ux", "uy", "uz"))
-    le = 0.5 * torch.log10(ux * ux + uy * uy + uz * uz)
-    le = le[alive & (le >= np.log10(lo)) & (le <= np.log10(hi))]
-    h = torch.histc(le, bins=bins, min=float(np.log10(lo)), max=float(np.log10(hi)))
-    return h.double().cpu().numpy()
+
+    def counts():
+        alive = photons._d("_to_be_pruned")[:n] == 0
+        ux, uy, uz = (photons._d(k)[:n] for k in ("ux", "uy", "uz"))
+        le = 0.5 * torch.log10(ux * ux + uy * uy + uz * uz)
+        le = le[alive & (le >= np.log10(lo)) & (le <= np.log10(hi))]
+        return torch.histc(le, bins=bins, min=float(np.log10(lo)), max=float(np.log10(hi)))
+
+    return _with_room(counts).double().cpu().numpy()
 
 
 def photon_histogram(photons, bins: int = 64, lo: float = 2.0, hi: float = 2500.0) -> np.ndarray:

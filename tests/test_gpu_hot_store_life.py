@@ -118,3 +118,24 @@ def test_a_growth_that_fits_only_without_the_store(together, monkeypatch):
     _same(one, many)
     for s in (one, many):
         s.finish()
+
+
+def test_a_spectrum_that_fits_only_without_the_store():
+    import torch
+    from sfparticles_b200.diagnostics import photon_spectrum_device
+    cuda_or_skip()
+    sim = _sim("fp32", _soft, n_ph=8_000_000)
+    sim.run_on_device(2)
+    sim.reserve(20)
+    sim.run_on_device(6)
+    assert _kept(sim) > 0  # about 228 MB
+    pho = sim.all_particles[2]
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    want = photon_spectrum_device(pho)
+    need = torch.cuda.max_memory_allocated() - before
+    with _LeaveFree(need - 100_000_000):
+        assert np.array_equal(photon_spectrum_device(pho), want)
+    assert want.sum() > 0 and _kept(sim) == 0
+    sim.finish()
