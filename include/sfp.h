@@ -231,7 +231,8 @@ int sfp_run_resume(sfp_run *r, void *stream);
 /* kernels that the run's step calls have launched so far (graph replays included) */
 int sfp_run_launches(sfp_run *r, int64_t *count);
 /* synchronous: photons in the store of the last step call, of which its photon
- * kernel read 40 bytes (float32 form; float64: 52) a step; 0 if it kept none */
+ * kernel read 40 bytes (float32 form; float64: 52) a step; 0 if it kept none,
+ * or gave it up (its room ran out, and the call went on over every photon) */
 int sfp_run_hot_photons(sfp_run *r, int64_t *count);
 /* Small populations run several steps per launch, with barriers between the
  * launch's blocks; a wait at one gives up after two seconds and sets the device

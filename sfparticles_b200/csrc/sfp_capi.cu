@@ -1888,8 +1888,11 @@ int sfp_run_hot_photons(sfp_run* r, int64_t* count) {
     std::lock_guard<std::mutex> own(r->mu);
     if (!r->hot_last) return SFP_OK;
     std::vector<unsigned long long> c(r->n_seg, 0);
+    int ok = 0;
+    SFP_CUDA(cudaMemcpyAsync(&ok, &r->h.st->hot_ok, sizeof(ok), cudaMemcpyDeviceToHost, r->s));
     SFP_CUDA(cudaMemcpyAsync(c.data(), r->h.hot.count, r->n_seg * sizeof(c[0]), cudaMemcpyDeviceToHost, r->s));
     SFP_CUDA(cudaStreamSynchronize(r->s));
+    if (!ok) return SFP_OK;  // given up on the device: the counts are of what found no room
     for (int s : r->pg.seg) *count += (int64_t)c[s];
     return SFP_OK;
 }

@@ -63,6 +63,47 @@ class _LeaveFree:
 
 
 @pytest.mark.parametrize("form", ["fp64", "fp32"])
+@pytest.mark.parametrize("energy,field,kept", [(_soft, "gauss", True), (_hard, "gauss", False),
+                                               (_soft, "focused", False)])
+def test_a_store_that_was_given_up_is_reported_as_none(form, energy, field, kept):
+    cuda_or_skip()
+    sim = _sim(form, energy, field=field)
+    _room(sim, 400_000)
+    sim.run_on_device(6)
+    n = _kept(sim)
+    assert (n > 0) == kept
+    if kept:  # one photon in ten is hot, and what the electrons emitted since
+        assert 0.09 * N < n < 0.2 * N
+    sim.finish()
+
+
+HOT = 1_300_000  # the store has room for 5/8 N + 65536 = 1440536
+
+
+def _nearly_full(r, n):
+    return np.where(np.arange(n) < HOT, r.uniform(100, 2500, n), r.uniform(2, 40, n))
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32"])
+def test_newborn_photons_fill_the_store_within_a_call(form):
+    cuda_or_skip()
+    steps = 40
+    few, one, many = (_sim(form, _nearly_full, n_e=300_000) for _ in range(3))
+    for s in (few, one, many):
+        _room(s, 3_000_000)
+    few.run_on_device(4)
+    assert HOT <= _kept(few) <= 1_440_536  # a short call keeps it
+    few.finish()
+    for _ in range(steps):
+        one.run_on_device(1)
+    many.run_on_device(steps)
+    assert _kept(many) == 0  # a long one does not
+    _same(one, many)
+    for s in (one, many):
+        s.finish()
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32"])
 @pytest.mark.parametrize("give_back", [False, True])
 def test_a_step_waits_for_room_while_the_store_is_live(form, give_back, monkeypatch):
     cuda_or_skip()
