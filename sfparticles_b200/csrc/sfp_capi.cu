@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <nvrtc.h>
 
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -995,7 +996,7 @@ struct sfp_run {
     run_block hot_block;                                        // their store
     long long hot_room = 0;                                     // entries it holds
     bool hot_last = false;                                      // the last call kept a store
-    long long hot_refused = 0;                                  // entries that found no memory
+    size_t hot_refused = SIZE_MAX, hot_refused_free = 0;        // bytes that the driver refused, and what was free then
     long long *d_hot_start = nullptr, *d_hot_cap = nullptr;
     int64_t launches = 0;                                       // kernels of its steps so far (graph replays too)
     int grid_h = 0;
@@ -1566,28 +1567,33 @@ constexpr int64_t HOT_MIN_STEPS = 4;
 constexpr int64_t SMALL_STEPS = 256;
 
 // room for n entries of the store, with some to grow into, in at most half of
-// the memory that is free; false, and remembered, where that is not enough
+// the memory that is free (the store's own counted).  Memory comes and goes
+// between calls, so each call that lacks room asks anew (cudaMemGetInfo, some
+// ten microseconds); only an allocation that the driver refused is not tried
+// again until more is free than then.
 static bool hot_room(sfp_run* r, long long n) {
-    if (r->hot_refused && n >= r->hot_refused) return false;
     const size_t each = r->hot_f64 ? 52 : 40;
     const bool f64 = r->hot_f64;
-    const long long room = r->hot_room ? n + n / 2 : n + n / 8;
+    size_t free_b = 0, all_b = 0;
+    if (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess) return false;
+    const size_t avail = free_b + r->hot_block.bytes;
+    auto fits = [&](long long entries) { return entries * each <= avail / 2 || block_cached(entries * each); };
+    long long room = r->hot_room ? n + n / 2 : n + n / 8;
+    if (!fits(room)) room = n + n / 8;
     const size_t bytes = (size_t)room * each;
+    if (!fits(room) || (bytes >= r->hot_refused && avail <= r->hot_refused_free)) return false;
     if (r->hot_block.p) {
         if (cudaStreamSynchronize(r->s) != cudaSuccess) return false;  // earlier calls still use it
         block_put(r->hot_block);
     }
     r->hot_block = run_block();
     r->hot_room = 0;
-    size_t free_b = 0, all_b = 0;
-    if (!block_cached(bytes) && (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || free_b / 2 < bytes)) {
-        r->hot_refused = n;
-        return false;
-    }
     if (!block_get(bytes, &r->hot_block)) {
-        r->hot_refused = n;
+        r->hot_refused = bytes;
+        r->hot_refused_free = avail;
         return false;
     }
+    r->hot_refused = SIZE_MAX;
     r->hot_room = room;
     char* p = static_cast<char*>(r->hot_block.p);
     const size_t d8 = (size_t)room * 8, du = (size_t)room * (f64 ? 8 : 4);

@@ -180,3 +180,16 @@ def test_a_spectrum_that_fits_only_without_the_store():
         assert np.array_equal(photon_spectrum_device(pho), want)
     assert want.sum() > 0 and _kept(sim) == 0
     sim.finish()
+
+
+def test_a_store_is_kept_again_once_there_is_memory():
+    cuda_or_skip()
+    sim = _sim("fp32", _soft, n_ph=8_000_000)
+    sim.run_on_device(2)
+    sim.reserve(30)
+    with _LeaveFree(120_000_000):  # half of it is less than a store of 1/4 takes (93 MB)
+        sim.run_on_device(5)
+        assert _kept(sim) == 0
+    sim.run_on_device(5)
+    assert _kept(sim) > 0
+    sim.finish()
