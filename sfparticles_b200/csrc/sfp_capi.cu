@@ -992,7 +992,8 @@ struct sfp_run {
     cudaKernel_t k_massive = nullptr, k_photon = nullptr, k_appends = nullptr, k_book = nullptr;
     cudaKernel_t k_massive_t = nullptr, k_photon_t = nullptr;  // any tile length
     cudaKernel_t k_sync = nullptr, k_epoch = nullptr;           // photon positions written out
-    cudaKernel_t k_hot = nullptr, k_hot_build = nullptr;        // hot photons (rejection sampling)
+    cudaKernel_t k_hot = nullptr, k_hot_build = nullptr, k_hot_bounded = nullptr;  // hot photons (rejection sampling)
+    int hot_bounded = -1;                                       // whether the fields have bounds (-1: not asked yet)
     run_block hot_block;                                        // their store
     long long hot_room = 0;                                     // entries it holds
     bool hot_last = false;                                      // the last call kept a store
@@ -1386,7 +1387,8 @@ int sfp_run_create(sfp_module* m, const sfp_run_config* cfg, int n_inst, const s
     for (size_t* q : {&r->smem_m, &r->smem_p, &r->smem_mt, &r->smem_pt}) *q = std::max(*q, r->smem_end);
     if (cfg->qed == SFP_QED_REJECTION && h.any_bw && h.pg.n_seg <= SFP_HOT_MAX_SEGS) {
         if ((rc = module_kernel(m, f64 ? "sfp_hot_fp64" : "sfp_hot_fp32", &r->k_hot)) ||
-            (rc = module_kernel(m, f64 ? "sfp_hot_build_fp64" : "sfp_hot_build_fp32", &r->k_hot_build)))
+            (rc = module_kernel(m, f64 ? "sfp_hot_build_fp64" : "sfp_hot_build_fp32", &r->k_hot_build)) ||
+            (rc = module_kernel(m, "sfp_hot_bounded_kernel", &r->k_hot_bounded)))
             return cleanup(rc);
         // the hot kernel keeps its tile map where the photon kernel has its ring
         r->smem_p = std::max(r->smem_p, (size_t)h.ring_off + (h.pg.n_seg + 1) * sizeof(long long));
@@ -1619,6 +1621,17 @@ static bool hot_room(sfp_run* r, long long n) {
 static bool hot_store(sfp_run* r, cudaStream_t caller) {
     if (!r->k_hot) return false;
     if (capturing(caller)) return false;  // a captured call gets launches only
+    if (r->hot_bounded < 0) {  // once per run, a launch and a wait of some 20 us
+        void* a[] = {&r->d};
+        int bounded = 0;
+        if (cudaLaunchKernel((const void*)r->k_hot_bounded, dim3(1), dim3(256), a, 0, r->s) != cudaSuccess ||
+            cudaMemcpyAsync(&bounded, &r->h.st->hot_ok, sizeof(bounded), cudaMemcpyDeviceToHost, r->s) != cudaSuccess ||
+            cudaStreamSynchronize(r->s) != cudaSuccess)
+            return false;
+        r->hot_bounded = bounded;
+        ++r->launches;
+    }
+    if (!r->hot_bounded) return false;
     std::vector<long long> start(r->n_seg, 0), cap(r->n_seg, 0);
     bool have = false;
     for (int eighths : {5, 3, 2}) {

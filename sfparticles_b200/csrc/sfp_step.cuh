@@ -1681,8 +1681,8 @@ __device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ 
 // momentum its tests read, events are marked in the segment and counted in
 // its tiles, so draws, results and their order are those of the full kernel.
 // The store lives for one call: buffers, flags and counts may change between
-// calls.  When its room runs out, or the field has no bound, hot_ok goes to
-// 0 and the steps run the full kernel.
+// calls.  When its room runs out, hot_ok goes to 0 and the steps run the full
+// kernel; a field without a bound gets no store (sfp_hot_bounded_body).
 // B200, a0 = 200, 24 % of the photons hot: 2.4e7 photons, float32 form 250 ->
 // 89 us a step; 1.2e7 photons, float64 form 502 -> 172 us.
 // ---------------------------------------------------------------------------
@@ -1715,6 +1715,22 @@ SFP_DEVICE_INLINE void sfp_hot_put(const sfp_run_dev* __restrict__ R, long long 
     H.idx[e] = idx;
 }
 
+// whether every field that a pair-creating photon flies in has a bound, to
+// st->hot_ok (one block).  Where one has none (a focused pulse, a user callable)
+// every photon is hot: the run keeps no store and takes no memory for one.
+__device__ __forceinline__ void sfp_hot_bounded_body(const sfp_run_dev* __restrict__ R) {
+    __shared__ int s_all;
+    if (threadIdx.x == 0) s_all = 1;
+    __syncthreads();
+    for (int j = threadIdx.x; j < R->pg.n_seg; j += blockDim.x) {
+        const sfp_segment& S = R->seg[R->pg.seg[j]];
+        if (S.bw && S.push && !(sfp_chi_per_gamma(sfp_field_params(R->inst[S.instance])) < __int_as_float(0x7f800000)))
+            s_all = 0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) R->st->hot_ok = s_all;
+}
+
 // copies the hot photons of every segment that creates pairs, a warp per
 // photon tile (the plan of the call's first step); one count per tile
 template <int FORM>
@@ -1739,7 +1755,7 @@ __device__ __forceinline__ void sfp_hot_build_body(const sfp_run_dev* __restrict
         const long long base = (tile - V.p_start[pos]) * (long long)V.ptile;
         const int len = (int)min(V.n_buf[si] - base, (long long)V.ptile);
         const float cpg = sfp_chi_per_gamma(sfp_field_params(R->inst[S.instance]));
-        if (!(cpg < __int_as_float(0x7f800000))) {  // no bound: every photon would be hot
+        if (!(cpg < __int_as_float(0x7f800000))) {  // no bound (parameters changed since the run asked)
             if (lane == 0) st->hot_ok = 0;
             return;
         }
@@ -2447,6 +2463,12 @@ __device__ __forceinline__ void sfp_sync_positions_body(const sfp_run_dev* __res
         }
     }
 }
+
+#if defined(SFP_STEP_QED_RS)
+extern "C" __global__ void __launch_bounds__(256) sfp_hot_bounded_kernel(const sfp_run_dev* __restrict__ R) {
+    sfp_hot_bounded_body(R);
+}
+#endif
 
 extern "C" __global__ void __launch_bounds__(32) sfp_epoch_kernel(const sfp_run_dev* __restrict__ R) {
     if (threadIdx.x == 0) R->st->pos_epoch = R->st->step;

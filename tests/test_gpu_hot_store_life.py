@@ -193,3 +193,19 @@ def test_a_store_is_kept_again_once_there_is_memory():
     sim.run_on_device(5)
     assert _kept(sim) > 0
     sim.finish()
+
+
+def test_a_field_without_a_bound_takes_no_store():
+    import torch
+    cuda_or_skip()
+    sim = _sim("fp32", _soft, field="focused")
+    _room(sim, 400_000)
+    sim.run_on_device(1)
+    torch.cuda.synchronize()
+    free, before = torch.cuda.mem_get_info()[0], _launches(sim)
+    sim.run_on_device(6)
+    assert torch.cuda.mem_get_info()[0] == free
+    sim.run_on_device(6)
+    # each call: the first step's bookkeeping, then three kernels a step; once in the run, the question for the bound
+    assert _launches(sim) - before <= 2 * (1 + 3 * 6) + 1
+    sim.finish()
