@@ -884,6 +884,16 @@ std::mutex g_pool_mu;
 std::vector<run_block> g_blocks;
 std::vector<run_stream> g_streams;
 
+// Another thread may be capturing a graph in the global mode, in which an
+// allocation, or a copy from pageable memory, by any thread breaks the capture.
+// What a run's store of hot photons takes of these belongs to no capture, so
+// the thread steps out of that rule meanwhile.
+struct outside_captures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    outside_captures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~outside_captures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 int device_now() {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1621,6 +1631,7 @@ static bool hot_room(sfp_run* r, long long n) {
 static bool hot_store(sfp_run* r, cudaStream_t caller) {
     if (!r->k_hot) return false;
     if (capturing(caller)) return false;  // a captured call gets launches only
+    const outside_captures oc;
     if (r->hot_bounded < 0) {  // once per run, a launch and a wait of some 20 us
         void* a[] = {&r->d};
         int bounded = 0;
@@ -1948,6 +1959,7 @@ int sfp_release_cached(void) {
 // so does one whose stream a caller captures.
 int sfp_release_stores(int64_t* freed) {
     if (freed) *freed = 0;
+    const outside_captures oc;
     int64_t n = 0;
     const int dev = device_now();
     std::vector<run_block> old;

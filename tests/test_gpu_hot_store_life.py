@@ -209,3 +209,53 @@ def test_a_field_without_a_bound_takes_no_store():
     # each call: the first step's bookkeeping, then three kernels a step; once in the run, the question for the bound
     assert _launches(sim) - before <= 2 * (1 + 3 * 6) + 1
     sim.finish()
+
+
+def test_steps_beside_a_capture_on_another_thread():
+    """A thread captures a graph in the global mode, in which no thread may make an unsafe call, while another steps
+    a run that takes its store's memory: the capture stays whole."""
+    import threading
+
+    import torch
+    cuda_or_skip()
+    one, many = (_sim("fp32", _soft) for _ in range(2))
+    for s in (one, many):
+        _room(s, 400_000)
+    for _ in range(7):
+        one.run_on_device(1)
+    many.run_on_device(1)
+    from sfparticles_b200 import _lib
+    x = torch.arange(1000, dtype=torch.float32, device="cuda")
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    began, stepped, fault = threading.Event(), threading.Event(), []
+
+    def capture():
+        try:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=torch.cuda.Stream(), capture_error_mode="global"):
+                y.copy_(x)
+                began.set()
+                stepped.wait(60)
+                y.mul_(2)
+            g.replay()
+            torch.cuda.synchronize()
+        except Exception as e:
+            fault.append(e)
+            began.set()
+
+    t = threading.Thread(target=capture)
+    t.start()
+    began.wait(60)
+    rc = _lib.load().sfp_run_steps(many._run, 6, 0, ctypes.c_void_p(0))
+    stepped.set()
+    t.join()
+    assert rc == 0 and not fault
+    assert torch.equal(y, 2 * x)
+    many._pos_dirty = True
+    nbuf, st = (ctypes.c_int64 * 3)(), _lib.RunState()
+    many._sync_state(many._run, st, nbuf)
+    assert not st.halted and _kept(many) > 0
+    _same(one, many)
+    for s in (one, many):
+        s.finish()
