@@ -188,6 +188,8 @@ class Ensemble(object):
         CUDA-event durations [ms] of its (massive, photon, appends)
         kernels, with the buffered counts before and after (per_call as in
         Simulation.time_step_kernel)."""
+        if int(per_call) < 1:
+            raise ValueError("per_call must be at least 1")
         if self._run is None:
             self._begin()
         L = _lib.load()

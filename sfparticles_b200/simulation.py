@@ -506,6 +506,8 @@ class Simulation(object):
         that waited for room is finished untimed and not reported.  per_call:
         steps of one native call; from four on, a large photon population is
         stepped through the call's store of hot photons, as in longer runs."""
+        if int(per_call) < 1:
+            raise ValueError("per_call must be at least 1")
         if getattr(self, "_run", None) is None:
             self._begin()
         before = [p.N_buffered for p in self.all_particles]
