@@ -553,7 +553,7 @@ class Particles(object):
         sizes = [v.element_size() for v in self._arr.values()]
         steps = [(new * s + 255) // 256 * 256 for s in sizes]
         dev = _device()
-        if not steps or sum(steps) > GROW_TOGETHER or any(
+        if not sum(steps) or sum(steps) > GROW_TOGETHER or any(
                 v.device != dev or v.dtype not in (torch.float64, torch.uint8) or v.shape != (old,) or not v.is_contiguous()
                 for v in self._arr.values()):
             return False
