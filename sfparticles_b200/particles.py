@@ -245,9 +245,18 @@ class Particles(object):
 
     def _drop_scratch(self):
         """Free the per-step scratch arrays and the stored 1/gamma; the fused
-        step keeps neither (1/gamma is recomputed from u on access)."""
-        for k in self._SCRATCH:
-            self._arr.pop(k, None)
+        step keeps neither (1/gamma is recomputed from u on access).  Scratch
+        that grew together with the state shares its block, which the state
+        then leaves for one of its own."""
+        gone = [self._arr.pop(k) for k in self._SCRATCH if k in self._arr]
+        if self._gpu and gone and self.buffer_size:
+            import torch
+            blocks = {v.untyped_storage().data_ptr() for v in gone}
+            if any(v.untyped_storage().data_ptr() in blocks for v in self._arr.values()):
+                try:
+                    self._grow_together(self.buffer_size, self.buffer_size)
+                except torch.OutOfMemoryError:
+                    pass  # no room for the move: the block stays whole
         self._touch()
 
     def _d(self, name, sync=True):
