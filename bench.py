@@ -889,38 +889,48 @@ class ClockSampler:
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
          "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
          "clocks_event_reasons.sw_power_cap")
+    EVERY_MS = 10  # between queries
 
     def __init__(self, gpu_index):
         self.idx = gpu_index
         self.rows = []
+        self.at = []  # when each row came
+        self.query = 0.0  # seconds that a query takes
         self.proc = None
 
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(["nvidia-smi", f"--id={self.idx}", f"--query-gpu={self.Q}",
-                                          "--format=csv,noheader,nounits", "-lms", "10"],
+                                          "--format=csv,noheader,nounits", "-lms", str(self.EVERY_MS)],
                                          stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
             # the timed region starts once sampling runs (short regions get samples)
             t0 = time.perf_counter()
-            while not self.rows and time.perf_counter() - t0 < 3.0:
-                time.sleep(0.01)
+            while len(self.rows) < 3 and time.perf_counter() - t0 < 3.0:
+                time.sleep(0.001)
+            if len(self.at) >= 3:
+                self.query = max(0.0, self.at[2] - self.at[1] - self.EVERY_MS * 1e-3)
             self.rows.clear()
+            self.at.clear()
         except Exception:
             self.proc = None
         return self
 
     def _read(self):
         for line in self.proc.stdout:
+            self.at.append(time.perf_counter())
             self.rows.append([c.strip() for c in line.split(",")])
 
     def __exit__(self, *a):
         if self.proc:
-            # a region shorter than a query (the collision window: 27 ms) has its sample in flight when it ends
-            t0 = time.perf_counter()
-            while not self.rows and time.perf_counter() - t0 < 0.2:
+            # a short region (the collision window: 27 ms; a query and its interval: 17) may end with its sample in
+            # flight: a row counts if its query began before the end
+            last = time.perf_counter() + self.query
+            while not self.rows and time.perf_counter() < last:
                 time.sleep(0.001)
+            n = sum(t <= last for t in list(self.at))
+            del self.rows[n:]
             self.proc.terminate()
             try:
                 self.proc.wait(timeout=5)
