@@ -240,10 +240,10 @@ int sfp_run_hot_photons(sfp_run *r, int64_t *count);
  * arrives, to exercise that path; synchronous; the run is of no use after. */
 int sfp_run_barrier_withheld(sfp_run *r, void *stream);
 int sfp_run_destroy(sfp_run *r);
-/* Destroyed runs leave their device blocks (bookkeeping, and the scratch
- * copies of photons that a call of several steps makes, 25 bytes per photon,
- * only where at least twice that is free) for later runs, at most 1 GiB in
- * all.  This gives the blocks above 32 MiB back to the driver. */
+/* Destroyed runs leave their device blocks (bookkeeping, and the store of hot
+ * photons that a call of several steps makes: 28 to 49 bytes per photon, less
+ * where memory is short, and only where at least twice that is free) for later
+ * runs, at most 1 GiB in all.  This gives the blocks above 32 MiB back to the driver. */
 int sfp_release_cached(void);
 /* Live runs keep the store of hot photons of their last call for the next one.
  * This gives the stores of the current device's runs back to the driver, with

@@ -859,11 +859,13 @@ struct sfp_group_host {
 // cudaMalloc / cudaFree calls, a stream and two events it cost 1.2 ms per
 // run (create 0.7, destroy 0.45; several times that on a busy host), against
 // 4 ms for 32 steps of 1e6 particles.  A run's store of hot photons is a
-// second block, of 25 bytes per photon.  Bounded: at most kPoolBlocks blocks
-// and kPoolBytes bytes, and as many streams, over all devices; the rest goes
-// back to the driver at once, blocks above kPoolKeep when a Simulation or
-// Ensemble ends (sfp_release_cached), and every block when an allocation
-// fails.  A run gives its blocks and stream back only once its stream is
+// second block: 40 or 52 bytes an entry, with entries for 5/8 of the photons
+// and an eighth or half of that to grow into, 28 to 49 bytes per photon.
+// Bounded: at most kPoolBlocks blocks and kPoolBytes bytes, and as many
+// streams, over all devices; the rest goes back to the driver at once, blocks
+// above kPoolKeep when a Simulation or Ensemble ends (sfp_release_cached), and
+// every block when an allocation fails, here or the caller's
+// (sfp_release_stores).  A run gives its blocks and stream back only once its stream is
 // idle, so no work in flight can reach them; the lists are under one lock.
 namespace {
 

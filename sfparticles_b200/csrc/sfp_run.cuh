@@ -17,16 +17,18 @@
 //              and push) and e-/e+ children of the marked photons (pushed),
 //              each written at the slot the reference's find_event_index +
 //              create_* gives it.
-// The last block of the step's last launch folds the step's appends and
+// The last block of the step's last event launch folds the step's appends and
 // prepares the next step; a bookkeeping kernel prepares the first of a call.
 // Both groups' segments start at multiples of 64 tiles, so a super-tile
-// never spans two segments.  No kernel waits on another block: there is no
-// spin-wait anywhere in a step.
+// never spans two segments.  No block of these launches waits for another.
+// Small populations take several steps in one cooperative launch instead
+// (sfp_steps_body), whose blocks meet at three grid barriers a step, each wait
+// with a time limit.
 #pragma once
 #include "sfp_types.h"
 
-// Tile length.  Each step the bookkeeping gives each group the shortest
-// power-of-two tile from SFP_TILE_MIN to SFP_TILE_MAX particles that cuts
+// Tile length.  Each step of three launches the bookkeeping gives each group the
+// shortest power-of-two tile from SFP_TILE_MIN to SFP_TILE_MAX particles that cuts
 // its population into at most SFP_TILE_TARGET tiles (massive group:
 // SFP_TILE_TARGET_M): a large population keeps 1024-particle tiles (32
 // sub-steps of the copy ring per ticket), a small one is spread over every
@@ -37,7 +39,8 @@
 // sampling), 183 -> 122 us (spin, learned sampler).  Results do not depend on
 // the tile: draws are keyed by particle index and children are written in
 // index order.  The tile counters hold SFP_TILE_TARGET_M tiles plus the
-// segments' padding at least, so the rule always fits.
+// segments' padding at least, so the rule always fits.  The one-launch kernel's
+// tiles are shares of the work, any multiple of 32 (sfp_small_tile).
 #define SFP_TILE_MIN 32
 #define SFP_TILE_MAX 1024
 #define SFP_TILE_TARGET 4096

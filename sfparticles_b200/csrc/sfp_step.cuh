@@ -2244,7 +2244,9 @@ __device__ __forceinline__ void sfp_appends_body(const sfp_run_dev* __restrict__
 // 1e3 e- 49 -> 31 / 34 -> 22 us, 1e4 63 -> 40 / 41 -> 23, 1e5 151 -> 95 /
 // 73 -> 37.
 // ---------------------------------------------------------------------------
-#define SFP_BARRIER_NS 2000000000ull  // 400 times the longest launch of the populations it serves
+// A wait lies within one step, under 0.8 ms at the largest populations that this
+// kernel serves: the limit is 2500 times that.
+#define SFP_BARRIER_NS 2000000000ull
 // segments of a run that may take this kernel
 #define SFP_SMALL_SEGS 64
 

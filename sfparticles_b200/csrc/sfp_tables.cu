@@ -21,8 +21,8 @@
 // Ai' come from sfp_airy.h.  The grids (z, chi rows, log-spaced delta) and
 // the rate prefactor are computed by the caller exactly as the reference
 // computes them (numpy linspace / logspace, -alpha m c^2 / hbar) and passed
-// in.  A warp per z point and per (chi row, delta column), a block of 21 warps
-// per total rate.
+// in.  A warp per z point, a thread per (chi row, delta column), a block of 21
+// warps per total rate.
 #include <cuda_runtime.h>
 
 #include <string>
