@@ -161,6 +161,21 @@ SFP_DEVICE_INLINE void field_simple(const double* __restrict__ P, double x, doub
     F[5] = (Ey / kC) * dir;
 }
 
+// (phase / kc)^2 + a, the exponent of a pulse's envelope.  The reciprocal of
+// kc^2 is the same for every particle, and so is its rounding, which the
+// exponent multiplies: with the square of phase times a rounded 1/kc, a pulse of
+// 3 fs was off by 1.54 times what the division by kc^2 leaves at 4 to 8 envelope
+// lengths (8.3e-15 instead of 5.4e-15), one of 25 fs by 1.03 times.  With the
+// reciprocal's remainder it is as exact as the division, and takes no longer:
+// 5e5 e- and 1.2e7 photons, 16 steps, 3.81 ms either way.
+SFP_DEVICE_INLINE double envelope_exponent(double phase, double kc, double a) {
+    const double kc2 = kc * kc, inv = 1.0 / kc2;
+    const double e = __fma_rn(-kc2, inv, 1.0);
+    const double rest = fabs(e) < 0.5 ? e * inv : 0.0;  // (kc infinite, a continuous wave: no remainder)
+    const double p2 = __dmul_rn(phase, phase);
+    return __fma_rn(p2, inv, __fma_rn(p2, rest, a));
+}
+
 // gaussian_laser_pulse, fields.py:152-168.
 // P = E0, k0, zR, w0, ctau, direction, x0, cep, cos(pol), sin(pol)
 
@@ -220,15 +235,15 @@ SFP_DEVICE_INLINE void field_gaussian(const double* __restrict__ P, double x, do
     // 5e5 e- and 1.2e7 photons, rejection sampling: massive kernel 78 -> 51 us,
     // hot photons 172 -> 113 us (with rsqrt, cbrt and one reciprocal in the push
     // and the rates).
-    const double izR = 1.0 / zR, iw0 = 1.0 / w0, ikc = 1.0 / kc;
+    const double izR = 1.0 / zR, iw0 = 1.0 / w0;
     const double xz = x * izR;
     const double rs = rsqrt(1.0 + xz * xz);
     const double rq = rs * rs;
     const double gouy = atan(xz);
     const double curv = x == 0.0 ? __longlong_as_double(0x7ff8000000000000ll) : ((0.5 * k0 * izR) * r2) * (xz * rq);
     const double phi = (kx + curv) - gouy;
-    const double rw = (iw0 * iw0) * r2, pk = phi * ikc;
-    const double E = ((E0 * cos(phi + cep)) * rs) * exp(-(rw * rq + pk * pk));
+    const double rw = (iw0 * iw0) * r2;
+    const double E = ((E0 * cos(phi + cep)) * rs) * exp(-envelope_exponent(phi, kc, rw * rq));
     const double Ey = E * cp, Ez = E * sp;
     F[0] = 0.0;
     F[1] = Ey;
@@ -247,7 +262,7 @@ SFP_DEVICE_INLINE void field_focused(const double* __restrict__ P, double x, dou
     x = dir * (x - xfoc);
     const double r2 = y * y + z * z;
     // the parameters' reciprocals are the same for every particle
-    const double izR = 1.0 / zR, iw0 = 1.0 / w0, ikc = 1.0 / (k0 * ctau);
+    const double izR = 1.0 / zR, iw0 = 1.0 / w0;
     const double xz = x * izR;
     const double eta = rsqrt(1.0 + xz * xz), eta2 = eta * eta;
     const double psiG = atan(xz);
@@ -258,8 +273,7 @@ SFP_DEVICE_INLINE void field_focused(const double* __restrict__ P, double x, dou
     const double xi = y * iw0;
     const double nu = z * iw0;
     const double rho2 = r2 * (iw0 * iw0), rho4 = rho2 * rho2, rho6 = rho4 * rho2, rho8 = rho4 * rho4;
-    const double pk = pc * ikc;
-    const double E = (E0 * eta) * exp(-(rho2 * eta2 + pk * pk));
+    const double E = (E0 * eta) * exp(-envelope_exponent(pc, k0 * ctau, rho2 * eta2));
     // C_n + i S_n = eta^n exp(i (psi + n psiG)): with cos psiG = eta and
     // sin psiG = eta x/zR, each is the one before times eta^2 (1 + i x/zR),
     // so one sincos serves all thirteen (1e6 e- with spin and the

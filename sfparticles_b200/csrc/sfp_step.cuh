@@ -1684,7 +1684,8 @@ __device__ __forceinline__ void sfp_photon_body(const sfp_run_dev* __restrict__ 
 // calls.  When its room runs out, hot_ok goes to 0 and the steps run the full
 // kernel; a field without a bound gets no store (sfp_hot_bounded_body).
 // B200, a0 = 200, 24 % of the photons hot: 2.4e7 photons, float32 form 250 ->
-// 89 us a step; 1.2e7 photons, float64 form 502 -> 172 us.
+// 89 us a step; 1.2e7 photons, float64 form 502 -> 172 us (113 with fewer
+// divisions in sfp_device.cuh).
 // ---------------------------------------------------------------------------
 template <int FORM>
 struct sfp_hot_real {
