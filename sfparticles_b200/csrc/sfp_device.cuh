@@ -164,8 +164,8 @@ SFP_DEVICE_INLINE void field_simple(const double* __restrict__ P, double x, doub
 // (phase / kc)^2 + a, the exponent of a pulse's envelope.  The reciprocal of
 // kc^2 is the same for every particle, and so is its rounding, which the
 // exponent multiplies: with the square of phase times a rounded 1/kc, a pulse of
-// 3 fs was off by 1.54 times what the division by kc^2 leaves at 4 to 8 envelope
-// lengths (8.3e-15 instead of 5.4e-15), one of 25 fs by 1.03 times.  With the
+// 3 fs (ctau / c) was off by 1.54 times what the division by kc^2 leaves at 4 to 8 envelope
+// lengths (8.3e-15 instead of 5.4e-15), one of 21 fs by 1.03 times.  With the
 // reciprocal's remainder it is as exact as the division, and takes no longer:
 // 5e5 e- and 1.2e7 photons, 16 steps, 3.81 ms either way.
 SFP_DEVICE_INLINE double envelope_exponent(double phase, double kc, double a) {
